@@ -20,9 +20,6 @@
 
 namespace topo {
 
-void level0_apply_bf16_input(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                             cudaStream_t s);
-
 static std::atomic<long long> g_launches{0};
 void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
@@ -262,13 +259,17 @@ Prec outer_prec(const topo_ctx* c) { return c->vec64 ? Prec::F64 : Prec::F32; }
 const void* outer_E(const topo_ctx* c) { return c->vec64 ? (const void*)c->E64 : (const void*)c->E32; }
 
 // ----------------------------------------------------------- operators
-void op_apply(topo_ctx* c, int l, Prec p, const void* u, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s) {
+// same_bits: the general level-0 kernels, whatever KE's symmetry. A V-cycle
+// with BF16 operators rounds its directions to BF16, and there a last-bit
+// difference of one product turns into 2^-8 of an entry in about 1e-5 of the
+// entries (2.5e-3 of the rms in the result). Krylov solves do not see that;
+// a single application through topo_gmg_apply keeps its results to the bit.
+void op_apply(topo_ctx* c, int l, Prec p, const void* u, void* y, Epi epi, const EpiArgs& ea, bool same_bits, cudaStream_t s) {
   Level& Lv = c->L[l];
   if (l == 0) {
     const void* E = (p == Prec::F64) ? (const void*)c->E64 : (const void*)c->E32;
-    if (p == Prec::BF16 && c->use_tc && level0_xs_supported(Lv.g))
-      level0_apply_xs(false, Lv.g, u, E, c->nmask0, y, epi, ea, s);
-    else level0_apply(p, Lv.g, u, E, Lv.mask, y, epi, ea, s);
+    if (p == Prec::BF16) level0_apply_bf16(c->use_tc, false, Lv.g, u, E, Lv.mask, c->nmask0, y, epi, ea, s, !same_bits);
+    else level0_apply(p, Lv.g, u, E, Lv.mask, y, epi, ea, s, !same_bits);
   } else {
     const void* S = p == Prec::F64 ? (const void*)Lv.S64 : p == Prec::F32 ? (const void*)Lv.S32 : (const void*)Lv.S16;
     stencil_apply(p, c->vec64, Lv.g, S, u, Lv.mask, y, epi, ea, s);
@@ -285,7 +286,7 @@ Prec hi_prec(const Level& Lv) { return Lv.prec == Prec::BF16 ? Prec::F32 : Lv.pr
 // operator only ever multiplies a direction. from_zero: x = 0 and r = b.
 // want_residual: also form the final residual r = b - K x (one more
 // application, which replaces the reference's separate residual matvec).
-void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const KrylovState* st, cudaStream_t s) {
+void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const KrylovState* st, bool same_bits, cudaStream_t s) {
   Level& Lv = c->L[l];
   const double lam = (std::isfinite(Lv.lam) ? Lv.lam : 1.0) * c->lam_safety;
   const Cheb ch = make_cheb(lam, c->cheb_lower, Lv.degree, c->cheb_form);
@@ -305,7 +306,7 @@ void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const Krylov
     ea.c2 = ch.c2[j];
     ea.ax = ch.ax[j];
     ea.st = const_cast<KrylovState*>(st);
-    op_apply(c, l, Lv.prec, dcur, nullptr, Epi::ChebR, ea, s);
+    op_apply(c, l, Lv.prec, dcur, nullptr, Epi::ChebR, ea, same_bits, s);
     std::swap(dcur, dnext);
   }
   if (want_residual) {
@@ -313,7 +314,7 @@ void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const Krylov
     ea.r = Lv.r;
     ea.s = ch.ax[Lv.degree - 1];
     ea.st = const_cast<KrylovState*>(st);
-    op_apply(c, l, Lv.prec, dcur, nullptr, Epi::RUpd, ea, s);
+    op_apply(c, l, Lv.prec, dcur, nullptr, Epi::RUpd, ea, same_bits, s);
   }
 }
 
@@ -333,18 +334,18 @@ void coarsest_solve(topo_ctx* c, const KrylovState* st, cudaStream_t s) {
 // Lv.x. Each coarse correction restricts the recursive residual, recurses,
 // adds e = P x_c and updates r -= K e, so the second correction of a W-cycle
 // restricts b - K x without a separate residual product.
-void vcycle(topo_ctx* c, int l, const KrylovState* st, cudaStream_t s) {
+void vcycle(topo_ctx* c, int l, const KrylovState* st, bool same_bits, cudaStream_t s) {
   Level& Lv = c->L[l];
   if (l == c->n_levels - 1) {
-    if (c->n_levels == 1) smooth(c, 0, true, false, st, s);
+    if (c->n_levels == 1) smooth(c, 0, true, false, st, same_bits, s);
     else coarsest_solve(c, st, s);
     return;
   }
-  smooth(c, l, true, true, st, s);  // x = S b, r = b - K x
+  smooth(c, l, true, true, st, same_bits, s);  // x = S b, r = b - K x
   Level& Lc = c->L[l + 1];
   for (int k = 0; k < c->cycle_gamma; ++k) {
     restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, Lc.b, st, s);
-    vcycle(c, l + 1, st, s);
+    vcycle(c, l + 1, st, same_bits, s);
     prolong_add(c->vec64, Lv.g, Lc.g, Lc.x, Lv.mask, Lv.x, Lv.e, st, s);  // x += e = P x_c
     EpiArgs ea{};
     ea.r = Lv.r;
@@ -353,18 +354,18 @@ void vcycle(topo_ctx* c, int l, const KrylovState* st, cudaStream_t s) {
     // r -= K e in FP32 even where the level's operator is BF16: the
     // post-smoother continues from this recursive residual, and BF16 here
     // raised the PCG iterations of the 1M-element cantilever from ~18 to ~95
-    op_apply(c, l, hi_prec(Lv), Lv.e, nullptr, Epi::RUpd, ea, s);  // r -= K e
+    op_apply(c, l, hi_prec(Lv), Lv.e, nullptr, Epi::RUpd, ea, same_bits, s);  // r -= K e
   }
-  smooth(c, l, false, false, st, s);
+  smooth(c, l, false, false, st, same_bits, s);
 }
 
-void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cudaStream_t s) {
+void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cudaStream_t s, bool same_bits = false) {
   Level& L0 = c->L[0];
   void* saved_b = L0.b;
   void* saved_x = L0.x;
   L0.b = const_cast<void*>(r);
   L0.x = z;
-  vcycle(c, 0, st, s);
+  vcycle(c, 0, st, same_bits, s);
   L0.b = saved_b;
   L0.x = saved_x;
 }
@@ -431,7 +432,9 @@ double lambda_fine(topo_ctx* c, cudaStream_t s) {
   const Prec p = f64 ? Prec::F64 : Prec::F32;
   for (int it = 0; it < 20; ++it) {
     EpiArgs ea{};
-    level0_apply(p, L0.g, v, f64 ? (const void*)c->E64 : (const void*)c->E32, L0.mask, Kv, Epi::Store, ea, s);
+    // mixed mode: the general kernel, so that the smoother's coefficients keep their bits (op_apply)
+    level0_apply(p, L0.g, v, f64 ? (const void*)c->E64 : (const void*)c->E32, L0.mask, Kv, Epi::Store, ea, s,
+                 c->mode != TOPO_MODE_MIXED);
     dotdiv(v, v, d);
     dot_to(f64, n, v, Kv, d + 1, c->red, s);
     if (f64) k_hadamard<double><<<gblocks(n), 256, 0, s>>>(n, (const double*)L0.dinv, (const double*)Kv, (double*)Av);
@@ -1109,6 +1112,7 @@ static void register_ke(topo_ctx* c, const double* KE) {
     host_galerkin_q(KE, Q.data());
     set_galerkin_q(Q.data());
     xs_prepare(KE);
+    pt_prepare(KE);
     d.ke.assign(KE, KE + 576);
   }
   d.live += 1;
@@ -1371,13 +1375,7 @@ int topo_matvec(topo_ctx* c, int dtype, const void* u, void* y, const void* E, v
     EpiArgs ea{};
     if (dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, Epi::Store, ea, c->cs);
     else if (dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, Epi::Store, ea, c->cs);
-    else if (dtype == TOPO_BF16) {
-      if (c->use_tc && level0_xs_supported(L0.g)) {
-        level0_apply_xs(true, L0.g, u, E, c->nmask0, y, Epi::Store, ea, c->cs);
-      } else {
-        level0_apply_bf16_input(L0.g, u, E, L0.mask, y, c->cs);
-      }
-    }
+    else if (dtype == TOPO_BF16) level0_apply_bf16(c->use_tc, true, L0.g, u, E, L0.mask, c->nmask0, y, Epi::Store, ea, c->cs);
     else throw std::invalid_argument("topo_matvec: bad dtype");
     return 0;
   } catch (const std::exception& e) {
@@ -1422,17 +1420,9 @@ int topo_level0_apply(topo_ctx* c, int u_dtype, int epi, const void* u, const vo
     ea.ax = ax;
     if (u_dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, ep, ea, c->cs);
     else if (u_dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, ep, ea, c->cs);
-    else if (u_dtype == TOPO_BF16 || u_dtype == TOPO_BF16_F32IN) {
-      const bool u16 = u_dtype == TOPO_BF16;
-      if (c->use_tc && level0_xs_supported(L0.g)) {
-        level0_apply_xs(u16, L0.g, u, E, c->nmask0, y, ep, ea, c->cs);
-      } else if (!u16) {
-        level0_apply(Prec::BF16, L0.g, u, E, L0.mask, y, ep, ea, c->cs);
-      } else {
-        if (ep != Epi::Store) throw std::runtime_error("topo_level0_apply: BF16-stored u on CUDA cores supports Store only");
-        level0_apply_bf16_input(L0.g, u, E, L0.mask, y, c->cs);
-      }
-    } else {
+    else if (u_dtype == TOPO_BF16 || u_dtype == TOPO_BF16_F32IN)
+      level0_apply_bf16(c->use_tc, u_dtype == TOPO_BF16, L0.g, u, E, L0.mask, c->nmask0, y, ep, ea, c->cs);
+    else {
       throw std::invalid_argument("topo_level0_apply: bad dtype");
     }
     return 0;
@@ -1455,7 +1445,7 @@ int topo_wait_status(topo_ctx* c, void* stream) {
 int topo_debug_bounds(int* tripped) {
   try {
     if (!tripped) throw std::invalid_argument("topo_debug_bounds: null pointer");
-    const int t = bounds_flag_level0() | bounds_flag_xs() | bounds_flag_cc() | bounds_flag_coarse() |
+    const int t = bounds_flag_level0() | bounds_flag_xs() | bounds_flag_cc() | bounds_flag_pt() | bounds_flag_coarse() |
                   bounds_flag_coarsest() | bounds_flag_design();
     *tripped = t ? 1 : 0;
 #ifdef TOPO_DEBUG_BOUNDS
@@ -1504,7 +1494,7 @@ int topo_gmg_apply(topo_ctx* c, const void* r, void* z, void* stream) {
     StreamGuard sg(c, stream);
     if (xs_error_flag(c->cs, false))
       throw std::runtime_error("level-0 K.u: an mbarrier wait of an earlier launch timed out");
-    vcycle_apply(c, r, z, nullptr, c->cs);
+    vcycle_apply(c, r, z, nullptr, c->cs, c->mode == TOPO_MODE_MIXED);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);

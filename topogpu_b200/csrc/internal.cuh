@@ -208,12 +208,18 @@ __device__ __forceinline__ void epilogue_store(const EpiDev<T>& e, long long i, 
 }
 
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                  Epi epi, const EpiArgs& ea, cudaStream_t s);
+                  Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true);
+// BF16-input operator (u stored BF16 or FP32, rounded); tc: the tensor-core
+// kernel may be used where the parity form does not apply. parity = false:
+// the general kernels only (same results to the last bit of rounding order)
+void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask,
+                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true);
 void level0_diag(const Grid& g, const double* E, const uint8_t* mask, double* diag, cudaStream_t s);
 // tensor-core BF16-input operator streaming along x (kmatvec_xs.cu); the
 // KE tile and the error flag are per device
 void xs_prepare(const double* KE_host);
 bool level0_xs_supported(const Grid& g);
+void level0_xs_check(const void* u, const void* E, const void* nmask, const EpiArgs& ea);  // throws on misaligned vectors
 // nmask: per-node free bits (bit c = DoF 3n+c free)
 void level0_apply_xs(bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* nmask, void* y, Epi epi,
                      const EpiArgs& ea, cudaStream_t s);
@@ -224,7 +230,13 @@ void cc_set_ke(const double* KE_host);
 bool level0_cc_supported(const Grid& g, bool f64);
 void level0_apply_cc(bool f64, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, Epi epi,
                      const EpiArgs& ea, int* err, cudaStream_t s);
+// level-0 K.u in parity form (kmatvec_pt.cu): KE with the cube's mirror symmetry
+void pt_prepare(const double* KE_host);
+bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u);
+void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
+                     Epi epi, const EpiArgs& ea, cudaStream_t s);
 void xs_debug(int skip_first_arrival, int poll_limit);
+void wait_debug(int& skip, int& poll);  // the test hook's current setting
 void modulus(long long n, const double* rho, double penal, double E0, double Emin, double* E,
              float* E32, cudaStream_t s);
 // dc_e = -penal (E0-Emin) rho_e^(penal-1) v_e^T KE u_e (v = u when null)
@@ -424,6 +436,7 @@ namespace topo {
 int bounds_flag_level0();
 int bounds_flag_xs();
 int bounds_flag_cc();
+int bounds_flag_pt();
 int bounds_flag_coarse();
 int bounds_flag_coarsest();
 int bounds_flag_design();

@@ -1,0 +1,677 @@
+// kmatvec_pt.cu - level-0 hex8 K.u in parity form (FP64, FP32 and BF16
+// inputs), streaming along x with TMA-staged node planes.
+//
+// The stiffness of a cube of an isotropic (or axis-aligned orthotropic)
+// material does not change under the three mirror images of the element. In
+// the basis of sums and differences of the corner values along x, y and z
+// (the 2x2x2 Hadamard transform of each displacement component) KE therefore
+// falls apart into eight 3x3 blocks, one per parity class, and one element
+// costs two separable transforms (adds) and 72 multiply-adds instead of 576.
+// Along x the transform of a node plane is shared by the two layers it
+// bounds, so the sums and differences in y and z are formed once per plane.
+// A KE without that symmetry takes the general kernels (kmatvec_xs.cu,
+// kmatvec_cc.cu): pt_prepare measures the couplings between the classes.
+//
+// Layout of the work. A plane is one contiguous run of nodes n = y*NZ + z. A
+// thread owns the element m (lower corner at node m; the elements with
+// z = nz or y = ny do not exist and have E = 0), loads the four nodes m, m+1,
+// m+NZ, m+NZ+1 of the next plane from shared memory and walks the layers of
+// its segment in x; the transformed previous plane (12 values) and the part
+// of the next plane's result already known (12 values) stay in registers.
+// Values are held as pairs over the parity in z (the z component's pair in
+// the opposite order, so that a pair belongs to one pair of classes): in FP32
+// each pair is one operand of the two-wide instructions (add / fma .f32x2),
+// which halves the issue slots of the arithmetic.
+// Back transform: in z with the neighbour lane's values (a warp covers 31
+// elements, its lane 0 repeats the last element of the warp before), in y
+// through shared memory: result(n) = P[n] + W[n - NZ]. The last addition and
+// the epilogue run one step later over the linear range of DoFs, so every
+// global access of the epilogue is coalesced, and one barrier per plane
+// suffices. A CTA is one (window of nodes, segment of planes) pair. What the
+// epilogue will read is prefetched to L2 two planes ahead.
+//
+// Staging: one cp.async.bulk (TMA, no multicast) per plane into a ring of
+// three slots, completed on mbarriers; start rounded down to 16 bytes, a
+// range ending in the vector's last partial 16-byte word gets that tail by
+// plain loads. Every wait is bounded: a timeout raises the device's error
+// flag, the copies in flight are drained (bounded) and the CTA exits.
+//
+// Bound: issue slots and the barrier per plane (about 280 instructions per
+// element and step; 20% of the elements are halo), not HBM: FP32 Store moves
+// 26 MB at 160x80x80 (4 us at the copy rate), ChebR 93 MB (14 us). Measured on
+// a B200, rotating buffers, against the kernels it replaced there (kernel
+// times): 160x80x80 FP32 Store 24.6 us (64), FP64 Store 42.7 us (130), ChebR
+// with BF16 rounding 36.0 us (67, tensor cores), FP32 RUpd 26.5 us (64);
+// 24x12x6 FP64 4.4 us (9.6). The tensor-core form of the same operator does
+// 1152 flop per element in 39 us of MMA issue; the parity form needs 312.
+//
+// Reference semantics: MatrixFreeKff.matvec (src/gpu_fem/solver_v2.py:1183-1223)
+// and fused_matvec_bf16 (src/gpu_fem/cuda_fused_matvec.py:112-246): the BF16
+// form multiplies BF16-rounded u by BF16-rounded KE and accumulates in FP32.
+#include "internal.cuh"
+#include "reduce.cuh"
+
+#include <atomic>
+#include <cmath>
+#include <cstring>
+#include <mutex>
+#include <stdexcept>
+#include <type_traits>
+#include <vector>
+
+namespace topo {
+namespace pt {
+
+// Class blocks K[q][c][d] of H KE H^T / 64: q = 4 qx + 2 qy + qz, member c of
+// class q is component c with parity q ^ e_c.
+// Stored as pairs over qz at ((2 qx + qy) * 9 + 3 c + d).
+__constant__ double2 cK64[36];
+__constant__ float2 cK32[36];  // of KE rounded to FP32: the FP32 operator is that of the rounded entries
+__constant__ float2 cKbf[36];  // of KE rounded to BF16
+
+constexpr int RING = 3;
+
+template <typename T>
+struct Params {
+  Grid g;
+  int PN, TO, nwin, nseg;  // nodes per plane, output nodes per window, windows, segments
+  const void* u;
+  const T* E;
+  const uint8_t* mask;
+  EpiDev<T> ep;
+  KrylovState* st;
+  RedWork red;
+  int* err;
+  int slot, off_pw, pw_n, off_bar;
+  int poll, skip;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+template <typename T>
+struct Pair;
+template <>
+struct Pair<double> {
+  using V = double2;
+};
+template <>
+struct Pair<float> {
+  using V = float2;
+};
+__device__ __forceinline__ double2 vadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 vsub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 vmul(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ double2 vfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.x, b.x, c.x), fma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+template <typename V, bool BF>
+__device__ __forceinline__ V kq(int i) {
+  if constexpr (std::is_same_v<V, double2>) return cK64[i];
+  else if constexpr (BF) return cKbf[i];
+  else return cK32[i];
+}
+
+template <typename T, typename TU>
+__device__ __forceinline__ T load_u(const TU* p) {
+  if constexpr (sizeof(TU) == 2) return (T)__bfloat162float(*p);
+  else return (T)*p;
+}
+
+// Hint: bring bytes [b, e) to L2 (thread 0; 16-byte granules, never past e).
+__device__ __forceinline__ void prefetch_l2(const void* b, const void* e) {
+  const unsigned long long a = (unsigned long long)b & ~15ULL;
+  const long long n = (long long)(((unsigned long long)e & ~15ULL) - a);
+  if (n > 0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)n) : "memory");
+}
+
+// Threads per CTA = 32 NW. MINB: CTAs per SM the registers are sized for.
+template <typename T, typename TU, bool BF, Epi EPI, int NW, int MINB>
+__global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_constant__ Params<T> P) {
+  if (P.st != nullptr && P.st->done) return;
+  extern __shared__ __align__(128) unsigned char sm[];
+  using V = typename Pair<T>::V;
+  constexpr int NT = 32 * NW, SU = (int)sizeof(TU), ST = (int)sizeof(T);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const Grid& g = P.g;
+  const int NZ = g.NZ, PN = P.PN;
+  const int w = (int)blockIdx.x % P.nwin, sg = (int)blockIdx.x / P.nwin;
+  const int n0 = w * P.TO, n1 = min(PN, n0 + P.TO);  // output nodes of a plane
+  const int xa = (int)((long long)g.NX * sg / P.nseg), xb = (int)((long long)g.NX * (sg + 1) / P.nseg);  // output planes
+  const int mlo = n0 - NZ - 1;                                             // first element of the window
+  const int ms = max(mlo, 0), me = min(PN, mlo + 31 * NW + NZ + 2);        // staged nodes of every plane
+  const int pf = max(xa - 1, 0), pl = min(xb, g.NX - 1);                   // planes read
+  const uint32_t bar0 = smem_u32(sm + P.off_bar);
+
+  for (int i = tid; i < P.off_pw / 16; i += NT) reinterpret_cast<uint4*>(sm)[i] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) {
+    for (int s = 0; s < RING; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8u * s), "r"(1) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+
+  // plane p -> slot (p - pf) % RING; node n of it at byte 16 + shift + 3 SU (n - mlo),
+  // where shift makes the copy's source and destination agree modulo 16
+  auto issue = [&](int p) {  // thread 0
+    const int sl = (p - pf) % RING;
+    const int shift = (int)((((long long)p * PN + mlo) * (3 * SU)) & 15);
+    const long long off0 = ((long long)p * PN + ms) * (3 * SU);
+    const long long n = (long long)(me - ms) * (3 * SU);
+    unsigned char* dst = sm + sl * P.slot + 16 + shift + (ms - mlo) * 3 * SU - (int)(off0 & 15);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(P.u);
+    const long long a = off0 & ~15LL, vfloor = (g.ndof * (long long)SU) & ~15LL;
+    long long e = (off0 + n + 15) & ~15LL;
+    if (e > vfloor) {
+      for (long long b = max(vfloor, a); b < off0 + n; ++b) dst[b - a] = src[b];
+      e = vfloor;
+    }
+    const uint32_t bytes = e > a ? (uint32_t)(e - a) : 0u, bar = bar0 + 8u * (uint32_t)sl;
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    if (bytes)
+      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
+                   "l"(src + a), "r"(bytes), "r"(bar)
+                   : "memory");
+  };
+  auto hint = [&](int x) {  // thread 0: what the epilogue of output plane x reads
+    const long long b = 3 * ((long long)x * PN + n0), e = 3 * ((long long)x * PN + n1);
+    if constexpr (EPI == Epi::Residual) prefetch_l2(P.ep.b + b, P.ep.b + e);
+    if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) prefetch_l2(P.ep.r + b, P.ep.r + e);
+    if constexpr (EPI == Epi::ChebR) {
+      prefetch_l2(P.ep.dinv + b, P.ep.dinv + e);
+      prefetch_l2(P.ep.x + b, P.ep.x + e);
+    }
+    prefetch_l2(P.mask + b, P.mask + e);
+  };
+  int issued = pf;  // planes pf .. issued-1 have been issued (thread 0)
+  if (tid == 0) {
+    for (; issued <= pl && issued < pf + RING; ++issued)
+      if (!(P.skip && issued == pf)) issue(issued);
+    hint(xa);
+  }
+
+  // this thread's element
+  const int li = 31 * warp + lane, m = mlo + li;
+  const int my = m >= 0 ? m / NZ : 0, mz = m - my * NZ;
+  const bool ev = m >= 0 && m < PN && my < g.ny && mz < g.nz;
+  const int le = g.ny * g.nz;
+  const T* Ep = P.E + (long long)pf * le + (ev ? my * g.nz + mz : 0);  // modulus of the current layer
+  const unsigned char* const ucol = sm + 16 + 3 * SU * li;            // node m in slot 0, without the shift
+  T* const pw = reinterpret_cast<T*>(sm + P.off_pw) + 3 * (li - 1);   // results (written by lanes >= 1): P, then W
+  const T* const pr = reinterpret_cast<const T*>(sm + P.off_pw) + tid;  // read in order of the DoFs
+  const int bsz = 2 * P.pw_n, cnt = 3 * (n1 - n0);
+
+  V prev[3][2], carry[3][2], other[3][2];
+  T Ecur = ev ? *Ep : (T)0;  // modulus of layer p-1 at step p
+#pragma unroll
+  for (int i = 0; i < 6; ++i) carry[i >> 1][i & 1].x = carry[i >> 1][i & 1].y = (T)0;
+  double part = 0.0;
+
+  // sums and differences of plane values in z and y: cur[c][py], pairs over pz
+  auto transform = [&](const unsigned char* q, V (&cur)[3][2]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      V t[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const TU* q0 = reinterpret_cast<const TU*>(q + r * 3 * SU * NZ);
+        T a0, a1;
+        if constexpr (SU == 4 && BF) {
+          const __nv_bfloat162 b0 = __floats2bfloat162_rn((float)q0[c], (float)q0[3 + c]);
+          a0 = __low2float(b0);
+          a1 = __high2float(b0);
+        } else {
+          a0 = load_u<T>(q0 + c);
+          a1 = load_u<T>(q0 + 3 + c);
+        }
+        t[r].x = c < 2 ? a0 + a1 : a1 - a0;
+        t[r].y = c < 2 ? a1 - a0 : a0 + a1;
+      }
+      cur[c][0] = vadd(t[0], t[1]);
+      cur[c][1] = vsub(t[1], t[0]);
+    }
+  };
+  // back transform: in z of one value pair (component c), with the neighbour lane
+  auto backz = [&](int c, const V& a) -> T {
+    const T even = c < 2 ? a.x : a.y, odd = c < 2 ? a.y : a.x;  // in z
+    return (even - odd) + __shfl_up_sync(0xffffffffu, even + odd, 1);
+  };
+  // in y of component c (t0, t1: its two y-parities) into buffer b: the shares
+  // of the element's lower (P) and upper (W) node row
+  auto backy = [&](int c, T t0, T t1, int b) {
+    if (lane > 0) {
+      pw[b * bsz + c] = t0 - t1;
+      pw[b * bsz + P.pw_n + c] = t0 + t1;
+    }
+  };
+  // what the epilogue of output plane x reads; then its last addition (from
+  // buffer b) and stores. Places tid + NT j of the window's DoFs.
+  struct Epv {
+    T r[3], d[3], x[3], u[3];
+    unsigned char m[3];
+  };
+  auto fetch = [&](int x, Epv& v) {
+    const long long base = 3 * ((long long)x * PN + n0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const unsigned i = tid + j * NT;
+      if (!((int)i < cnt && topo_in_range(base + i, g.ndof))) continue;
+      v.m[j] = (P.mask + base)[i];
+      if constexpr (EPI == Epi::Residual) v.r[j] = (P.ep.b + base)[i];
+      if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) v.r[j] = (P.ep.r + base)[i];
+      if constexpr (EPI == Epi::ChebR) {
+        v.d[j] = (P.ep.dinv + base)[i];
+        v.x[j] = (P.ep.x + base)[i];
+      }
+      if constexpr (EPI == Epi::ChebR || EPI == Epi::StoreDot) v.u[j] = load_u<T>(reinterpret_cast<const TU*>(P.u) + base + i);
+    }
+  };
+  auto finish = [&](int x, int b, const Epv& v) {
+    const long long base = 3 * ((long long)x * PN + n0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const unsigned i = tid + j * NT;
+      if (!((int)i < cnt && topo_in_range(base + i, g.ndof))) continue;
+      const bool fr = v.m[j] != 0;
+      const T a = pr[b * bsz + 3 * NZ + j * NT] + pr[b * bsz + P.pw_n + j * NT];
+      if constexpr (EPI == Epi::Store) {
+        (P.ep.y + base)[i] = fr ? a : (T)0;
+      } else if constexpr (EPI == Epi::StoreDot) {
+        const T y = fr ? a : (T)0;
+        (P.ep.y + base)[i] = y;
+        part += (double)v.u[j] * (double)y;
+      } else if constexpr (EPI == Epi::Residual) {
+        (P.ep.y + base)[i] = fr ? v.r[j] - a : (T)0;
+      } else if constexpr (EPI == Epi::RUpd) {
+        (P.ep.r + base)[i] = fr ? v.r[j] - P.ep.s * a : (T)0;
+      } else {
+        const T rv = v.r[j] - P.ep.s * a;
+        const T dn = P.ep.c1 * v.u[j] + P.ep.c2 * (v.d[j] * rv);
+        (P.ep.r + base)[i] = fr ? rv : (T)0;
+        (P.ep.d_out + base)[i] = fr ? dn : (T)0;
+        if (fr) (P.ep.x + base)[i] = v.x[j] + P.ep.ax * dn;
+      }
+    }
+  };
+
+  int slot = 0;                                                      // of the current plane
+  uint32_t phase = 0;                                                // of that slot's barrier
+  int shift = (int)((((long long)pf * PN + mlo) * (3 * SU)) & 15);   // of the current plane
+  const int dshift = (int)(((long long)PN * (3 * SU)) & 15);
+  // wait for the current plane; also a CTA barrier: the step before has read
+  // its slot and written its results
+  auto arrive = [&]() -> bool {
+    bool got = false;
+    for (int it = 0; it < P.poll && !got; ++it) got = mbar_try(bar0 + 8u * slot, phase);
+    if (!got) {
+      *(volatile int*)P.err = 1;  // mapped host memory: readable without a device sync
+      __threadfence_system();
+    }
+    return __syncthreads_and(got);
+  };
+  auto advance = [&]() {
+    shift = (shift + dshift) & 15;
+    if (++slot == RING) {
+      slot = 0;
+      phase ^= 1u;
+    }
+  };
+  // step p: layer p-1 between planes p-1 (a) and p (read into b)
+  auto step = [&](int p, V (&a)[3][2], V (&b)[3][2], int buf) -> bool {
+    if (!arrive()) return false;
+    if (tid == 0) {
+      if (issued <= pl) issue(issued++);  // into the slot of plane p - 1
+      if (p < xb) hint(p);
+    }
+    Ep += le;
+    const T En = (ev && p < pl) ? *Ep : (T)0;
+    // FP32: the epilogue's loads of plane p - 2 arrive behind the arithmetic
+    // of this step (FP64 has no registers left for them)
+    Epv ev2;
+    const bool fin = p - 2 >= xa;
+    if (ST == 4 && fin) fetch(p - 2, ev2);
+    transform(ucol + slot * P.slot + shift, b);
+    V Ev;
+    T t[3];
+    Ev.x = Ev.y = Ecur;
+    Ecur = En;
+#pragma unroll
+    for (int qy = 0; qy < 2; ++qy) {
+      // the classes (0,qy,qz) and (1,qy,qz), as pairs over qz, hold both
+      // x-parities of one value pair of each component
+      // class (0,qy,qz): x component odd in x, y and z components even
+      // class (1,qy,qz): x component even, y and z components odd
+      V v0[3], v1[3];
+      if constexpr (ST == 4) {
+        V S[3], D[3];  // x-sum and x-difference
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int py = c == 1 ? qy ^ 1 : qy;
+          S[c] = vadd(a[c][py], b[c][py]);
+          D[c] = vsub(b[c][py], a[c][py]);
+        }
+        const V u0[3] = {D[0], S[1], S[2]}, u1[3] = {S[0], D[1], D[2]};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const int i0 = qy * 9 + 3 * c, i1 = (2 + qy) * 9 + 3 * c;
+          v0[c] = vfma(kq<V, BF>(i0 + 2), u0[2], vfma(kq<V, BF>(i0 + 1), u0[1], vmul(kq<V, BF>(i0), u0[0])));
+          v1[c] = vfma(kq<V, BF>(i1 + 2), u1[2], vfma(kq<V, BF>(i1 + 1), u1[1], vmul(kq<V, BF>(i1), u1[0])));
+        }
+      } else {
+        // one qz after the other: half the registers
+#pragma unroll
+        for (int qz = 0; qz < 2; ++qz) {
+          auto el = [&](const V& v) -> T { return qz ? v.y : v.x; };
+          T S[3], D[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int py = c == 1 ? qy ^ 1 : qy;
+            S[c] = el(a[c][py]) + el(b[c][py]);
+            D[c] = el(b[c][py]) - el(a[c][py]);
+          }
+          const T u0[3] = {D[0], S[1], S[2]}, u1[3] = {S[0], D[1], D[2]};
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int i0 = qy * 9 + 3 * c, i1 = (2 + qy) * 9 + 3 * c;
+            (qz ? v0[c].y : v0[c].x) = el(kq<V, BF>(i0)) * u0[0] + el(kq<V, BF>(i0 + 1)) * u0[1] + el(kq<V, BF>(i0 + 2)) * u0[2];
+            (qz ? v1[c].y : v1[c].x) = el(kq<V, BF>(i1)) * u1[0] + el(kq<V, BF>(i1 + 1)) * u1[1] + el(kq<V, BF>(i1 + 2)) * u1[2];
+          }
+        }
+      }
+      const V even[3] = {v1[0], v0[1], v0[2]}, odd[3] = {v0[0], v1[1], v1[2]};  // in x
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int py = c == 1 ? qy ^ 1 : qy;
+        const T tc = backz(c, vfma(Ev, vsub(even[c], odd[c]), carry[c][py]));
+        carry[c][py] = vmul(Ev, vadd(even[c], odd[c]));
+        // results of plane p - 1 (not an output of this segment where p - 1 < xa)
+        if (qy == 0) t[c] = tc;
+        else if (c == 1) backy(c, tc, t[c], buf);
+        else backy(c, t[c], tc, buf);
+      }
+    }
+    if (fin) {
+      if (ST == 8) fetch(p - 2, ev2);
+      finish(p - 2, buf ^ 1, ev2);
+    }
+    advance();
+    return true;
+  };
+
+  bool ok = arrive();
+  if (ok) {
+    transform(ucol + shift, prev);
+    advance();
+  }
+  // two steps per round, so that the two planes' registers swap roles
+  for (int p = pf + 1; ok && p <= pl; p += 2) {
+    ok = step(p, prev, other, 0);
+    if (!ok || p + 1 > pl) break;
+    ok = step(p + 1, other, prev, 1);
+  }
+  if (ok) {
+    const int buf = (pl - pf) & 1;  // buffer of the next results; the other one holds plane pl - 1
+    __syncthreads();
+    Epv v;
+    if (pl - 1 >= xa) {
+      fetch(pl - 1, v);
+      finish(pl - 1, buf ^ 1, v);
+    }
+    if (xb == g.NX) {  // the last plane has no layer above it
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const T t0 = backz(c, carry[c][0]), t1 = backz(c, carry[c][1]);
+        backy(c, t0, t1, buf);
+      }
+      fetch(g.NX - 1, v);
+      __syncthreads();
+      finish(g.NX - 1, buf, v);
+    }
+  } else if (tid == 0) {
+    for (int j = max(pf, issued - RING); j < issued; ++j)
+      if (!(P.skip && j == pf))
+        for (int it = 0; it < P.poll && !mbar_try(bar0 + 8u * (uint32_t)((j - pf) % RING), (uint32_t)(((j - pf) / RING) & 1)); ++it) {
+        }
+  }
+  if constexpr (EPI == Epi::StoreDot) {
+    double v[1] = {part};
+    double tot[1];
+    if (grid_sum<1>(v, P.red, tot) && tid == 0) {
+      P.st->pAp = tot[0];
+      P.st->alpha = P.st->rz / tot[0];
+    }
+  }
+}
+
+}  // namespace pt
+
+// ----------------------------------------------------------------- host side
+namespace {
+struct PtDevice {
+  bool sym64 = false, sym32 = false, symbf = false;  // KE / KE rounded to FP32 / BF16 has the mirror symmetry
+  int nsm = 0;
+};
+std::mutex g_pt_mu;
+std::vector<PtDevice> g_pt;
+
+PtDevice& pt_device() {
+  int dev = 0;
+  TOPO_CUDA_CHECK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(g_pt_mu);
+  if ((int)g_pt.size() <= dev) g_pt.resize(dev + 1);
+  PtDevice& d = g_pt[dev];
+  if (d.nsm == 0) TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev));
+  return d;
+}
+
+// Class blocks of H KE H^T / 64; false when a coupling between classes is
+// above 1e-12 of the largest entry (KE then needs the general kernels).
+bool class_blocks(const double* KE, double* K) {
+  static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
+  auto h = [&](int p, int a) {  // basis function of parity p = 4 px + 2 py + pz at corner a
+    int s = 1;
+    for (int d = 0; d < 3; ++d)
+      if (((p >> (2 - d)) & 1) && !corner[a][d]) s = -s;
+    return s;
+  };
+  static const int e[3] = {4, 2, 1};
+  double top = 0.0, cross = 0.0;
+  for (int c = 0; c < 3; ++c)
+    for (int d = 0; d < 3; ++d)
+      for (int p = 0; p < 8; ++p)
+        for (int r = 0; r < 8; ++r) {
+          double v = 0.0;
+          for (int a = 0; a < 8; ++a)
+            for (int b = 0; b < 8; ++b) v += h(p, a) * h(r, b) * KE[(3 * a + c) * 24 + 3 * b + d];
+          v /= 64.0;
+          top = std::max(top, std::fabs(v));
+          if ((p ^ e[c]) == (r ^ e[d])) K[(p ^ e[c]) * 9 + 3 * c + d] = v;
+          else cross = std::max(cross, std::fabs(v));
+        }
+  return std::isfinite(top) && cross <= 1e-12 * top;
+}
+
+// Kernel widths: the (warps per CTA, CTAs per SM) pairs an instance is
+// compiled for, FP64 384 threads per SM (168 registers each), FP32 512 (128).
+// More threads with fewer registers spill: FP32 Store at 160x80x80 24.6 us
+// with 512 threads per SM, 30.4 with 768, 32.5 with 1024.
+template <typename T>
+struct Width {
+  static constexpr int NW[3] = {4, sizeof(T) == 8 ? 6 : 8, sizeof(T) == 8 ? 12 : 16};
+  static constexpr int PER[3] = {sizeof(T) == 8 ? 3 : 4, 2, 1};
+};
+constexpr int kPtSmem = 200 * 1024;  // dynamic shared memory of one CTA at most
+
+struct PtLayout {
+  int w, TO, nwin, nseg, slot, off_pw, pw_n, off_bar, total;
+};
+
+// Window width and segments. A CTA of NW warps yields 31 NW - NZ nodes per
+// plane (NZ of its elements are the window's halo row) and pays one extra
+// layer per segment. The three widths are compared by the layers a CTA walks
+// times the warps that share its SM (at least 8: below that a step is
+// latency and costs the same), over the waves of CTAs. A width that spends more
+// than 3/4 of its elements on the halo is left out; with none left (NZ above
+// 372, in FP64 279) the general kernels take the mesh.
+template <typename T>
+bool pt_layout(const Grid& g, int s_u, int nsm, PtLayout& best) {
+  const long long PN = (long long)g.NY * g.NZ;
+  if (PN >= (1 << 28)) return false;
+  double cost = 1e300;
+  for (int w = 0; w < 3; ++w) {
+    const int NW = Width<T>::NW[w], TO = 31 * NW - g.NZ;
+    if (TO < 31 * NW / 4) continue;
+    PtLayout L;
+    L.w = w;
+    L.TO = TO;
+    L.nwin = (int)((PN + TO - 1) / TO);
+    const long long slots = (long long)nsm * Width<T>::PER[w];
+    L.nseg = (int)std::max<long long>(1, std::min<long long>(g.NX, slots / L.nwin));
+    const long long ctas = (long long)L.nwin * L.nseg;
+    const double waves = std::ceil((double)ctas / (double)slots);
+    const double per = std::min<double>(Width<T>::PER[w], std::ceil((double)ctas / nsm));
+    const double c = waves * ((g.NX + L.nseg - 1) / L.nseg + 1) * std::max(8.0, per * NW);
+    const auto al = [](long long x) { return (int)((x + 127) & ~127LL); };
+    L.slot = al(64 + 3LL * s_u * (31 * NW + g.NZ + 3));
+    L.off_pw = pt::RING * L.slot;
+    L.pw_n = (3 * 31 * NW + 3) & ~3;
+    L.off_bar = L.off_pw + al(4LL * L.pw_n * (int)sizeof(T));
+    L.total = L.off_bar + 128;
+    if (L.total <= kPtSmem / Width<T>::PER[w] && c < cost) {
+      cost = c;
+      best = L;
+    }
+  }
+  return cost < 1e300;
+}
+
+template <typename T, typename TU, bool BF, Epi EPI, int W>
+void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, cudaStream_t s) {
+  auto* k = pt::k_level0_pt<T, TU, BF, EPI, Width<T>::NW[W], Width<T>::PER[W]>;
+  static std::atomic<uint64_t> raised{0};  // devices where this instance's shared-memory limit is raised
+  int dev = 0;
+  TOPO_CUDA_CHECK(cudaGetDevice(&dev));
+  if (L.total > 48 * 1024 && (dev > 63 || !(raised.load() >> dev & 1))) {
+    TOPO_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
+    if (dev <= 63) raised |= 1ull << dev;
+  }
+  k<<<(unsigned)(L.nwin * L.nseg), 32 * Width<T>::NW[W], L.total, s>>>(P);
+  TOPO_LAUNCH_CHECK();
+}
+
+template <typename T, typename TU, bool BF, Epi EPI>
+void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, const EpiArgs& ea, cudaStream_t s) {
+  PtLayout L;
+  if (!pt_layout<T>(g, (int)sizeof(TU), pt_device().nsm, L))
+    throw std::runtime_error("level0 K.u: mesh not supported by the parity form");
+  pt::Params<T> P;
+  P.g = g;
+  P.PN = g.NY * g.NZ;
+  P.TO = L.TO;
+  P.nwin = L.nwin;
+  P.nseg = L.nseg;
+  P.u = u;
+  P.E = (const T*)E;
+  P.mask = mask;
+  P.ep = make_epi<T>(y, ea);
+  P.st = ea.st;
+  P.red = ea.red;
+  P.err = wait_error_flag();
+  P.slot = L.slot;
+  P.off_pw = L.off_pw;
+  P.pw_n = L.pw_n;
+  P.off_bar = L.off_bar;
+  P.poll = 1 << 22;
+  P.skip = 0;
+  if (BF) wait_debug(P.skip, P.poll);
+  switch (L.w) {
+    case 0: launch_pt_w<T, TU, BF, EPI, 0>(L, P, s); break;
+    case 1: launch_pt_w<T, TU, BF, EPI, 1>(L, P, s); break;
+    default: launch_pt_w<T, TU, BF, EPI, 2>(L, P, s); break;
+  }
+}
+}  // namespace
+
+void pt_prepare(const double* KE) {
+  double K[72], Kf[72], Kb[72], KEf[576], KEb[576];
+  double2 d64[36];
+  float2 f[36], fb[36];
+  for (int i = 0; i < 576; ++i) {
+    const float x = (float)KE[i];
+    uint32_t b;
+    std::memcpy(&b, &x, 4);
+    b = (b + 0x7FFFu + ((b >> 16) & 1u)) & 0xFFFF0000u;
+    float r;
+    std::memcpy(&r, &b, 4);
+    KEb[i] = r;
+    KEf[i] = x;
+  }
+  const bool s64 = class_blocks(KE, K), s32 = class_blocks(KEf, Kf), sbf = class_blocks(KEb, Kb);
+  for (int q = 0; q < 4; ++q)  // q = 2 qx + qy; class 2 q + qz
+    for (int i = 0; i < 9; ++i) {
+      const int e = 18 * q + i, o = e + 9;
+      d64[9 * q + i] = make_double2(K[e], K[o]);
+      f[9 * q + i] = make_float2((float)Kf[e], (float)Kf[o]);
+      fb[9 * q + i] = make_float2((float)Kb[e], (float)Kb[o]);
+    }
+  TOPO_CUDA_CHECK(cudaMemcpyToSymbol(pt::cK64, d64, sizeof(d64)));
+  TOPO_CUDA_CHECK(cudaMemcpyToSymbol(pt::cK32, f, sizeof(f)));
+  TOPO_CUDA_CHECK(cudaMemcpyToSymbol(pt::cKbf, fb, sizeof(fb)));
+  PtDevice& d = pt_device();
+  d.sym64 = s64;
+  d.sym32 = s32;
+  d.symbf = sbf;
+}
+
+// The parity form takes this operator: the element stiffness has the mirror
+// symmetry, the mesh a window layout, and the copies' 16-byte alignment holds.
+bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
+  const PtDevice& d = pt_device();
+  PtLayout L;
+  return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 &&
+         (f64 ? pt_layout<double>(g, 8, d.nsm, L) : pt_layout<float>(g, 4, d.nsm, L));
+}
+
+// f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
+// where it is read) or stored BF16 (u_bf16). Epilogues as level0_apply.
+void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
+                     Epi epi, const EpiArgs& ea, cudaStream_t s) {
+#define TOPO_PT_CASE(EP)                                                                                     \
+  case Epi::EP:                                                                                              \
+    if (f64) launch_pt<double, double, false, Epi::EP>(g, u, E, mask, y, ea, s);                             \
+    else if (u_bf16) launch_pt<float, __nv_bfloat16, true, Epi::EP>(g, u, E, mask, y, ea, s);                \
+    else if (bf) launch_pt<float, float, true, Epi::EP>(g, u, E, mask, y, ea, s);                            \
+    else launch_pt<float, float, false, Epi::EP>(g, u, E, mask, y, ea, s);                                   \
+    break;
+  switch (epi) {
+    TOPO_PT_CASE(Store)
+    TOPO_PT_CASE(Residual)
+    TOPO_PT_CASE(ChebR)
+    TOPO_PT_CASE(RUpd)
+    case Epi::StoreDot:
+      if (f64) launch_pt<double, double, false, Epi::StoreDot>(g, u, E, mask, y, ea, s);
+      else if (!bf) launch_pt<float, float, false, Epi::StoreDot>(g, u, E, mask, y, ea, s);
+      else throw std::runtime_error("level0 K.u: the dot product goes with the FP32 and FP64 operators");
+      break;
+  }
+#undef TOPO_PT_CASE
+}
+
+TOPO_BOUNDS_READER(bounds_flag_pt)
+
+}  // namespace topo

@@ -247,10 +247,15 @@ static void launch_level0(const Grid& g, const void* u, const void* E, const uin
 }
 
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, Epi epi,
-                  const EpiArgs& ea, cudaStream_t s) {
-  // FP64 / FP32: the x-streaming kernel (kmatvec_cc.cu) when its planes fit
-  // in shared memory; the brick kernel below otherwise and for the BF16
-  // emulation on CUDA cores.
+                  const EpiArgs& ea, cudaStream_t s, bool parity) {
+  // The parity form (kmatvec_pt.cu) takes every mesh with a window layout when
+  // KE has the cube's mirror symmetry. Without it FP64 / FP32 run the
+  // x-streaming kernel (kmatvec_cc.cu) when its planes fit in shared memory;
+  // the brick kernel below otherwise and for the BF16 emulation.
+  if (parity && level0_pt_supported(g, p == Prec::F64, p == Prec::BF16, u)) {
+    level0_apply_pt(p == Prec::F64, p == Prec::BF16, false, g, u, E, mask, y, epi, ea, s);
+    return;
+  }
   const bool al = ((uintptr_t)u & 15) == 0 && ((uintptr_t)E & 15) == 0;
   switch (p) {
     case Prec::F64:
@@ -265,11 +270,21 @@ void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uin
   }
 }
 
-// BF16-storage input variant used by the public matvec entry (u in bf16).
-void level0_apply_bf16_input(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                             cudaStream_t s) {
-  EpiArgs ea{};
-  launch_level0<float, __nv_bfloat16, true>(g, u, E, mask, y, Epi::Store, ea, s);
+// The tensor-core kernel's meshes and pointers (16-byte aligned vectors) are
+// what the fused epilogues accept with tc set, whichever kernel runs them.
+void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask,
+                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity) {
+  if (tc && level0_xs_supported(g)) {
+    level0_xs_check(u, E, nmask, ea);
+    if (parity && level0_pt_supported(g, false, true, u)) level0_apply_pt(false, true, u_bf16, g, u, E, mask, y, epi, ea, s);
+    else level0_apply_xs(u_bf16, g, u, E, nmask, y, epi, ea, s);
+  } else if (!u_bf16) {
+    level0_apply(Prec::BF16, g, u, E, mask, y, epi, ea, s, parity);
+  } else {
+    if (epi != Epi::Store) throw std::runtime_error("topo_level0_apply: BF16-stored u on CUDA cores supports Store only");
+    if (parity && level0_pt_supported(g, false, true, u)) level0_apply_pt(false, true, true, g, u, E, mask, y, epi, ea, s);
+    else launch_level0<float, __nv_bfloat16, true>(g, u, E, mask, y, epi, ea, s);
+  }
 }
 
 // ------------------------------------------------------------------ diagonal
