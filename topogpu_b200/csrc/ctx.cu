@@ -209,7 +209,8 @@ struct topo_ctx {
   RedWork red{};
   double* dtmp = nullptr;       // 64 device doubles
   double* oc_state = nullptr;
-  double* Hs = nullptr;
+  double* Hs = nullptr;        // nelem doubles: scratch of the filter and the OC updates
+  double* oc_cand = nullptr;   // candidates of the projected OC (allocated by its first call)
   FilterStencil fstencil;
   bool ke_registered = false;  // holds a reference on its device's KE
   cudaStream_t cs = nullptr;
@@ -1211,7 +1212,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->red.partials = c->alloc<double>(1 << 18);
     c->red.ticket = c->alloc<unsigned int>(1);
     c->dtmp = c->alloc<double>(64);
-    c->oc_state = c->alloc<double>(16);
+    c->oc_state = c->alloc<double>(32);
     c->Hs = c->alloc<double>(g0.nelem);
     c->fstencil.off = c->alloc<int>(3 * kMaxFilterOff);
     c->fstencil.w = c->alloc<double>(kMaxFilterOff);
@@ -1641,8 +1642,8 @@ int topo_oc_filtered(topo_ctx* c, const double* rho, const double* dc, const dou
   try {
     if (!c || !rho || !dc || !dv || !colsum || !out) throw std::invalid_argument("topo_oc_filtered: null pointer");
     StreamGuard sg(c, stream);
-    const int ev = oc_update_filtered(c->L[0].g.nelem, rho, dc, dv, colsum, volfrac, move, rho_min, out, c->red,
-                                      c->oc_state, c->cs);
+    const int ev = oc_update_filtered(c->L[0].g.nelem, rho, dc, dv, colsum, volfrac, move, rho_min, out, c->Hs,
+                                      c->red, c->oc_state, c->cs);
     if (out_evals) *out_evals = ev;
     return 0;
   } catch (const std::exception& e) {
@@ -1672,8 +1673,9 @@ int topo_oc_projected(topo_ctx* c, double rmin, const double* rho, const double*
     if (out == rho || out == dc || out == dv)
       throw std::invalid_argument("topo_oc_projected: out must not alias rho, dc or dv");
     StreamGuard sg(c, stream);
+    if (!c->oc_cand) c->oc_cand = c->alloc<double>(oc_projected_candidates() * c->L[0].g.nelem);
     const int ev = oc_update_projected(c->fstencil, c->L[0].g, rmin, rho, dc, dv, beta, eta, volfrac, move, rho_min, out, c->Hs,
-                                       c->red, c->oc_state, c->cs);
+                                       c->oc_cand, c->red, c->oc_state, c->cs);
     if (out_evals) *out_evals = ev;
     return 0;
   } catch (const std::exception& e) {

@@ -356,24 +356,31 @@ void scale_dev(bool f64, long long n, const void* x, const double* num, const do
 // device memory owned by a context (so contexts with different radii, or on
 // different devices, never share it).
 constexpr int kMaxFilterOff = 1331;  // (2*5+1)^3: rmin < 6
+constexpr int kMaxFilterR = 5;
+struct TapGroups {  // taps start[dz + R] .. start[dz + R + 1] - 1 have this dz
+  int R;
+  int start[2 * kMaxFilterR + 2];
+};
 struct FilterStencil {
   double rmin = -1.0;
   int n = 0;
+  TapGroups tg{};
   int* off = nullptr;    // 3 * kMaxFilterOff
   double* w = nullptr;   // kMaxFilterOff
 };
 void filter_apply(FilterStencil& fs, const Grid& g, double rmin, const double* in, double* out, bool transpose,
-                  double* Hs_work, cudaStream_t s);
+                  double* work, cudaStream_t s);
 int oc_update(long long n, const double* rho, const double* dc, double volfrac, double move,
               double rho_min, double* out, RedWork red, double* state, cudaStream_t s);
 int oc_update_filtered(long long n, const double* rho, const double* dc, const double* dv,
                        const double* colsum, double volfrac, double move, double rho_min, double* out,
-                       RedWork red, double* state, cudaStream_t s);
+                       double* work, RedWork red, double* state, cudaStream_t s);
 void heaviside_apply(long long n, const double* rho_f, double beta, double eta, double* phys, double* dh,
                      cudaStream_t s);
 int oc_update_projected(FilterStencil& fs, const Grid& g, double rmin, const double* rho, const double* dc, const double* dv,
                         double beta, double eta, double volfrac, double move, double rho_min, double* out,
-                        double* Hs_work, RedWork red, double* st, cudaStream_t s);
+                        double* work, double* cand, RedWork red, double* st, cudaStream_t s);
+int oc_projected_candidates();  // cand holds this many doubles per element
 void field_stats(long long n, const double* x, double* out4_dev, RedWork red, cudaStream_t s);
 
 // error plumbing
