@@ -32,153 +32,186 @@ __device__ __forceinline__ void node_xyz(const Grid& g, long long n, int& ix, in
 
 // ------------------------------------------------------------ level-1 Galerkin
 // Coarse element e contributes Kc_e = sum_stu E_f(2e+stu, clamped) Q_stu
-// (multigrid_v4.py:182-203, 256). One thread per coarse node I gathers, for
-// each neighbour J = I + delta, the 3x3 block sum over the coarse elements
-// that contain both I and J.
-__global__ void k_level1_assemble(Grid f, Grid c, const double* __restrict__ Ef, const uint8_t* __restrict__ mc,
-                                  double* __restrict__ S) {
-  const long long I = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (I >= c.nnodes) return;
-  int ix, iy, iz;
-  node_xyz(c, I, ix, iy, iz);
-  for (int k = 0; k < 27; ++k) {
-    const int dx = k / 9 - 1, dy = (k / 3) % 3 - 1, dz = k % 3 - 1;
-    const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
-    double B[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const bool jin = jx >= 0 && jx < c.NX && jy >= 0 && jy < c.NY && jz >= 0 && jz < c.NZ;
-    if (jin) {
-      for (int ox = -1; ox <= 0; ++ox) {
-        const int mx = dx - ox;
-        if (mx < 0 || mx > 1) continue;
-        const int ex = ix + ox;
-        if (ex < 0 || ex >= c.nx) continue;
-        for (int oy = -1; oy <= 0; ++oy) {
-          const int my = dy - oy;
-          if (my < 0 || my > 1) continue;
-          const int ey = iy + oy;
-          if (ey < 0 || ey >= c.ny) continue;
-          for (int oz = -1; oz <= 0; ++oz) {
-            const int mz = dz - oz;
-            if (mz < 0 || mz > 1) continue;
-            const int ez = iz + oz;
-            if (ez < 0 || ez >= c.nz) continue;
-            const int a = corner_of(-ox, -oy, -oz);
-            const int m = corner_of(mx, my, mz);
-            for (int stu = 0; stu < 8; ++stu) {
-              const int s = stu >> 2, t = (stu >> 1) & 1, u = stu & 1;
-              const int fx = min(2 * ex + s, f.nx - 1), fy = min(2 * ey + t, f.ny - 1), fz = min(2 * ez + u, f.nz - 1);
-              const double Ee = Ef[((long long)fx * f.ny + fy) * f.nz + fz];
-              const double* Q = cQ + stu * 576;
+// (multigrid_v4.py:182-203, 256). One thread per (coarse node I, neighbour
+// J = I + delta) gathers the 3x3 block sum over the coarse elements that
+// contain both. The offset k is uniform over a CTA (blockIdx.y): the at most
+// 64 blocks Q_stu[a][m] it needs sit in shared memory, and a thread forms its
+// block for L1N nodes, so that a (broadcast) load feeds L1N multiply-adds.
+// Bound by the 627 M FP64 multiply-adds at 160x80x80 (35 us). There: a node's
+// 27 blocks as one thread's loop over constant memory 324 us, one thread per
+// block 280 us, now 222 us.
+constexpr int L1T = 128, L1N = 2;
+__global__ void __launch_bounds__(L1T) k_level1_assemble(Grid f, Grid c, const double* __restrict__ Ef,
+                                                         const uint8_t* __restrict__ mc, double* __restrict__ S) {
+  __shared__ __align__(16) double qs[64][10];  // [o * 8 + stu][3 cc + dd]
+  const int k = blockIdx.y;
+  const int dx = k / 9 - 1, dy = (k / 3) % 3 - 1, dz = k % 3 - 1;
+  for (int i = threadIdx.x; i < 64 * 9; i += L1T) {
+    const int os = i / 9, q = i % 9, o = os >> 3;
+    const int ox = (o >> 2) - 1, oy = ((o >> 1) & 1) - 1, oz = (o & 1) - 1;
+    const int mx = dx - ox, my = dy - oy, mz = dz - oz;
+    if (mx < 0 || mx > 1 || my < 0 || my > 1 || mz < 0 || mz > 1) continue;
+    qs[os][q] = cQ[(os & 7) * 576 + (3 * corner_of(-ox, -oy, -oz) + q / 3) * 24 + 3 * corner_of(mx, my, mz) + q % 3];
+  }
+  __syncthreads();
+  long long I[L1N];
+  int ix[L1N], iy[L1N], iz[L1N];
+  bool in[L1N], jin[L1N];
+  double B[L1N][9];
 #pragma unroll
-              for (int cc = 0; cc < 3; ++cc)
+  for (int n = 0; n < L1N; ++n) {
+    I[n] = (blockIdx.x * (long long)L1N + n) * L1T + threadIdx.x;
+    in[n] = I[n] < c.nnodes;
+    node_xyz(c, in[n] ? I[n] : 0, ix[n], iy[n], iz[n]);
+    const int jx = ix[n] + dx, jy = iy[n] + dy, jz = iz[n] + dz;
+    jin[n] = in[n] && jx >= 0 && jx < c.NX && jy >= 0 && jy < c.NY && jz >= 0 && jz < c.NZ;
 #pragma unroll
-                for (int dd = 0; dd < 3; ++dd) B[cc * 3 + dd] += Ee * Q[(3 * a + cc) * 24 + 3 * m + dd];
-            }
-          }
-        }
+    for (int q = 0; q < 9; ++q) B[n][q] = 0.0;
+  }
+  for (int o = 0; o < 8; ++o) {
+    const int ox = (o >> 2) - 1, oy = ((o >> 1) & 1) - 1, oz = (o & 1) - 1;
+    const int mx = dx - ox, my = dy - oy, mz = dz - oz;
+    if (mx < 0 || mx > 1 || my < 0 || my > 1 || mz < 0 || mz > 1) continue;  // uniform
+    double Ee[L1N][8];
+#pragma unroll
+    for (int n = 0; n < L1N; ++n) {
+      const int ex = ix[n] + ox, ey = iy[n] + oy, ez = iz[n] + oz;
+      const bool e = jin[n] && ex >= 0 && ex < c.nx && ey >= 0 && ey < c.ny && ez >= 0 && ez < c.nz;
+#pragma unroll
+      for (int stu = 0; stu < 8; ++stu) {
+        const int fx = min(2 * ex + (stu >> 2), f.nx - 1), fy = min(2 * ey + ((stu >> 1) & 1), f.ny - 1),
+                  fz = min(2 * ez + (stu & 1), f.nz - 1);
+        Ee[n][stu] = e ? Ef[((long long)fx * f.ny + fy) * f.nz + fz] : 0.0;
       }
     }
-    const long long J = jin ? (((long long)jx * c.NY + jy) * c.NZ + jz) : 0;
 #pragma unroll
-    for (int cc = 0; cc < 3; ++cc)
+    for (int stu = 0; stu < 8; ++stu) {
+      const double* Q = qs[o * 8 + stu];
+      double qv[9];
 #pragma unroll
-      for (int dd = 0; dd < 3; ++dd) {
-        const bool keep = jin && mc[3 * I + cc] && mc[3 * J + dd];
-        S[(long long)(k * 9 + cc * 3 + dd) * c.nnodes + I] = keep ? B[cc * 3 + dd] : 0.0;
+      for (int q = 0; q < 8; q += 2) {
+        const double2 v = *reinterpret_cast<const double2*>(Q + q);
+        qv[q] = v.x;
+        qv[q + 1] = v.y;
       }
+      qv[8] = Q[8];
+#pragma unroll
+      for (int n = 0; n < L1N; ++n)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) B[n][q] += Ee[n][stu] * qv[q];
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < L1N; ++n) {
+    if (!in[n]) continue;
+    const long long J = jin[n] ? (((long long)(ix[n] + dx) * c.NY + iy[n] + dy) * c.NZ + iz[n] + dz) : 0;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const bool keep = jin[n] && mc[3 * I[n] + q / 3] && mc[3 * J + q % 3];
+      S[(long long)(k * 9 + q) * c.nnodes + I[n]] = keep ? B[n][q] : 0.0;
+    }
   }
 }
 
 void level1_assemble(const Grid& fine, const Grid& coarse, const double* E_f, const uint8_t* mask_c, double* S,
                      cudaStream_t s) {
-  const int bs = 128;
-  k_level1_assemble<<<(unsigned)((coarse.nnodes + bs - 1) / bs), bs, 0, s>>>(fine, coarse, E_f, mask_c, S);
+  const int bs = L1T * L1N;
+  k_level1_assemble<<<dim3((unsigned)((coarse.nnodes + bs - 1) / bs), 27), L1T, 0, s>>>(fine, coarse, E_f, mask_c, S);
   TOPO_LAUNCH_CHECK();
 }
 
 // ---------------------------------------------------------------------- R.A.P
 // K_c = P^T K_f P with the row-normalised trilinear P restricted to free DoFs
-// (multigrid_v4.py:747-751). Block (I, J = I + d) of K_c is
-//   sum_{i, j} P[i,I] P[j,J] K_f[i,j]
-// over fine nodes i = 2I + s, j = 2J + t (s, t in {-1,0,1}^3) that are
-// stencil neighbours (|j - i| <= 1 per dimension). Per dimension that leaves
-// 7 (s, t) pairs for d = 0 and 3 for d = +-1. One thread per (I, d) keeps its
-// 3x3 block in registers; threads of a warp share d (uniform loops) and take
-// consecutive I.
-struct PairList {
-  int n;
-  int s[7], t[7];
+// (multigrid_v4.py:747-751). P is a product of one-dimensional prolongations,
+// and a 27-point stencil stays one under each of them, so the product is formed
+// in three passes, coarsening z, then y, then x. Along the coarsened dimension
+// block (I, J = I + d) sums over the fine pairs i = 2I + s, j = i + e
+// (s, e in {-1,0,1}): node 2I is I's own; 2I+1 belongs to I with weight a and
+// to I+1 with 1/2 (a = 1/2, or 1 where I+1 lies beyond the coarse grid); 2I-1
+// to I-1 and I with 1/2 each. Nine reads give the three blocks d = -1, 0, 1.
+// One thread per (output node, coefficient of the other two dimensions and of
+// the 3x3 block), lanes along z. Couplings to neighbours outside a grid are
+// zero in the input and written as zero. Bound by HBM: level 1 of 160x80x80
+// is read once (265 MB) and the passes write 136, 69 and 35 MB. The direct form
+// (one thread per block over up to 343 pairs) took 1500 us for both levels of
+// that hierarchy, the passes 152 us.
+struct RapDim {
+  int nf, nc;            // fine / coarse elements along the dimension
+  long long inner;       // nodes below it (stride of the dimension)
+  long long outer;       // nodes above it
+  int kstride;           // step of the dimension's offset in k: 9, 3 or 1
 };
 
-__host__ __device__ inline PairList rap_pairs(int d) {
-  PairList p;
-  p.n = 0;
-  for (int s = -1; s <= 1; ++s)
-    for (int t = -1; t <= 1; ++t) {
-      const int gap = 2 * d + t - s;
-      if (gap >= -1 && gap <= 1) {
-        p.s[p.n] = s;
-        p.t[p.n] = t;
-        ++p.n;
-      }
-    }
-  return p;
-}
-
-__global__ void __launch_bounds__(128) k_rap(Grid f, Grid c, const double* __restrict__ Sf, const uint8_t* __restrict__ mc,
-                                             double* __restrict__ Sc) {
-  // CTA b: neighbour offset kd = b % 27 (uniform per CTA) of coarse nodes
-  // [128 (b / 27), +128); the 27 offsets of a node range are adjacent in
-  // launch order, so they read that range's fine coefficients from L2
-  const int kd = (int)(blockIdx.x % 27);
-  const long long I = (long long)(blockIdx.x / 27) * blockDim.x + threadIdx.x;
-  if (I >= c.nnodes) return;
-  int Ix, Iy, Iz;
-  node_xyz(c, I, Ix, Iy, Iz);
-  const int dx = kd / 9 - 1, dy = (kd / 3) % 3 - 1, dz = kd % 3 - 1;
-  const int Jx = Ix + dx, Jy = Iy + dy, Jz = Iz + dz;
-  const bool jin = Jx >= 0 && Jx < c.NX && Jy >= 0 && Jy < c.NY && Jz >= 0 && Jz < c.NZ;
-  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (jin) {
-    const PairList px = rap_pairs(dx), py = rap_pairs(dy), pz = rap_pairs(dz);
-    for (int a = 0; a < px.n; ++a) {
-      const int ix = 2 * Ix + px.s[a], jx = 2 * Jx + px.t[a];
-      if (ix < 0 || ix > f.nx || jx < 0 || jx > f.nx) continue;
-      const double wx = prolong_w1(ix, Ix, c.nx) * prolong_w1(jx, Jx, c.nx);
-      if (wx == 0.0) continue;
-      for (int b = 0; b < py.n; ++b) {
-        const int iy = 2 * Iy + py.s[b], jy = 2 * Jy + py.t[b];
-        if (iy < 0 || iy > f.ny || jy < 0 || jy > f.ny) continue;
-        const double wxy = wx * prolong_w1(iy, Iy, c.ny) * prolong_w1(jy, Jy, c.ny);
-        if (wxy == 0.0) continue;
-        for (int e = 0; e < pz.n; ++e) {
-          const int iz = 2 * Iz + pz.s[e], jz = 2 * Jz + pz.t[e];
-          if (iz < 0 || iz > f.nz || jz < 0 || jz > f.nz) continue;
-          const double w = wxy * prolong_w1(iz, Iz, c.nz) * prolong_w1(jz, Jz, c.nz);
-          if (w == 0.0) continue;
-          const long long i = ((long long)ix * f.NY + iy) * f.NZ + iz;
-          const int kt = (jx - ix + 1) * 9 + (jy - iy + 1) * 3 + (jz - iz + 1);
-          const double* K = Sf + (long long)kt * 9 * f.nnodes + i;
-#pragma unroll
-          for (int q = 0; q < 9; ++q) acc[q] = fma(w, __ldg(K + (long long)q * f.nnodes), acc[q]);
-        }
-      }
-    }
+template <bool MASK>
+__global__ void __launch_bounds__(256) k_rap_dim(RapDim D, const double* __restrict__ Sin, double* __restrict__ Sout, Grid c,
+                                                 const uint8_t* __restrict__ mc) {
+  const long long nin = D.outer * (D.nf + 1) * D.inner, nout = D.outer * (D.nc + 1) * D.inner;
+  const long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (o >= nout) return;
+  const int cq = blockIdx.y;  // (other two offsets) * 9 + coefficient
+  const int q = cq % 9, kk = cq / 9;
+  // k of the middle block (offset 0 along the dimension)
+  const int k0 = D.kstride == 1 ? kk * 3 + 1 : D.kstride == 3 ? (kk / 3) * 9 + 3 + kk % 3 : 9 + kk;
+  const long long in_ = o % D.inner, t = o / D.inner;
+  const int I = (int)(t % (D.nc + 1));
+  const long long out_ = t / (D.nc + 1);
+  const double* base = Sin + (long long)(k0 * 9 + q) * nin + (out_ * (D.nf + 1) + 2 * I) * D.inner + in_;
+  const long long ks = (long long)D.kstride * 9 * nin;
+  const bool h = I + 1 <= D.nc, up = 2 * I + 1 <= D.nf, dn = I >= 1;
+  const double a = h ? 0.5 : 1.0;
+  double m0 = 0.0, mp = 0.0, mm = 0.0, p0 = 0.0, pp = 0.0, pm = 0.0, d0 = 0.0, dp = 0.0, dm = 0.0;
+  if (2 * I <= D.nf) {  // (one fine element: nodes 0 and 1 only)
+    m0 = __ldg(base);
+    mp = __ldg(base + ks);
+    mm = __ldg(base - ks);
   }
-  const long long J = jin ? (((long long)Jx * c.NY + Jy) * c.NZ + Jz) : 0;
+  if (up) {
+    p0 = __ldg(base + D.inner);
+    pp = __ldg(base + D.inner + ks);
+    pm = __ldg(base + D.inner - ks);
+  }
+  if (dn) {
+    d0 = __ldg(base - D.inner);
+    dp = __ldg(base - D.inner + ks);
+    dm = __ldg(base - D.inner - ks);
+  }
+  double r[3];
+  r[1] = m0 + a * mp + 0.5 * mm + a * (pm + a * p0) + 0.5 * (dp + 0.5 * d0);
+  r[2] = h ? 0.5 * mp + a * (0.5 * p0 + pp) : 0.0;
+  r[0] = dn ? 0.5 * mm + 0.5 * (0.5 * d0 + dm) : 0.0;
 #pragma unroll
-  for (int cc = 0; cc < 3; ++cc)
-#pragma unroll
-    for (int dd = 0; dd < 3; ++dd) {
-      const bool keep = jin && mc[3 * I + cc] && mc[3 * J + dd];
-      Sc[(long long)(kd * 9 + cc * 3 + dd) * c.nnodes + I] = keep ? acc[cc * 3 + dd] : 0.0;
+  for (int d = 0; d < 3; ++d) {
+    const int k = k0 + (d - 1) * D.kstride;
+    double v = r[d];
+    if (MASK) {  // last pass: rows and columns of fixed DoFs
+      int ix, iy, iz;
+      node_xyz(c, o, ix, iy, iz);
+      const int jx = ix + k / 9 - 1, jy = iy + (k / 3) % 3 - 1, jz = iz + k % 3 - 1;
+      const bool jin = jx >= 0 && jx < c.NX && jy >= 0 && jy < c.NY && jz >= 0 && jz < c.NZ;
+      const long long J = jin ? ((long long)jx * c.NY + jy) * c.NZ + jz : 0;
+      if (!(jin && mc[3 * o + q / 3] && mc[3 * J + q % 3])) v = 0.0;
     }
+    Sout[(long long)(k * 9 + q) * nout + o] = v;
+  }
 }
 
-void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c,
+// Doubles of scratch the passes need between `fine` and `coarse`.
+long long rap_scratch(const Grid& f, const Grid& c) {
+  return 243LL * ((long long)f.NX * f.NY * c.NZ + (long long)f.NX * c.NY * c.NZ);
+}
+
+void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c, double* scratch,
          cudaStream_t s) {
-  const int bs = 128;
-  k_rap<<<(unsigned)(27 * ((coarse.nnodes + bs - 1) / bs)), bs, 0, s>>>(fine, coarse, S_f, mask_c, S_c);
+  const Grid &f = fine, &c = coarse;
+  double* T1 = scratch;
+  double* T2 = scratch + 243LL * f.NX * f.NY * c.NZ;
+  const RapDim dz{f.nz, c.nz, 1, (long long)f.NX * f.NY, 1}, dy{f.ny, c.ny, c.NZ, f.NX, 3}, dx{f.nx, c.nx, (long long)c.NY * c.NZ, 1, 9};
+  auto nb = [](const RapDim& D) { return dim3((unsigned)((D.outer * (D.nc + 1) * D.inner + 255) / 256), 81); };
+  k_rap_dim<false><<<nb(dz), 256, 0, s>>>(dz, S_f, T1, c, mask_c);
+  TOPO_LAUNCH_CHECK();
+  k_rap_dim<false><<<nb(dy), 256, 0, s>>>(dy, T1, T2, c, mask_c);
+  TOPO_LAUNCH_CHECK();
+  k_rap_dim<true><<<nb(dx), 256, 0, s>>>(dx, T2, S_c, c, mask_c);
   TOPO_LAUNCH_CHECK();
 }
 
@@ -331,24 +364,34 @@ void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* d
   TOPO_LAUNCH_CHECK();
 }
 
-// FP64 setup stencil (coefficient-major) -> packed FP32 / BF16 apply copies.
-__global__ void k_convert(long long nnodes, const double* __restrict__ S, float* __restrict__ S32,
-                          __nv_bfloat16* __restrict__ S16) {
-  const long long total = 27 * nnodes;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const long long k = t / nnodes, n = t - k * nnodes;
+// FP64 setup stencil (coefficient-major) -> packed FP32 / BF16 apply copies:
+// one thread per 3x3 block, its 12 slots written as three vector stores.
+__global__ void __launch_bounds__(256) k_convert(long long nnodes, const double* __restrict__ S, float* __restrict__ S32,
+                                                 __nv_bfloat16* __restrict__ S16) {
+  const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x, k = blockIdx.y;
+  if (n >= nnodes) return;
+  float v[kPack] = {};
 #pragma unroll
-    for (int q = 0; q < kPack; ++q) {
-      const double v = q < 9 ? S[(k * 9 + q) * nnodes + n] : 0.0;
-      if (S32) S32[t * kPack + q] = (float)v;
-      if (S16) S16[t * kPack + q] = __float2bfloat16_rn((float)v);
+  for (int q = 0; q < 9; ++q) v[q] = (float)S[(k * 9 + q) * nnodes + n];
+  const long long t = k * nnodes + n;
+  if (S32) {
+    float4* o = reinterpret_cast<float4*>(S32 + t * kPack);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  }
+  if (S16) {
+    uint2* o = reinterpret_cast<uint2*>(S16 + t * kPack);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v[4 * j], v[4 * j + 1]), hi = __floats2bfloat162_rn(v[4 * j + 2], v[4 * j + 3]);
+      o[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     }
   }
 }
 
 // nnodes: nodes of the level; the apply copies hold 27 * 12 * nnodes values.
 void stencil_convert(long long nnodes, const double* S, float* S32, __nv_bfloat16* S16, cudaStream_t s) {
-  k_convert<<<1184, 256, 0, s>>>(nnodes, S, S32, S16);
+  k_convert<<<dim3((unsigned)((nnodes + 255) / 256), 27), 256, 0, s>>>(nnodes, S, S32, S16);
   TOPO_LAUNCH_CHECK();
 }
 

@@ -57,25 +57,28 @@ __device__ __forceinline__ long long bidx(long long i, long long j, int band, lo
 }
 
 // --------------------------------------------------------------- assembly
+// one thread per (node, neighbour block)
 __global__ void k_band_assemble(Grid g, const double* __restrict__ S, const int* __restrict__ dof_index, int band,
                                 long long ldb, double* __restrict__ A) {
   const long long I = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (I >= g.nnodes) return;
   const int iz = (int)(I % g.NZ), iy = (int)((I / g.NZ) % g.NY), ix = (int)(I / ((long long)g.NZ * g.NY));
+  const int k = blockIdx.y;
+  const int jx = ix + k / 9 - 1, jy = iy + (k / 3) % 3 - 1, jz = iz + k % 3 - 1;
+  if (jx < 0 || jx >= g.NX || jy < 0 || jy >= g.NY || jz < 0 || jz >= g.NZ) return;
+  const long long J = ((long long)jx * g.NY + jy) * g.NZ + jz;
+  int row[3], col[3];
+#pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const int row = dof_index[3 * I + c];
-    if (row < 0) continue;
-    for (int k = 0; k < 27; ++k) {
-      const int jx = ix + k / 9 - 1, jy = iy + (k / 3) % 3 - 1, jz = iz + k % 3 - 1;
-      if (jx < 0 || jx >= g.NX || jy < 0 || jy >= g.NY || jz < 0 || jz >= g.NZ) continue;
-      const long long J = ((long long)jx * g.NY + jy) * g.NZ + jz;
-      for (int d = 0; d < 3; ++d) {
-        const int col = dof_index[3 * J + d];
-        if (col < 0 || col > row || row - col > band) continue;
-        A[bidx(row, col, band, ldb)] = S[(long long)(k * 9 + c * 3 + d) * g.nnodes + I];
-      }
-    }
+    row[c] = dof_index[3 * I + c];
+    col[c] = dof_index[3 * J + c];
   }
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (row[c] >= 0 && col[d] >= 0 && col[d] <= row[c] && row[c] - col[d] <= band)
+        A[bidx(row[c], col[d], band, ldb)] = S[(long long)(k * 9 + c * 3 + d) * g.nnodes + I];
 }
 
 __global__ void k_band_add_diag(int n, int band, long long ldb, double* A, double eps) {
@@ -815,7 +818,7 @@ void coarsest_alloc(CoarsestFactor& f, const CoarsestPlan& p, int band, bool f64
 void coarsest_assemble(CoarsestFactor& f, const Grid& g, const double* S, const int* dof_index, cudaStream_t s) {
   TOPO_CUDA_CHECK(cudaMemsetAsync(f.A, 0, sizeof(double) * (size_t)std::max(f.plan.n, 1) * f.ldb, s));
   const int bs = 128;
-  cst::k_band_assemble<<<(unsigned)((g.nnodes + bs - 1) / bs), bs, 0, s>>>(g, S, dof_index, f.band, f.ldb, f.A);
+  cst::k_band_assemble<<<dim3((unsigned)((g.nnodes + bs - 1) / bs), 27), bs, 0, s>>>(g, S, dof_index, f.band, f.ldb, f.A);
   TOPO_LAUNCH_CHECK();
 }
 

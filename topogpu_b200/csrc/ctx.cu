@@ -184,6 +184,7 @@ struct topo_ctx {
   float* E32 = nullptr;
   uint8_t* nmask0 = nullptr;  // level 0: per-node free bits, bit c = DoF 3n+c (read by the tensor-core K.u)
   double* diag0 = nullptr;
+  double* rap_tmp = nullptr;  // between the passes of R.A.P (sized for levels 1 -> 2, the largest)
   double lam_Emax = NAN;
   bool problem_set = false;
   bool setup_done = false;
@@ -596,7 +597,7 @@ void do_setup(topo_ctx* c, const double* E, cudaStream_t s) {
   for (int l = 1; l < c->n_levels; ++l) {
     Level& Lv = c->L[l];
     if (l == 1) level1_assemble(c->L[0].g, Lv.g, c->E64, Lv.mask, Lv.S64, s);
-    else rap(c->L[l - 1].g, Lv.g, c->L[l - 1].S64, Lv.mask, Lv.S64, s);
+    else rap(c->L[l - 1].g, Lv.g, c->L[l - 1].S64, Lv.mask, Lv.S64, c->rap_tmp, s);
   }
   TOPO_CUDA_CHECK(cudaEventRecord(c->ev_ph[2], s));
   TOPO_CUDA_CHECK(cudaEventRecord(c->ev_ph[3], s));
@@ -1198,6 +1199,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->E32 = c->alloc<float>(g0.nelem);
     c->nmask0 = c->alloc<uint8_t>(g0.nnodes + 16);
     c->diag0 = c->alloc<double>(g0.ndof);
+    if (n_levels > 2) c->rap_tmp = c->alloc<double>(rap_scratch(c->L[1].g, c->L[2].g));
     c->kr = c->valloc(g0.ndof);
     c->kz = c->valloc(g0.ndof);
     c->kp = c->valloc(g0.ndof);

@@ -745,18 +745,34 @@ __global__ void k_stats(long long n, const double* __restrict__ x, double* out4,
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  // the last block adds the partials: thread t those of blocks t, t + 256, ...,
+  // then the same tree as above (a fixed order)
+  double w[4] = {0.0, 0.0, 0.0, 0.0};
+  mn = INFINITY;
+  mx = -INFINITY;
+  for (unsigned b = threadIdx.x; b < nb; b += blockDim.x) {
+    w[0] += __ldcg(red.partials + (size_t)b * 4 + 0);
+    w[1] += __ldcg(red.partials + (size_t)b * 4 + 1);
+    mn = fmin(mn, __ldcg(red.partials + (size_t)b * 4 + 2));
+    mx = fmax(mx, __ldcg(red.partials + (size_t)b * 4 + 3));
+  }
+  mn = warp_min(mn);
+  mx = warp_max(mx);
+  if (lane == 0) {
+    smn[wid] = mn;
+    smx[wid] = mx;
+  }
+  block_sum<4>(w);
   if (threadIdx.x == 0) {
-    double S = 0.0, G = 0.0, MN = INFINITY, MX = -INFINITY;
-    for (unsigned b = 0; b < nb; ++b) {
-      S += __ldcg(red.partials + (size_t)b * 4 + 0);
-      G += __ldcg(red.partials + (size_t)b * 4 + 1);
-      MN = fmin(MN, __ldcg(red.partials + (size_t)b * 4 + 2));
-      MX = fmax(MX, __ldcg(red.partials + (size_t)b * 4 + 3));
+    const int nw = blockDim.x >> 5;
+    for (int k = 0; k < nw; ++k) {
+      mn = fmin(mn, smn[k]);
+      mx = fmax(mx, smx[k]);
     }
-    out4[0] = S / (double)n;
-    out4[1] = MN;
-    out4[2] = MX;
-    out4[3] = 4.0 * (G / (double)n);
+    out4[0] = w[0] / (double)n;
+    out4[1] = mn;
+    out4[2] = mx;
+    out4[3] = 4.0 * (w[1] / (double)n);
     *red.ticket = 0u;
   }
 }

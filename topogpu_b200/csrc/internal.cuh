@@ -246,7 +246,8 @@ void sensitivity(const Grid& g, const void* u, const void* v, bool u_f32, const 
 // coarse levels (coarse.cu): 27-point block stencils S[k*9 + c*3 + d][node]
 void level1_assemble(const Grid& fine, const Grid& coarse, const double* E_f, const uint8_t* mask_c,
                      double* S, cudaStream_t s);
-void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c,
+long long rap_scratch(const Grid& fine, const Grid& coarse);  // doubles
+void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c, double* scratch,
          cudaStream_t s);
 void stencil_apply(Prec p, bool vec64, const Grid& g, const void* S, const void* u, const uint8_t* mask,
                    void* y, Epi epi, const EpiArgs& ea, cudaStream_t s);
