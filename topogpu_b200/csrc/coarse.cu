@@ -25,6 +25,13 @@ __host__ __device__ constexpr int corner_of(int bx, int by, int bz) {
 }
 
 __device__ __forceinline__ void node_xyz(const Grid& g, long long n, int& ix, int& iy, int& iz) {
+  if (g.nnodes < (1LL << 31)) {  // 32-bit division
+    const unsigned u = (unsigned)n, r = u / (unsigned)g.NZ;
+    iz = (int)(u - r * (unsigned)g.NZ);
+    ix = (int)(r / (unsigned)g.NY);
+    iy = (int)(r - (unsigned)ix * (unsigned)g.NY);
+    return;
+  }
   iz = (int)(n % g.NZ);
   iy = (int)((n / g.NZ) % g.NY);
   ix = (int)(n / ((long long)g.NZ * g.NY));
@@ -216,110 +223,128 @@ void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t*
 }
 
 // ------------------------------------------------------------- stencil apply
-template <typename TC>
-__device__ __forceinline__ float coef_f(const TC* p) {
-  if constexpr (sizeof(TC) == 2) return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(p));
-  else return (float)*p;
-}
-
-// Coefficients of block k of node n:
-//  * FP64 (setup copy): S[(k*9 + q) * nnodes + n], q = c*3 + d;
-//  * FP32 / BF16 (apply copies): packed per block, 12 slots (9 used) at
-//    S[(k * nnodes + n) * 12 + q], so a block is three 16-byte (FP32) or
-//    8-byte (BF16) vector loads and a warp reads 32 consecutive blocks.
-constexpr int kPack = 12;
-
-template <typename TC, typename T>
-__device__ __forceinline__ void load_block(const TC* __restrict__ S, int k, long long n, long long nnodes, T (&s)[9]) {
-  if constexpr (sizeof(TC) == 8) {
-    const TC* Sk = S + (long long)(k * 9) * nnodes + n;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) s[q] = (T)Sk[(long long)q * nnodes];
-  } else if constexpr (sizeof(TC) == 4) {
-    const float4* p = reinterpret_cast<const float4*>(S + ((long long)k * nnodes + n) * kPack);
-    const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w;
-    s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
-    s[8] = c.x;
-  } else {
-    const uint2* p = reinterpret_cast<const uint2*>(S + ((long long)k * nnodes + n) * kPack);
-    const uint2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    const uint32_t w[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
-#pragma unroll
-    for (int q = 0; q < 9; ++q) {
-      const uint32_t h = (q & 1) ? (w[q >> 1] & 0xFFFF0000u) : (w[q >> 1] << 16);
-      s[q] = (T)__uint_as_float(h);
-    }
-  }
-}
+// Coefficient q = c*3 + d of block k of node n at S[(k*9 + q) * ns + n], in
+// every precision; ns is the node count (BF16: rounded up to even, because a
+// thread reads the coefficients of two nodes at once).
+//
+// A CTA owns 32 NPT consecutive nodes and has one warp per component c: a
+// thread accumulates row c of its NPT nodes, 81 coefficients each, coalesced
+// over the lanes and fetched a third (9 blocks) ahead of their use. The u
+// values of the nine (dx, dy) runs of nodes around the CTA's are staged once
+// in shared memory (rounded to BF16 there when BF). Couplings to nodes outside
+// the grid are zero, so the run's neighbours in memory stand in for them. The
+// rows meet in shared memory and the epilogue runs in order of the DoFs.
+// The sums of a row are those of a thread per node, in the same order.
+//
+// Bound by HBM / L2 on large levels (243 coefficients per node), by one chain
+// of three fetches on small ones. Against one thread per node (FP32 / BF16
+// blocks padded to 12 coefficients), Chebyshev step, B200: FP64 4,225 nodes
+// 21.9 -> 6.1 us, 30,625 nodes (59 MB of coefficients) 43 -> 18 us; BF16
+// 136,161 nodes (66 MB) 30 -> 26 us.
+template <typename TC, int NPT>
+struct CoefV;
+template <>
+struct CoefV<double, 1> {
+  using V = double;
+};
+template <>
+struct CoefV<float, 1> {
+  using V = float;
+};
+template <>
+struct CoefV<__nv_bfloat16, 2> {
+  using V = uint32_t;
+};
 
 // TC: stencil coefficient type; T: vector type; BF: round u to BF16.
-template <typename TC, typename T, bool BF, Epi EPI>
-__global__ void __launch_bounds__(128)
-k_stencil(Grid g, const TC* __restrict__ S, const T* __restrict__ u, const uint8_t* __restrict__ mask,
+template <typename TC, typename T, bool BF, Epi EPI, int NPT>
+__global__ void __launch_bounds__(96)
+k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ u, const uint8_t* __restrict__ mask,
           EpiDev<T> ep, const KrylovState* st) {
   if (st != nullptr && st->done) return;
-  const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (n >= g.nnodes) return;
-  int ix, iy, iz;
-  node_xyz(g, n, ix, iy, iz);
-  // clamped neighbour coordinates (out-of-grid couplings have zero
-  // coefficients, so any in-grid value serves) and the nine row bases
-  const int jxs[3] = {max(ix - 1, 0), ix, min(ix + 1, g.NX - 1)};
-  const int jys[3] = {max(iy - 1, 0), iy, min(iy + 1, g.NY - 1)};
-  const int jzs[3] = {max(iz - 1, 0), iz, min(iz + 1, g.NZ - 1)};
-  long long rb[9];
+  using V = typename CoefV<TC, NPT>::V;
+  constexpr int NN = 32 * NPT, RUN = 3 * (NN + 2);
+  __shared__ T us[9][RUN];
+  __shared__ T os[3 * NN];
+  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+  const long long n0 = blockIdx.x * (long long)NN, n = n0 + lane * NPT;
+  const bool live = n < g.nnodes;
+  const V* Sp = reinterpret_cast<const V*>(S + (long long)(3 * c) * ns + (live ? n : 0));
+  const long long step = ns / NPT;  // in V
+  V cf[2][27];
+  auto fetch = [&](int dx, V (&w)[27]) {
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
+    for (int k = 0; k < 9; ++k)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) rb[a * 3 + b] = ((long long)jxs[a] * g.NY + jys[b]) * g.NZ;
-  T a0 = 0, a1 = 0, a2 = 0;
+      for (int d = 0; d < 3; ++d) w[3 * k + d] = live ? __ldg(Sp + (long long)((9 * dx + k) * 9 + d) * step) : (V)0;
+  };
+  fetch(0, cf[0]);
+  // nodes n0 - 1 .. n0 + NN of each run, shifted by (dx, dy)
 #pragma unroll
-  for (int k = 0; k < 27; ++k) {
-    long long j = rb[k / 3] + jzs[k % 3];
-    if (!topo_in_range(j, g.nnodes)) j = n;
-    T uj[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      T v = u[3 * j + d];
+  for (int r = 0; r < 9; ++r) {
+    const long long base = 3 * (n0 - 1 + ((long long)(r / 3 - 1) * g.NY + (r % 3 - 1)) * g.NZ);
+    for (int i = threadIdx.x; i < RUN; i += 96) {
+      const long long j = base + i;
+      T v = (j >= 0 && j < g.ndof && topo_in_range(j, g.ndof)) ? u[j] : (T)0;
       if constexpr (BF) v = __bfloat162float(__float2bfloat16_rn((float)v));
-      uj[d] = v;
+      us[r][i] = v;
     }
-    T s[9];
-    load_block<TC, T>(S, k, n, g.nnodes, s);
-    a0 += s[0] * uj[0] + s[1] * uj[1] + s[2] * uj[2];
-    a1 += s[3] * uj[0] + s[4] * uj[1] + s[5] * uj[2];
-    a2 += s[6] * uj[0] + s[7] * uj[1] + s[8] * uj[2];
   }
-  const T acc[3] = {a0, a1, a2};
+  __syncthreads();
+  T a[NPT];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const long long i = 3 * n + c;
-    if (!topo_in_range(i, g.ndof)) continue;
-    epilogue_store<T, EPI>(ep, i, mask[i] != 0, acc[c], u[i]);
+  for (int p = 0; p < NPT; ++p) a[p] = 0;
+#pragma unroll
+  for (int dx = 0; dx < 3; ++dx) {
+    if (dx < 2) fetch(dx + 1, cf[(dx + 1) & 1]);
+    const V(&w)[27] = cf[dx & 1];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+#pragma unroll
+      for (int p = 0; p < NPT; ++p) {
+        const T* uj = &us[3 * dx + k / 3][3 * (lane * NPT + p + k % 3)];
+        T s[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if constexpr (NPT == 2) s[d] = (T)__uint_as_float(p ? (w[3 * k + d] & 0xFFFF0000u) : (w[3 * k + d] << 16));
+          else s[d] = (T)w[3 * k + d];
+        }
+        a[p] += fma(s[2], uj[2], fma(s[0], uj[0], s[1] * uj[1]));
+      }
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < NPT; ++p) os[3 * (lane * NPT + p) + c] = a[p];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NPT; ++q) {
+    const int t = threadIdx.x + 96 * q;
+    const long long i = 3 * n0 + t;
+    if (i < g.ndof && topo_in_range(i, g.ndof)) epilogue_store<T, EPI>(ep, i, mask[i] != 0, os[t], u[i]);
   }
 }
 
 template <typename TC, typename T, bool BF>
 static void launch_stencil(const Grid& g, const void* S, const void* u, const uint8_t* mask, void* y, Epi epi,
                            const EpiArgs& ea, cudaStream_t s) {
-  const int bs = 128;
-  const unsigned nb = (unsigned)((g.nnodes + bs - 1) / bs);
+  constexpr int NPT = sizeof(TC) == 2 ? 2 : 1;
+  const unsigned nb = (unsigned)((g.nnodes + 32 * NPT - 1) / (32 * NPT));
+  const long long ns = NPT == 2 ? stencil16_stride(g.nnodes) : g.nnodes;
   const TC* SS = (const TC*)S;
   const T* uu = (const T*)u;
   const EpiDev<T> ep = make_epi<T>(y, ea);
   switch (epi) {
     case Epi::Store:
-      k_stencil<TC, T, BF, Epi::Store><<<nb, bs, 0, s>>>(g, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::Store, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
       break;
     case Epi::Residual:
-      k_stencil<TC, T, BF, Epi::Residual><<<nb, bs, 0, s>>>(g, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::Residual, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
       break;
     case Epi::ChebR:
-      k_stencil<TC, T, BF, Epi::ChebR><<<nb, bs, 0, s>>>(g, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::ChebR, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
       break;
     case Epi::RUpd:
-      k_stencil<TC, T, BF, Epi::RUpd><<<nb, bs, 0, s>>>(g, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::RUpd, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
       break;
     default:
       throw std::runtime_error("stencil_apply: unsupported epilogue");
@@ -364,34 +389,26 @@ void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* d
   TOPO_LAUNCH_CHECK();
 }
 
-// FP64 setup stencil (coefficient-major) -> packed FP32 / BF16 apply copies:
-// one thread per 3x3 block, its 12 slots written as three vector stores.
-__global__ void __launch_bounds__(256) k_convert(long long nnodes, const double* __restrict__ S, float* __restrict__ S32,
+// FP64 setup stencil -> FP32 / BF16 apply copies in the same order.
+__global__ void __launch_bounds__(256) k_convert(long long nnodes, long long ns16, const double* __restrict__ S, float* __restrict__ S32,
                                                  __nv_bfloat16* __restrict__ S16) {
-  const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x, k = blockIdx.y;
+  const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (n >= nnodes) return;
-  float v[kPack] = {};
 #pragma unroll
-  for (int q = 0; q < 9; ++q) v[q] = (float)S[(k * 9 + q) * nnodes + n];
-  const long long t = k * nnodes + n;
-  if (S32) {
-    float4* o = reinterpret_cast<float4*>(S32 + t * kPack);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) o[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-  }
-  if (S16) {
-    uint2* o = reinterpret_cast<uint2*>(S16 + t * kPack);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const __nv_bfloat162 lo = __floats2bfloat162_rn(v[4 * j], v[4 * j + 1]), hi = __floats2bfloat162_rn(v[4 * j + 2], v[4 * j + 3]);
-      o[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-    }
+  for (int q = 0; q < 9; ++q) {
+    const long long k = blockIdx.y * 9LL + q;
+    const float v = (float)S[k * nnodes + n];
+    if (S32) S32[k * nnodes + n] = v;
+    if (S16) S16[k * ns16 + n] = __float2bfloat16_rn(v);
   }
 }
 
-// nnodes: nodes of the level; the apply copies hold 27 * 12 * nnodes values.
+long long stencil16_stride(long long nnodes) { return (nnodes + 1) & ~1LL; }
+
+// nnodes: nodes of the level; the copies hold 243 nnodes (S16: 243
+// stencil16_stride(nnodes)) values.
 void stencil_convert(long long nnodes, const double* S, float* S32, __nv_bfloat16* S16, cudaStream_t s) {
-  k_convert<<<dim3((unsigned)((nnodes + 255) / 256), 27), 256, 0, s>>>(nnodes, S, S32, S16);
+  k_convert<<<dim3((unsigned)((nnodes + 255) / 256), 27), 256, 0, s>>>(nnodes, stencil16_stride(nnodes), S, S32, S16);
   TOPO_LAUNCH_CHECK();
 }
 
@@ -417,94 +434,95 @@ void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_
   TOPO_LAUNCH_CHECK();
 }
 
-// r_c = mask_c * P^T r_f
+// r_c = mask_c * P^T r_f: one thread per coarse DoF, its 27 reads issued
+// together (missing ones have weight zero). With `compact` (the coarsest
+// level) the value of free DoF i also goes to compact[index[i]] in FP64, the
+// right-hand side of the coarsest solve. Latency bound on small levels: one
+// thread per node over three nested loops took 7.5 us there, this RESTRICT_US.
 template <typename T>
-__global__ void k_restrict(Grid f, Grid c, const T* __restrict__ rf, const uint8_t* __restrict__ mc,
-                           T* __restrict__ rc, const KrylovState* st) {
+__global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* __restrict__ rf, const uint8_t* __restrict__ mc,
+                                                  T* __restrict__ rc, const int* __restrict__ index, double* __restrict__ compact,
+                                                  const KrylovState* st) {
   if (st != nullptr && st->done) return;
-  const long long I = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (I >= c.nnodes) return;
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= c.ndof) return;
+  const long long I = i / 3;
+  const int d = (int)(i - 3 * I);
   int Ix, Iy, Iz;
   node_xyz(c, I, Ix, Iy, Iz);
-  T a[3] = {0, 0, 0};
-  for (int sx = -1; sx <= 1; ++sx) {
-    const int ix = 2 * Ix + sx;
-    if (ix < 0 || ix > f.nx) continue;
-    const T wx = (T)prolong_w1(ix, Ix, c.nx);
-    if (wx == (T)0) continue;
-    for (int sy = -1; sy <= 1; ++sy) {
-      const int iy = 2 * Iy + sy;
-      if (iy < 0 || iy > f.ny) continue;
-      const T wy = (T)prolong_w1(iy, Iy, c.ny);
-      if (wy == (T)0) continue;
-      for (int sz = -1; sz <= 1; ++sz) {
-        const int iz = 2 * Iz + sz;
-        if (iz < 0 || iz > f.nz) continue;
-        const T wz = (T)prolong_w1(iz, Iz, c.nz);
-        if (wz == (T)0) continue;
-        const T w = wx * wy * wz;
-        const long long i = ((long long)ix * f.NY + iy) * f.NZ + iz;
-        if (!topo_in_range(i, f.nnodes)) continue;
-        a[0] += w * rf[3 * i];
-        a[1] += w * rf[3 * i + 1];
-        a[2] += w * rf[3 * i + 2];
-      }
-    }
-  }
+  T wx[3], wy[3], wz[3];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) rc[3 * I + d] = mc[3 * I + d] ? a[d] : (T)0;
+  for (int s = 0; s < 3; ++s) {
+    const int x = 2 * Ix + s - 1, y = 2 * Iy + s - 1, z = 2 * Iz + s - 1;
+    wx[s] = (x < 0 || x > f.nx) ? (T)0 : (T)prolong_w1(x, Ix, c.nx);
+    wy[s] = (y < 0 || y > f.ny) ? (T)0 : (T)prolong_w1(y, Iy, c.ny);
+    wz[s] = (z < 0 || z > f.nz) ? (T)0 : (T)prolong_w1(z, Iz, c.nz);
+  }
+  T v[27];
+#pragma unroll
+  for (int k = 0; k < 27; ++k) {
+    const T w = wx[k / 9] * wy[(k / 3) % 3] * wz[k % 3];
+    const long long n = ((long long)(2 * Ix + k / 9 - 1) * f.NY + (2 * Iy + (k / 3) % 3 - 1)) * f.NZ + (2 * Iz + k % 3 - 1);
+    v[k] = (w != (T)0 && topo_in_range(n, f.nnodes)) ? rf[3 * n + d] : (T)0;
+  }
+  T a = 0;
+#pragma unroll
+  for (int k = 0; k < 27; ++k) a += (wx[k / 9] * wy[(k / 3) % 3] * wz[k % 3]) * v[k];
+  const T r = mc[i] ? a : (T)0;
+  rc[i] = r;
+  if (compact != nullptr && index[i] >= 0) compact[index[i]] = (double)r;
 }
 
 void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc, void* rc,
-                  const KrylovState* st, cudaStream_t s) {
+                  const int* index, double* compact, const KrylovState* st, cudaStream_t s) {
   const int bs = 128;
-  const unsigned nb = (unsigned)((coarse.nnodes + bs - 1) / bs);
+  const unsigned nb = (unsigned)((coarse.ndof + bs - 1) / bs);
   if (vec64)
-    k_restrict<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)rf, mc, (double*)rc, st);
+    k_restrict<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st);
   else
-    k_restrict<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)rf, mc, (float*)rc, st);
+    k_restrict<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st);
   TOPO_LAUNCH_CHECK();
 }
 
-// x_f += mask_f * P e_c
+// x_f += mask_f * P e_c: one thread per fine DoF, its (at most) eight reads
+// issued together.
 template <typename T>
-__global__ void k_prolong_add(Grid f, Grid c, const T* __restrict__ ec, const uint8_t* __restrict__ mf,
-                              T* __restrict__ xf, T* __restrict__ e_out, const KrylovState* st) {
+__global__ void __launch_bounds__(256) k_prolong_add(Grid f, Grid c, const T* __restrict__ ec, const uint8_t* __restrict__ mf,
+                                                     T* __restrict__ xf, T* __restrict__ e_out, const KrylovState* st) {
   if (st != nullptr && st->done) return;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= f.nnodes) return;
+  if (i >= f.ndof) return;
+  const long long n = i / 3;
+  const int d = (int)(i - 3 * n);
   int ix, iy, iz;
-  node_xyz(f, i, ix, iy, iz);
-  T a[3] = {0, 0, 0};
-  const int px0 = ix >> 1, px1 = (ix & 1) ? px0 + 1 : px0;
-  const int py0 = iy >> 1, py1 = (iy & 1) ? py0 + 1 : py0;
-  const int pz0 = iz >> 1, pz1 = (iz & 1) ? pz0 + 1 : pz0;
-  for (int Jx = px0; Jx <= min(px1, c.nx); ++Jx) {
-    const T wx = (T)prolong_w1(ix, Jx, c.nx);
-    for (int Jy = py0; Jy <= min(py1, c.ny); ++Jy) {
-      const T wy = (T)prolong_w1(iy, Jy, c.ny);
-      for (int Jz = pz0; Jz <= min(pz1, c.nz); ++Jz) {
-        const T w = wx * wy * (T)prolong_w1(iz, Jz, c.nz);
-        const long long J = ((long long)Jx * c.NY + Jy) * c.NZ + Jz;
-        if (!topo_in_range(J, c.nnodes)) continue;
-        a[0] += w * ec[3 * J];
-        a[1] += w * ec[3 * J + 1];
-        a[2] += w * ec[3 * J + 2];
-      }
-    }
-  }
+  node_xyz(f, n, ix, iy, iz);
+  const bool fr = mf[i] != 0;
+  const T x = xf[i];
+  const int px = ix >> 1, py = iy >> 1, pz = iz >> 1;
+  // weights of the lower and upper parent (none: zero)
+  const bool hx = (ix & 1) && px + 1 <= c.nx, hy = (iy & 1) && py + 1 <= c.ny, hz = (iz & 1) && pz + 1 <= c.nz;
+  const T wx[2] = {hx ? (T)0.5 : (T)1, hx ? (T)0.5 : (T)0};
+  const T wy[2] = {hy ? (T)0.5 : (T)1, hy ? (T)0.5 : (T)0};
+  const T wz[2] = {hz ? (T)0.5 : (T)1, hz ? (T)0.5 : (T)0};
+  T v[8];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const T v = mf[3 * i + d] ? a[d] : (T)0;
-    xf[3 * i + d] += v;
-    if (e_out) e_out[3 * i + d] = v;
+  for (int k = 0; k < 8; ++k) {
+    const bool in = (!(k & 4) || hx) && (!(k & 2) || hy) && (!(k & 1) || hz);
+    const long long J = ((long long)(px + (k >> 2)) * c.NY + py + ((k >> 1) & 1)) * c.NZ + pz + (k & 1);
+    v[k] = (in && topo_in_range(J, c.nnodes)) ? ec[3 * J + d] : (T)0;
   }
+  T a = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) a += (wx[k >> 2] * wy[(k >> 1) & 1] * wz[k & 1]) * v[k];
+  const T e = fr ? a : (T)0;
+  xf[i] = x + e;
+  if (e_out) e_out[i] = e;
 }
 
 void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* ec, const uint8_t* mf, void* xf,
                  void* e_out, const KrylovState* st, cudaStream_t s) {
-  const int bs = 128;
-  const unsigned nb = (unsigned)((fine.nnodes + bs - 1) / bs);
+  const int bs = 256;
+  const unsigned nb = (unsigned)((fine.ndof + bs - 1) / bs);
   if (vec64)
     k_prolong_add<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)ec, mf, (double*)xf, (double*)e_out, st);
   else

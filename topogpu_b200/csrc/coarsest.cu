@@ -637,20 +637,9 @@ __global__ void __launch_bounds__(256) k_couplings(int band, long long ldb, cons
 // starts 16-byte aligned), FP64 accumulation, the RW partial sums added
 // through shared memory. With four warps per row one block
 // (about 4 band rows) is a single short wave, so the 2P dependent launches of
-// an apply cost about 5 us each. The compact right-hand side is gathered
-// once; both passes read the compact vectors through L1.
+// an apply cost about 5 us each. The restriction to the coarsest level writes
+// the compact right-hand side; both passes read the compact vectors through L1.
 constexpr int RW = 4;  // warps per row
-
-template <typename T>
-__global__ void k_coarse_gather(int n, long long nfull, const int* __restrict__ free_list, const T* __restrict__ rhs,
-                                double* __restrict__ rc, const KrylovState* st) {
-  if (st != nullptr && st->done) return;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < n) {
-    const int f = free_list[j];
-    rc[j] = topo_in_range(f, nfull) ? (double)rhs[f] : 0.0;
-  }
-}
 
 // One warp's share of sum_{j in [lo, hi)} Ci[j] v[j] over a row segment:
 // chunks c = sub, sub+RW, ... of 32 lanes x one 16-byte load, four chunks in
@@ -884,10 +873,9 @@ int coarsest_status(CoarsestFactor& f, cudaStream_t s) {
 }
 
 // work: 2n doubles (y, then the compact right-hand side, overwritten by the
-// compact solution in the second pass).
+// compact solution in the second pass). Only the free DoFs of x are written.
 template <typename T, typename TX>
-static void apply_blocks(const CoarsestFactor& f, const T* rhs, double* work, T* x, const KrylovState* st,
-                         cudaStream_t s) {
+static void apply_blocks(const CoarsestFactor& f, double* work, T* x, const KrylovState* st, cudaStream_t s) {
   const CoarsestPlan& p = f.plan;
   const CoarseBlocks& bk = f.blk;
   const int n = p.n;
@@ -895,8 +883,6 @@ static void apply_blocks(const CoarsestFactor& f, const T* rhs, double* work, T*
   double* y = work;
   double* rc = work + n;
   const TX* C = (const TX*)f.C;
-  cst::k_coarse_gather<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, p.nfull, f.d_free, rhs, rc, st);
-  TOPO_LAUNCH_CHECK();
   for (int q = 0; q < bk.P; ++q) {
     const int m = bk.b[q + 1] - bk.b[q];
     cst::k_coarse_lower<TX><<<(unsigned)((m + rpb - 1) / rpb), 256, 0, s>>>(
@@ -912,16 +898,15 @@ static void apply_blocks(const CoarsestFactor& f, const T* rhs, double* work, T*
   }
 }
 
-void coarsest_apply(const CoarsestFactor& f, bool vec64, const void* rhs, double* work, void* x, const KrylovState* st,
-                    cudaStream_t s) {
+void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s) {
   if (f.plan.n == 0) return;
   if (vec64) {
     if (!f.f64) throw std::runtime_error("coarsest apply: FP64 vectors need the FP64 inverse");
-    apply_blocks<double, double>(f, (const double*)rhs, work, (double*)x, st, s);
+    apply_blocks<double, double>(f, work, (double*)x, st, s);
   } else if (f.f64) {
-    apply_blocks<float, double>(f, (const float*)rhs, work, (float*)x, st, s);
+    apply_blocks<float, double>(f, work, (float*)x, st, s);
   } else {
-    apply_blocks<float, float>(f, (const float*)rhs, work, (float*)x, st, s);
+    apply_blocks<float, float>(f, work, (float*)x, st, s);
   }
 }
 

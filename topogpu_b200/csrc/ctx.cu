@@ -83,12 +83,6 @@ __global__ void k_mask_to(long long n, const uint8_t* __restrict__ m, T* __restr
     v[i] = m[i] ? (random ? (T)hashed_unit((unsigned long long)i) : (T)1) : (T)0;
 }
 
-template <typename T>
-__global__ void k_gather_zero(long long n_full, T* __restrict__ x) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n_full; i += (long long)gridDim.x * blockDim.x)
-    x[i] = 0;
-}
-
 // Per-node free bits from the per-DoF mask: bit c set <=> DoF 3n+c is free.
 __global__ void k_node_mask(long long nnodes, const uint8_t* __restrict__ mask, uint8_t* __restrict__ nmask) {
   for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nnodes; n += (long long)gridDim.x * blockDim.x)
@@ -288,12 +282,18 @@ Prec hi_prec(const Level& Lv) { return Lv.prec == Prec::BF16 ? Prec::F32 : Lv.pr
 // operator only ever multiplies a direction. from_zero: x = 0 and r = b.
 // want_residual: also form the final residual r = b - K x (one more
 // application, which replaces the reference's separate residual matvec).
-void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const KrylovState* st, bool same_bits, cudaStream_t s) {
-  Level& Lv = c->L[l];
+// started: the first step (direction Lv.d) has been taken by the kernel before.
+Cheb level_cheb(const topo_ctx* c, const Level& Lv) {
   const double lam = (std::isfinite(Lv.lam) ? Lv.lam : 1.0) * c->lam_safety;
-  const Cheb ch = make_cheb(lam, c->cheb_lower, Lv.degree, c->cheb_form);
+  return make_cheb(lam, c->cheb_lower, Lv.degree, c->cheb_form);
+}
+
+void smooth(topo_ctx* c, int l, bool from_zero, bool started, bool want_residual, const KrylovState* st, bool same_bits,
+            cudaStream_t s) {
+  Level& Lv = c->L[l];
+  const Cheb ch = level_cheb(c, Lv);
   const long long n = Lv.g.ndof;
-  cheb_start(c->vec64, n, from_zero ? Lv.b : nullptr, Lv.r, Lv.dinv, ch.c2[0], ch.ax[0], Lv.x, Lv.d, from_zero, st,
+  if (!started) cheb_start(c->vec64, n, from_zero ? Lv.b : nullptr, Lv.r, Lv.dinv, ch.c2[0], ch.ax[0], Lv.x, Lv.d, from_zero, st,
              s);
   void* dcur = Lv.d;
   void* dnext = Lv.d2;
@@ -320,15 +320,11 @@ void smooth(topo_ctx* c, int l, bool from_zero, bool want_residual, const Krylov
   }
 }
 
+// The compact right-hand side was written by the restriction to this level;
+// x is zero at the fixed DoFs (topo_set_problem) and written at the free ones.
 void coarsest_solve(topo_ctx* c, const KrylovState* st, cudaStream_t s) {
-  const int l = c->n_levels - 1;
-  Level& Lv = c->L[l];
-  const long long n_full = Lv.g.ndof;
-  if (c->vec64) k_gather_zero<double><<<gblocks(n_full), 256, 0, s>>>(n_full, (double*)Lv.x);
-  else k_gather_zero<float><<<gblocks(n_full), 256, 0, s>>>(n_full, (float*)Lv.x);
-  TOPO_LAUNCH_CHECK();
   if (c->C.n == 0) return;
-  coarsest_apply(c->C.cur.f, c->vec64, Lv.b, c->C.y, Lv.x, st, s);
+  coarsest_apply(c->C.cur.f, c->vec64, c->C.y, c->L[c->n_levels - 1].x, st, s);
 }
 
 // One V-cycle (cycle_gamma 1, multigrid_v4.py:986-1008) or W-cycle
@@ -339,26 +335,41 @@ void coarsest_solve(topo_ctx* c, const KrylovState* st, cudaStream_t s) {
 void vcycle(topo_ctx* c, int l, const KrylovState* st, bool same_bits, cudaStream_t s) {
   Level& Lv = c->L[l];
   if (l == c->n_levels - 1) {
-    if (c->n_levels == 1) smooth(c, 0, true, false, st, same_bits, s);
+    if (c->n_levels == 1) smooth(c, 0, true, false, false, st, same_bits, s);
     else coarsest_solve(c, st, s);
     return;
   }
-  smooth(c, l, true, true, st, same_bits, s);  // x = S b, r = b - K x
+  smooth(c, l, true, false, true, st, same_bits, s);  // x = S b, r = b - K x
   Level& Lc = c->L[l + 1];
   for (int k = 0; k < c->cycle_gamma; ++k) {
-    restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, Lc.b, st, s);
+    const bool bottom = l + 1 == c->n_levels - 1;
+    restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, Lc.b, bottom ? c->C.dof_index : nullptr,
+                 bottom ? c->C.y + std::max(c->C.n, 1) : nullptr, st, s);
     vcycle(c, l + 1, st, same_bits, s);
     prolong_add(c->vec64, Lv.g, Lc.g, Lc.x, Lv.mask, Lv.x, Lv.e, st, s);  // x += e = P x_c
     EpiArgs ea{};
     ea.r = Lv.r;
     ea.s = 1.0;
     ea.st = const_cast<KrylovState*>(st);
+    Epi epi = Epi::RUpd;
+    if (k + 1 == c->cycle_gamma) {
+      // the post-smoother's first step d = c2 D^-1 r, x += ax d in the same
+      // kernel (a Chebyshev step without the previous direction)
+      const Cheb ch = level_cheb(c, Lv);
+      epi = Epi::ChebR;
+      ea.dinv = Lv.dinv;
+      ea.x = Lv.x;
+      ea.d_out = Lv.d;
+      ea.c1 = 0.0;
+      ea.c2 = ch.c2[0];
+      ea.ax = ch.ax[0];
+    }
     // r -= K e in FP32 even where the level's operator is BF16: the
     // post-smoother continues from this recursive residual, and BF16 here
     // raised the PCG iterations of the 1M-element cantilever from ~18 to ~95
-    op_apply(c, l, hi_prec(Lv), Lv.e, nullptr, Epi::RUpd, ea, same_bits, s);  // r -= K e
+    op_apply(c, l, hi_prec(Lv), Lv.e, nullptr, epi, ea, same_bits, s);  // r -= K e
   }
-  smooth(c, l, false, false, st, same_bits, s);
+  smooth(c, l, false, true, false, st, same_bits, s);
 }
 
 void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cudaStream_t s, bool same_bits = false) {
@@ -1189,8 +1200,8 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
       if (l >= 1) {
         Lv.S64 = c->alloc<double>(243LL * Lv.g.nnodes);
         if (l < n_levels - 1) {
-          if (Lv.prec != Prec::F64) Lv.S32 = c->alloc<float>(27LL * 12 * Lv.g.nnodes);
-          if (Lv.prec == Prec::BF16) Lv.S16 = c->alloc<__nv_bfloat16>(27LL * 12 * Lv.g.nnodes);
+          if (Lv.prec != Prec::F64) Lv.S32 = c->alloc<float>(243LL * Lv.g.nnodes);
+          if (Lv.prec == Prec::BF16) Lv.S16 = c->alloc<__nv_bfloat16>(243LL * stencil16_stride(Lv.g.nnodes));
         }
       }
     }
@@ -1343,6 +1354,7 @@ int topo_set_problem(topo_ctx* c, const uint8_t* free_mask, const double* F, voi
           alloc_slot(c, c->C.nxt);
         }
       }
+      TOPO_CUDA_CHECK(cudaMemsetAsync(Lc.x, 0, c->vsize() * Lc.g.ndof, s));
       TOPO_CUDA_CHECK(cudaMemcpyAsync(c->C.dof_index, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, s));
       TOPO_CUDA_CHECK(cudaMemcpyAsync(c->C.free_list, fl.data(), sizeof(int) * std::max<size_t>(fl.size(), 1),
                                       cudaMemcpyHostToDevice, s));

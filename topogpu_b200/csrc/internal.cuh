@@ -253,11 +253,12 @@ void stencil_apply(Prec p, bool vec64, const Grid& g, const void* S, const void*
                    void* y, Epi epi, const EpiArgs& ea, cudaStream_t s);
 void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* dinv64, float* dinv32,
                   cudaStream_t s);
-// FP64 coefficient-major stencil -> packed FP32 / BF16 apply copies (27*12 values per node)
+// FP64 stencil -> FP32 / BF16 apply copies in the same order (BF16: node stride rounded up to even)
+long long stencil16_stride(long long nnodes);
 void stencil_convert(long long nnodes, const double* S, float* S32, __nv_bfloat16* S16, cudaStream_t s);
 void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_t* mc, cudaStream_t s);
 void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc,
-                  void* rc, const KrylovState* st, cudaStream_t s);
+                  void* rc, const int* index, double* compact, const KrylovState* st, cudaStream_t s);
 // x_f += e = mask_f * P e_c ; e is also written to e_out when not null
 void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* ec, const uint8_t* mf,
                  void* xf, void* e_out, const KrylovState* st, cudaStream_t s);
@@ -310,8 +311,8 @@ void coarsest_assemble(CoarsestFactor& f, const Grid& g, const double* S, const 
 void coarsest_regularise(CoarsestFactor& f, double* dtmp, cudaStream_t s);
 void coarsest_factor(CoarsestFactor& f, cudaStream_t s);
 int coarsest_status(CoarsestFactor& f, cudaStream_t s);
-void coarsest_apply(const CoarsestFactor& f, bool vec64, const void* rhs, double* work, void* x, const KrylovState* st,
-                    cudaStream_t s);
+// work: 2n doubles, the right-hand side (compact) in the second half
+void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s);
 
 // block PCG kernels (blockops.cu): FP64 column blocks as pointer lists
 void set_ke_block(const double* KE_host);
