@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nel,levels", [((6, 6, 6), 3), ((14, 6, 6), 3), ((13, 9, 7), 3), ((62, 2, 2), 3), ((9, 3, 20), 3),
-                                        ((30, 14, 2), 3), ((2, 2, 62), 3), ((4, 30, 4), 4)])
+                                        ((30, 14, 2), 3), ((2, 2, 62), 3), ((4, 30, 4), 3)])
 def test_level_spectral_bound(cuda_dev, nel, levels):
     import torch
 
