@@ -257,15 +257,19 @@ struct CoefV<__nv_bfloat16, 2> {
 };
 
 // TC: stencil coefficient type; T: vector type; BF: round u to BF16.
-template <typename TC, typename T, bool BF, Epi EPI, int NPT>
+// NV columns (vs entries apart) share the coefficients a thread has fetched;
+// blockIdx.y is the group of NV columns (of nv).
+template <typename TC, typename T, bool BF, Epi EPI, int NPT, int NV>
 __global__ void __launch_bounds__(96)
 k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ u, const uint8_t* __restrict__ mask,
-          EpiDev<T> ep, const KrylovState* st) {
+          EpiDev<T> ep, const KrylovState* st, int nv, long long vs) {
   if (st != nullptr && st->done) return;
   using V = typename CoefV<TC, NPT>::V;
   constexpr int NN = 32 * NPT, RUN = 3 * (NN + 2);
-  __shared__ T us[9][RUN];
-  __shared__ T os[3 * NN];
+  __shared__ T us[NV][9][RUN];
+  __shared__ T os[NV][3 * NN];
+  const int v0 = NV > 1 ? blockIdx.y * NV : 0, nc = NV > 1 ? min(NV, nv - v0) : 1;
+  u += v0 * vs;
   const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
   const long long n0 = blockIdx.x * (long long)NN, n = n0 + lane * NPT;
   const bool live = n < g.nnodes;
@@ -285,15 +289,21 @@ k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ 
     const long long base = 3 * (n0 - 1 + ((long long)(r / 3 - 1) * g.NY + (r % 3 - 1)) * g.NZ);
     for (int i = threadIdx.x; i < RUN; i += 96) {
       const long long j = base + i;
-      T v = (j >= 0 && j < g.ndof && topo_in_range(j, g.ndof)) ? u[j] : (T)0;
-      if constexpr (BF) v = __bfloat162float(__float2bfloat16_rn((float)v));
-      us[r][i] = v;
+      const bool in = j >= 0 && j < g.ndof && topo_in_range(j, g.ndof);
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        T v = (in && q < nc) ? u[q * vs + j] : (T)0;
+        if constexpr (BF) v = __bfloat162float(__float2bfloat16_rn((float)v));
+        us[q][r][i] = v;
+      }
     }
   }
   __syncthreads();
-  T a[NPT];
+  T a[NV][NPT];
 #pragma unroll
-  for (int p = 0; p < NPT; ++p) a[p] = 0;
+  for (int q = 0; q < NV; ++q)
+#pragma unroll
+    for (int p = 0; p < NPT; ++p) a[q][p] = 0;
 #pragma unroll
   for (int dx = 0; dx < 3; ++dx) {
     if (dx < 2) fetch(dx + 1, cf[(dx + 1) & 1]);
@@ -302,49 +312,67 @@ k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ 
     for (int k = 0; k < 9; ++k) {
 #pragma unroll
       for (int p = 0; p < NPT; ++p) {
-        const T* uj = &us[3 * dx + k / 3][3 * (lane * NPT + p + k % 3)];
         T s[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           if constexpr (NPT == 2) s[d] = (T)__uint_as_float(p ? (w[3 * k + d] & 0xFFFF0000u) : (w[3 * k + d] << 16));
           else s[d] = (T)w[3 * k + d];
         }
-        a[p] += fma(s[2], uj[2], fma(s[0], uj[0], s[1] * uj[1]));
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          const T* uj = &us[q][3 * dx + k / 3][3 * (lane * NPT + p + k % 3)];
+          a[q][p] += fma(s[2], uj[2], fma(s[0], uj[0], s[1] * uj[1]));
+        }
       }
     }
   }
 #pragma unroll
-  for (int p = 0; p < NPT; ++p) os[3 * (lane * NPT + p) + c] = a[p];
+  for (int q = 0; q < NV; ++q)
+#pragma unroll
+    for (int p = 0; p < NPT; ++p) os[q][3 * (lane * NPT + p) + c] = a[q][p];
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < NPT; ++q) {
-    const int t = threadIdx.x + 96 * q;
-    const long long i = 3 * n0 + t;
-    if (i < g.ndof && topo_in_range(i, g.ndof)) epilogue_store<T, EPI>(ep, i, mask[i] != 0, os[t], u[i]);
+  for (int q = 0; q < NV; ++q) {
+    if (q >= nc) break;
+    const long long co = (v0 + q) * vs;
+    EpiDev<T> e = ep;
+    if constexpr (EPI == Epi::Store || EPI == Epi::Residual) e.y += co;
+    if constexpr (EPI == Epi::Residual) e.b += co;
+    if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) e.r += co;
+    if constexpr (EPI == Epi::ChebR) {
+      e.x += co;
+      e.d_out += co;
+    }
+#pragma unroll
+    for (int h = 0; h < NPT; ++h) {
+      const int t = threadIdx.x + 96 * h;
+      const long long i = 3 * n0 + t;
+      if (i < g.ndof && topo_in_range(i, g.ndof)) epilogue_store<T, EPI>(e, i, mask[i] != 0, os[q][t], u[q * vs + i]);
+    }
   }
 }
 
-template <typename TC, typename T, bool BF>
+template <typename TC, typename T, bool BF, int NV>
 static void launch_stencil(const Grid& g, const void* S, const void* u, const uint8_t* mask, void* y, Epi epi,
-                           const EpiArgs& ea, cudaStream_t s) {
+                           const EpiArgs& ea, cudaStream_t s, int nv, long long vs) {
   constexpr int NPT = sizeof(TC) == 2 ? 2 : 1;
-  const unsigned nb = (unsigned)((g.nnodes + 32 * NPT - 1) / (32 * NPT));
+  const dim3 nb((unsigned)((g.nnodes + 32 * NPT - 1) / (32 * NPT)), (unsigned)((nv + NV - 1) / NV));
   const long long ns = NPT == 2 ? stencil16_stride(g.nnodes) : g.nnodes;
   const TC* SS = (const TC*)S;
   const T* uu = (const T*)u;
   const EpiDev<T> ep = make_epi<T>(y, ea);
   switch (epi) {
     case Epi::Store:
-      k_stencil<TC, T, BF, Epi::Store, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::Store, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::Residual:
-      k_stencil<TC, T, BF, Epi::Residual, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::Residual, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::ChebR:
-      k_stencil<TC, T, BF, Epi::ChebR, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::ChebR, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::RUpd:
-      k_stencil<TC, T, BF, Epi::RUpd, NPT><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st);
+      k_stencil<TC, T, BF, Epi::RUpd, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     default:
       throw std::runtime_error("stencil_apply: unsupported epilogue");
@@ -352,18 +380,27 @@ static void launch_stencil(const Grid& g, const void* S, const void* u, const ui
   TOPO_LAUNCH_CHECK();
 }
 
+// Columns that share one fetch of the coefficients (static shared memory: FP64 4 x 8.1 KB).
+constexpr int kStencilCols = 4;
+
 void stencil_apply(Prec p, bool vec64, const Grid& g, const void* S, const void* u, const uint8_t* mask, void* y,
-                   Epi epi, const EpiArgs& ea, cudaStream_t s) {
+                   Epi epi, const EpiArgs& ea, cudaStream_t s, int nv, long long vs) {
+#define TOPO_STENCIL(TC, T, BF)                                                            \
+  do {                                                                                     \
+    if (nv > 1) launch_stencil<TC, T, BF, kStencilCols>(g, S, u, mask, y, epi, ea, s, nv, vs); \
+    else launch_stencil<TC, T, BF, 1>(g, S, u, mask, y, epi, ea, s, 1, 0);                 \
+  } while (0)
   if (vec64) {
     if (p != Prec::F64) throw std::runtime_error("stencil_apply: FP64 vectors need an FP64 stencil");
-    launch_stencil<double, double, false>(g, S, u, mask, y, epi, ea, s);
+    TOPO_STENCIL(double, double, false);
   } else if (p == Prec::F32) {
-    launch_stencil<float, float, false>(g, S, u, mask, y, epi, ea, s);
+    TOPO_STENCIL(float, float, false);
   } else if (p == Prec::BF16) {
-    launch_stencil<__nv_bfloat16, float, true>(g, S, u, mask, y, epi, ea, s);
+    TOPO_STENCIL(__nv_bfloat16, float, true);
   } else {
-    launch_stencil<double, float, false>(g, S, u, mask, y, epi, ea, s);
+    throw std::runtime_error("stencil_apply: FP32 vectors need an FP32 or BF16 stencil");
   }
+#undef TOPO_STENCIL
 }
 
 // Jacobi inverse diagonal from the centre block (k = 13), with the
@@ -442,8 +479,11 @@ void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_
 template <typename T>
 __global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* __restrict__ rf, const uint8_t* __restrict__ mc,
                                                   T* __restrict__ rc, const int* __restrict__ index, double* __restrict__ compact,
-                                                  const KrylovState* st) {
+                                                  const KrylovState* st, long long vsf, long long vsc, long long vscompact) {
   if (st != nullptr && st->done) return;
+  rf += blockIdx.y * vsf;  // column
+  rc += blockIdx.y * vsc;
+  if (compact != nullptr) compact += blockIdx.y * vscompact;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= c.ndof) return;
   const long long I = i / 3;
@@ -474,13 +514,14 @@ __global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* __res
 }
 
 void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc, void* rc,
-                  const int* index, double* compact, const KrylovState* st, cudaStream_t s) {
+                  const int* index, double* compact, const KrylovState* st, cudaStream_t s, int nv, long long vsf,
+                  long long vsc, long long vscompact) {
   const int bs = 128;
-  const unsigned nb = (unsigned)((coarse.ndof + bs - 1) / bs);
+  const dim3 nb((unsigned)((coarse.ndof + bs - 1) / bs), (unsigned)nv);
   if (vec64)
-    k_restrict<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st);
+    k_restrict<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st, vsf, vsc, vscompact);
   else
-    k_restrict<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st);
+    k_restrict<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st, vsf, vsc, vscompact);
   TOPO_LAUNCH_CHECK();
 }
 
@@ -488,8 +529,12 @@ void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* 
 // issued together.
 template <typename T>
 __global__ void __launch_bounds__(256) k_prolong_add(Grid f, Grid c, const T* __restrict__ ec, const uint8_t* __restrict__ mf,
-                                                     T* __restrict__ xf, T* __restrict__ e_out, const KrylovState* st) {
+                                                     T* __restrict__ xf, T* __restrict__ e_out, const KrylovState* st,
+                                                     long long vsf, long long vsc) {
   if (st != nullptr && st->done) return;
+  ec += blockIdx.y * vsc;  // column
+  xf += blockIdx.y * vsf;
+  if (e_out) e_out += blockIdx.y * vsf;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= f.ndof) return;
   const long long n = i / 3;
@@ -520,13 +565,13 @@ __global__ void __launch_bounds__(256) k_prolong_add(Grid f, Grid c, const T* __
 }
 
 void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* ec, const uint8_t* mf, void* xf,
-                 void* e_out, const KrylovState* st, cudaStream_t s) {
+                 void* e_out, const KrylovState* st, cudaStream_t s, int nv, long long vsf, long long vsc) {
   const int bs = 256;
-  const unsigned nb = (unsigned)((fine.ndof + bs - 1) / bs);
+  const dim3 nb((unsigned)((fine.ndof + bs - 1) / bs), (unsigned)nv);
   if (vec64)
-    k_prolong_add<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)ec, mf, (double*)xf, (double*)e_out, st);
+    k_prolong_add<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)ec, mf, (double*)xf, (double*)e_out, st, vsf, vsc);
   else
-    k_prolong_add<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)ec, mf, (float*)xf, (float*)e_out, st);
+    k_prolong_add<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)ec, mf, (float*)xf, (float*)e_out, st, vsf, vsc);
   TOPO_LAUNCH_CHECK();
 }
 

@@ -695,8 +695,10 @@ __device__ __forceinline__ double row_sum(double acc, int warp, int lane) {
 template <typename TX>
 __global__ void __launch_bounds__(256) k_coarse_lower(int m, int b0, long long ld, int gofs, int band, int prev,
                                                       const TX* __restrict__ Cq, const double* __restrict__ rc,
-                                                      double* y, const KrylovState* st) {
+                                                      double* y, const KrylovState* st, long long vswork) {
   if (st != nullptr && st->done) return;  // uniform over the grid
+  rc += blockIdx.y * vswork;              // column
+  y += blockIdx.y * vswork;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = (int)blockIdx.x * (8 / RW) + warp / RW, sub = warp % RW;
   const bool live = row < m;
@@ -716,8 +718,12 @@ template <typename T, typename TX>
 __global__ void __launch_bounds__(256) k_coarse_upper(int m, int b0, long long ld, int hofs, int band, int next,
                                                       long long nfull, const TX* __restrict__ Cq,
                                                       const int* __restrict__ free_list, const double* y, double* z,
-                                                      T* __restrict__ x, const KrylovState* st) {
+                                                      T* __restrict__ x, const KrylovState* st, long long vswork,
+                                                      long long vsx) {
   if (st != nullptr && st->done) return;  // uniform over the grid
+  y += blockIdx.y * vswork;               // column
+  z += blockIdx.y * vswork;
+  x += blockIdx.y * vsx;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = (int)blockIdx.x * (8 / RW) + warp / RW, sub = warp % RW;
   const bool live = row < m;
@@ -875,7 +881,8 @@ int coarsest_status(CoarsestFactor& f, cudaStream_t s) {
 // work: 2n doubles (y, then the compact right-hand side, overwritten by the
 // compact solution in the second pass). Only the free DoFs of x are written.
 template <typename T, typename TX>
-static void apply_blocks(const CoarsestFactor& f, double* work, T* x, const KrylovState* st, cudaStream_t s) {
+static void apply_blocks(const CoarsestFactor& f, double* work, T* x, const KrylovState* st, cudaStream_t s, int nv,
+                         long long vswork, long long vsx) {
   const CoarsestPlan& p = f.plan;
   const CoarseBlocks& bk = f.blk;
   const int n = p.n;
@@ -885,28 +892,29 @@ static void apply_blocks(const CoarsestFactor& f, double* work, T* x, const Kryl
   const TX* C = (const TX*)f.C;
   for (int q = 0; q < bk.P; ++q) {
     const int m = bk.b[q + 1] - bk.b[q];
-    cst::k_coarse_lower<TX><<<(unsigned)((m + rpb - 1) / rpb), 256, 0, s>>>(
-        m, bk.b[q], bk.ld[q], bk.gofs[q], f.band, (int)(q > 0), C + bk.off[q], rc, y, st);
+    cst::k_coarse_lower<TX><<<dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s>>>(
+        m, bk.b[q], bk.ld[q], bk.gofs[q], f.band, (int)(q > 0), C + bk.off[q], rc, y, st, vswork);
     TOPO_LAUNCH_CHECK();
   }
   for (int q = bk.P - 1; q >= 0; --q) {
     const int m = bk.b[q + 1] - bk.b[q];
-    cst::k_coarse_upper<T, TX><<<(unsigned)((m + rpb - 1) / rpb), 256, 0, s>>>(
+    cst::k_coarse_upper<T, TX><<<dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s>>>(
         m, bk.b[q], bk.ld[q], bk.hofs[q], f.band, (int)(q < bk.P - 1), p.nfull, C + bk.off[q], f.d_free, y, rc, x,
-        st);
+        st, vswork, vsx);
     TOPO_LAUNCH_CHECK();
   }
 }
 
-void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s) {
+void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s, int nv,
+                    long long vswork, long long vsx) {
   if (f.plan.n == 0) return;
   if (vec64) {
     if (!f.f64) throw std::runtime_error("coarsest apply: FP64 vectors need the FP64 inverse");
-    apply_blocks<double, double>(f, work, (double*)x, st, s);
+    apply_blocks<double, double>(f, work, (double*)x, st, s, nv, vswork, vsx);
   } else if (f.f64) {
-    apply_blocks<float, double>(f, work, (float*)x, st, s);
+    apply_blocks<float, double>(f, work, (float*)x, st, s, nv, vswork, vsx);
   } else {
-    apply_blocks<float, float>(f, work, (float*)x, st, s);
+    apply_blocks<float, float>(f, work, (float*)x, st, s, nv, vswork, vsx);
   }
 }
 

@@ -124,6 +124,10 @@ struct Level {
   __nv_bfloat16* S16 = nullptr;
   double lam = NAN;
   int degree = 2;
+  // the V-cycle's vectors for several columns (x, r, d, d2, e, b; allocated by
+  // the first block solve), vs entries from column to column
+  void* cols[6] = {};
+  long long vs = 0;
 };
 
 // One factorisation of the coarsest operator, with the stencil it is built from.
@@ -196,6 +200,10 @@ struct topo_ctx {
   std::vector<double> pcg_key;
   // block PCG workspace (FP64 columns R, Z, P, Q, Pn; allocated per block width)
   int blk_nv = 0;
+  int bw = 1;                   // columns the V-cycle works on
+  int blk_cols = 0;             // columns the levels' block vectors hold
+  int blk_n = 0;                // coarsest size they were made for
+  double* blk_y = nullptr;      // coarsest work of every column
   double* blk = nullptr;
   double* blk_part = nullptr;
   double* blk_G = nullptr;
@@ -264,11 +272,11 @@ void op_apply(topo_ctx* c, int l, Prec p, const void* u, void* y, Epi epi, const
   Level& Lv = c->L[l];
   if (l == 0) {
     const void* E = (p == Prec::F64) ? (const void*)c->E64 : (const void*)c->E32;
-    if (p == Prec::BF16) level0_apply_bf16(c->use_tc, false, Lv.g, u, E, Lv.mask, c->nmask0, y, epi, ea, s, !same_bits);
-    else level0_apply(p, Lv.g, u, E, Lv.mask, y, epi, ea, s, !same_bits);
+    if (p == Prec::BF16) level0_apply_bf16(c->use_tc, false, Lv.g, u, E, Lv.mask, c->nmask0, y, epi, ea, s, !same_bits, c->bw, Lv.vs);
+    else level0_apply(p, Lv.g, u, E, Lv.mask, y, epi, ea, s, !same_bits, c->bw, Lv.vs);
   } else {
     const void* S = p == Prec::F64 ? (const void*)Lv.S64 : p == Prec::F32 ? (const void*)Lv.S32 : (const void*)Lv.S16;
-    stencil_apply(p, c->vec64, Lv.g, S, u, Lv.mask, y, epi, ea, s);
+    stencil_apply(p, c->vec64, Lv.g, S, u, Lv.mask, y, epi, ea, s, c->bw, Lv.vs);
   }
 }
 
@@ -294,7 +302,7 @@ void smooth(topo_ctx* c, int l, bool from_zero, bool started, bool want_residual
   const Cheb ch = level_cheb(c, Lv);
   const long long n = Lv.g.ndof;
   if (!started) cheb_start(c->vec64, n, from_zero ? Lv.b : nullptr, Lv.r, Lv.dinv, ch.c2[0], ch.ax[0], Lv.x, Lv.d, from_zero, st,
-             s);
+             s, c->bw, Lv.vs);
   void* dcur = Lv.d;
   void* dnext = Lv.d2;
   for (int j = 1; j < Lv.degree; ++j) {
@@ -324,7 +332,8 @@ void smooth(topo_ctx* c, int l, bool from_zero, bool started, bool want_residual
 // x is zero at the fixed DoFs (topo_set_problem) and written at the free ones.
 void coarsest_solve(topo_ctx* c, const KrylovState* st, cudaStream_t s) {
   if (c->C.n == 0) return;
-  coarsest_apply(c->C.cur.f, c->vec64, c->C.y, c->L[c->n_levels - 1].x, st, s);
+  coarsest_apply(c->C.cur.f, c->vec64, c->bw > 1 ? c->blk_y : c->C.y, c->L[c->n_levels - 1].x, st, s, c->bw, 2LL * c->C.n,
+                 c->L[c->n_levels - 1].vs);
 }
 
 // One V-cycle (cycle_gamma 1, multigrid_v4.py:986-1008) or W-cycle
@@ -344,9 +353,10 @@ void vcycle(topo_ctx* c, int l, const KrylovState* st, bool same_bits, cudaStrea
   for (int k = 0; k < c->cycle_gamma; ++k) {
     const bool bottom = l + 1 == c->n_levels - 1;
     restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, Lc.b, bottom ? c->C.dof_index : nullptr,
-                 bottom ? c->C.y + std::max(c->C.n, 1) : nullptr, st, s);
+                 bottom ? (c->bw > 1 ? c->blk_y : c->C.y) + std::max(c->C.n, 1) : nullptr, st, s, c->bw, Lv.vs, Lc.vs,
+                 2LL * c->C.n);
     vcycle(c, l + 1, st, same_bits, s);
-    prolong_add(c->vec64, Lv.g, Lc.g, Lc.x, Lv.mask, Lv.x, Lv.e, st, s);  // x += e = P x_c
+    prolong_add(c->vec64, Lv.g, Lc.g, Lc.x, Lv.mask, Lv.x, Lv.e, st, s, c->bw, Lv.vs, Lc.vs);  // x += e = P x_c
     EpiArgs ea{};
     ea.r = Lv.r;
     ea.s = 1.0;
@@ -381,6 +391,43 @@ void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cu
   vcycle(c, 0, st, same_bits, s);
   L0.b = saved_b;
   L0.x = saved_x;
+}
+
+// The V-cycle on nv columns at once: level 0's b and x are the first and the
+// last of its block vectors. Every kernel covers all columns, so a launch and
+// (on the coarse levels) a fetch of the coefficients serve all of them; the
+// columns one after another left most kernels latency bound.
+void block_reserve(topo_ctx* c, int nv) {
+  if (c->blk_cols >= nv && c->blk_n == c->C.n) return;
+  for (Level& Lv : c->L) {
+    Lv.vs = (Lv.g.ndof + 3) & ~3LL;  // columns 16-byte aligned in FP32 and FP64
+    for (void*& p : Lv.cols) p = c->valloc(nv * Lv.vs);
+  }
+  c->blk_y = c->alloc<double>(2LL * std::max(c->C.n, 1) * nv);
+  c->blk_n = c->C.n;
+  c->blk_cols = nv;
+}
+
+void vcycle_columns(topo_ctx* c, int nv, cudaStream_t s) {
+  std::vector<Level> saved = c->L;
+  for (Level& Lv : c->L) {
+    Lv.x = Lv.cols[0];
+    Lv.r = Lv.cols[1];
+    Lv.d = Lv.cols[2];
+    Lv.d2 = Lv.cols[3];
+    Lv.e = Lv.cols[4];
+    Lv.b = Lv.cols[5];
+  }
+  c->bw = nv;
+  try {
+    vcycle(c, 0, nullptr, false, s);
+  } catch (...) {
+    c->bw = 1;
+    c->L = saved;
+    throw;
+  }
+  c->bw = 1;
+  c->L = saved;
 }
 
 // ------------------------------------------------------- spectral bounds
@@ -861,8 +908,9 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
                  double* out_relres, cudaStream_t s) {
   Level& L0 = c->L[0];
   const long long n = L0.g.ndof;
+  const long long ld = (n + 3) & ~3LL;  // column stride: 16-byte aligned columns
   if (c->blk_nv != nv) {
-    c->blk = c->alloc<double>(5LL * nv * n);
+    c->blk = c->alloc<double>(5LL * nv * ld);
     if (!c->blk_part) {
       c->blk_part = c->alloc<double>((long long)block_gram_partials());
       c->blk_G = c->alloc<double>(64);
@@ -870,23 +918,31 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     }
     c->blk_nv = nv;
   }
-  double *R0 = c->blk, *Z0 = R0 + (long long)nv * n, *P0 = Z0 + (long long)nv * n, *Q0 = P0 + (long long)nv * n,
-         *N0 = Q0 + (long long)nv * n;
-  auto col = [&](double* base, int j) { return base + (long long)j * n; };
+  block_reserve(c, nv);
+  double *R0 = c->blk, *Z0 = R0 + nv * ld, *P0 = Z0 + nv * ld, *Q0 = P0 + nv * ld, *N0 = Q0 + nv * ld;
+  auto col = [&](double* base, int j) { return base + j * ld; };
   auto gram = [&](double* const* A, int na, double* const* Bm, int nb, double* Gout) {
     block_gram(n, (const double* const*)A, na, (const double* const*)Bm, nb, c->blk_part, c->blk_G, s);
     TOPO_CUDA_CHECK(cudaMemcpyAsync(c->blk_Gh, c->blk_G, 64 * sizeof(double), cudaMemcpyDeviceToHost, s));
     TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
     std::memcpy(Gout, c->blk_Gh, 64 * sizeof(double));
   };
-  auto precond = [&](const double* r, double* z) {
-    if (c->vec64) {
-      vcycle_apply(c, r, z, nullptr, s);
-    } else {
-      vcast(n, r, true, c->kr, false, s);
-      vcycle_apply(c, c->kr, c->kz, nullptr, s);
-      vcast(n, c->kz, false, z, true, s);
-    }
+  // Z_a = M R_a for the k active columns at once
+  auto precond = [&](double* const* r, double* const* z, int k) {
+    Level& L0b = c->L[0];
+    char* b0 = (char*)L0b.cols[5];
+    char* x0 = (char*)L0b.cols[0];
+    const long long st = L0b.vs * (long long)c->vsize();
+    for (int a = 0; a < k; ++a) vcast(n, r[a], true, b0 + a * st, c->vec64, s);
+    vcycle_columns(c, k, s);
+    for (int a = 0; a < k; ++a) vcast(n, x0 + a * st, c->vec64, z[a], true, s);
+  };
+  // Y = K U: one launch for all columns where the parity form applies
+  auto apply = [&](double* const* U, double* const* Y, int k) {
+    if (level0_pt_supported(L0.g, true, false, c->blk))
+      level0_columns_pt(L0.g, (const double* const*)U, c->E64, L0.mask, Y, k, s);
+    else
+      level0_apply_block(L0.g, (const double* const*)U, c->E64, L0.mask, Y, k, s);
   };
   std::vector<int> act;
   double* Xc[8];
@@ -915,7 +971,9 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
   double bnorm[8];
   for (int j = 0; j < nv; ++j) bnorm[j] = std::sqrt(std::max(G[j * 8 + j], 0.0));
   // R = mask(B) - A X
-  level0_apply_block(L0.g, (const double* const*)Xc, c->E64, L0.mask, Qc, nv, s);
+  for (int j = 0; j < nv; ++j)  // (X's columns need not be 16-byte aligned)
+    TOPO_CUDA_CHECK(cudaMemcpyAsync(Nc[j], Xc[j], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+  apply(Nc, Qc, nv);
   {
     double I8[64] = {};
     for (int j = 0; j < 8; ++j) I8[j * 8 + j] = 1.0;
@@ -938,10 +996,9 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     pick(Zc, aZ);
     pick(Pc, aP);
     const int k = (int)act.size();
-    for (int a = 0; a < k; ++a) {
-      precond(aR[a], aZ[a]);
+    precond(aR, aZ, k);
+    for (int a = 0; a < k; ++a)
       TOPO_CUDA_CHECK(cudaMemcpyAsync(aP[a], aZ[a], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-    }
     gram(aZ, k, aR, k, rz);
     it = 1;
   }
@@ -953,7 +1010,7 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     pick(Qc, aQ);
     pick(Nc, aN);
     pick(Xc, aX);
-    level0_apply_block(L0.g, (const double* const*)aP, c->E64, L0.mask, aQ, k, s);
+    apply(aP, aQ, k);
     gram(aP, k, aQ, k, G);  // P^T Q
     if (!small_chol_solve(k, G, rz, A8)) throw std::runtime_error("block PCG: P^T K P lost definiteness");
     block_combine(n, (const double* const*)aP, k, (const double* const*)aX, aX, k, A8, 1.0, s);
@@ -983,7 +1040,7 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     pick(Zc, aZ);
     pick(Pc, aP);
     pick(Nc, aN);
-    for (int a = 0; a < k2; ++a) precond(aR[a], aZ[a]);
+    precond(aR, aZ, k2);
     gram(aZ, k2, aR, k2, H);  // Z^T R
     // P's surviving columns
     double* Pk[8];
@@ -1355,6 +1412,7 @@ int topo_set_problem(topo_ctx* c, const uint8_t* free_mask, const double* F, voi
         }
       }
       TOPO_CUDA_CHECK(cudaMemsetAsync(Lc.x, 0, c->vsize() * Lc.g.ndof, s));
+      if (Lc.cols[0]) TOPO_CUDA_CHECK(cudaMemsetAsync(Lc.cols[0], 0, c->vsize() * Lc.vs * c->blk_cols, s));
       TOPO_CUDA_CHECK(cudaMemcpyAsync(c->C.dof_index, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, s));
       TOPO_CUDA_CHECK(cudaMemcpyAsync(c->C.free_list, fl.data(), sizeof(int) * std::max<size_t>(fl.size(), 1),
                                       cudaMemcpyHostToDevice, s));

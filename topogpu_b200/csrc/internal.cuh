@@ -208,12 +208,15 @@ __device__ __forceinline__ void epilogue_store(const EpiDev<T>& e, long long i, 
 }
 
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                  Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true);
+                  Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true, int nv = 1, long long vs = 0);
+// nv > 1: that many columns, every vector of column v starting v * vs entries on
+// (vs a multiple of 4); epilogues Store, Residual, ChebR, RUpd.
 // BF16-input operator (u stored BF16 or FP32, rounded); tc: the tensor-core
 // kernel may be used where the parity form does not apply. parity = false:
 // the general kernels only (same results to the last bit of rounding order)
 void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask,
-                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true);
+                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true, int nv = 1,
+                       long long vs = 0);
 void level0_diag(const Grid& g, const double* E, const uint8_t* mask, double* diag, cudaStream_t s);
 // tensor-core BF16-input operator streaming along x (kmatvec_xs.cu); the
 // KE tile and the error flag are per device
@@ -234,7 +237,9 @@ void level0_apply_cc(bool f64, const Grid& g, const void* u, const void* E, cons
 void pt_prepare(const double* KE_host);
 bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u);
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                     Epi epi, const EpiArgs& ea, cudaStream_t s);
+                     Epi epi, const EpiArgs& ea, cudaStream_t s, int nv = 1, long long vs = 0);
+void level0_columns_pt(const Grid& g, const double* const* U, const double* E, const uint8_t* mask, double* const* Y, int nv,
+                       cudaStream_t s);
 void xs_debug(int skip_first_arrival, int poll_limit);
 void wait_debug(int& skip, int& poll);  // the test hook's current setting
 void modulus(long long n, const double* rho, double penal, double E0, double Emin, double* E,
@@ -250,7 +255,7 @@ long long rap_scratch(const Grid& fine, const Grid& coarse);  // doubles
 void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c, double* scratch,
          cudaStream_t s);
 void stencil_apply(Prec p, bool vec64, const Grid& g, const void* S, const void* u, const uint8_t* mask,
-                   void* y, Epi epi, const EpiArgs& ea, cudaStream_t s);
+                   void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, int nv = 1, long long vs = 0);
 void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* dinv64, float* dinv32,
                   cudaStream_t s);
 // FP64 stencil -> FP32 / BF16 apply copies in the same order (BF16: node stride rounded up to even)
@@ -258,10 +263,12 @@ long long stencil16_stride(long long nnodes);
 void stencil_convert(long long nnodes, const double* S, float* S32, __nv_bfloat16* S16, cudaStream_t s);
 void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_t* mc, cudaStream_t s);
 void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc,
-                  void* rc, const int* index, double* compact, const KrylovState* st, cudaStream_t s);
+                  void* rc, const int* index, double* compact, const KrylovState* st, cudaStream_t s, int nv = 1,
+                  long long vsf = 0, long long vsc = 0, long long vscompact = 0);
 // x_f += e = mask_f * P e_c ; e is also written to e_out when not null
 void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* ec, const uint8_t* mf,
-                 void* xf, void* e_out, const KrylovState* st, cudaStream_t s);
+                 void* xf, void* e_out, const KrylovState* st, cudaStream_t s, int nv = 1, long long vsf = 0,
+                 long long vsc = 0);
 // coarsest level (coarsest.cu): band Cholesky of the free-DoF operator and
 // the inverses of its diagonal blocks. Compact DoF i -> full DoF free[i].
 struct CoarsestPlan {
@@ -312,7 +319,8 @@ void coarsest_regularise(CoarsestFactor& f, double* dtmp, cudaStream_t s);
 void coarsest_factor(CoarsestFactor& f, cudaStream_t s);
 int coarsest_status(CoarsestFactor& f, cudaStream_t s);
 // work: 2n doubles, the right-hand side (compact) in the second half
-void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s);
+void coarsest_apply(const CoarsestFactor& f, bool vec64, double* work, void* x, const KrylovState* st, cudaStream_t s,
+                    int nv = 1, long long vswork = 0, long long vsx = 0);
 
 // block PCG kernels (blockops.cu): FP64 column blocks as pointer lists
 void set_ke_block(const double* KE_host);
@@ -334,7 +342,7 @@ void vmask(bool f64, long long n, void* x, const uint8_t* mask, cudaStream_t s);
 // First Chebyshev step on residual r (copied from b first when b is not
 // null): d = c2 D^-1 r ; x = (x_is_zero ? 0 : x) + ax d
 void cheb_start(bool f64, long long n, const void* b, void* r, const void* dinv, double c2, double ax, void* x,
-                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s);
+                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s, int nv = 1, long long vs = 0);
 // out = sum a_i b_i (fp64 accumulate) to a device double
 void dot_to(bool f64, long long n, const void* a, const void* b, double* out, RedWork red,
             cudaStream_t s);

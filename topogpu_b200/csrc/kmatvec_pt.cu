@@ -79,6 +79,10 @@ struct Params {
   const T* E;
   const uint8_t* mask;
   EpiDev<T> ep;
+  long long vs;             // column v = blockIdx.y of every vector starts v * vs entries on (u 16-byte aligned)
+  int list;                 // != 0: u and y of column v are ucol[v], ycol[v]
+  const void* ucol[8];
+  T* ycol[8];
   KrylovState* st;
   RedWork red;
   int* err;
@@ -150,6 +154,9 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Grid& g = P.g;
   const int NZ = g.NZ, PN = P.PN;
+  const long long co = (long long)blockIdx.y * P.vs;
+  const TU* const uc = P.list ? reinterpret_cast<const TU*>(P.ucol[blockIdx.y]) : reinterpret_cast<const TU*>(P.u) + co;
+  T* const yc = P.list ? P.ycol[blockIdx.y] : P.ep.y + co;
   const int w = (int)blockIdx.x % P.nwin, sg = (int)blockIdx.x / P.nwin;
   const int n0 = w * P.TO, n1 = min(PN, n0 + P.TO);  // output nodes of a plane
   const int xa = (int)((long long)g.NX * sg / P.nseg), xb = (int)((long long)g.NX * (sg + 1) / P.nseg);  // output planes
@@ -174,7 +181,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
     const long long off0 = ((long long)p * PN + ms) * (3 * SU);
     const long long n = (long long)(me - ms) * (3 * SU);
     unsigned char* dst = sm + sl * P.slot + 16 + shift + (ms - mlo) * 3 * SU - (int)(off0 & 15);
-    const unsigned char* src = reinterpret_cast<const unsigned char*>(P.u);
+    const unsigned char* src = reinterpret_cast<const unsigned char*>(uc);
     const long long a = off0 & ~15LL, vfloor = (g.ndof * (long long)SU) & ~15LL;
     long long e = (off0 + n + 15) & ~15LL;
     if (e > vfloor) {
@@ -190,11 +197,11 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   };
   auto hint = [&](int x) {  // thread 0: what the epilogue of output plane x reads
     const long long b = 3 * ((long long)x * PN + n0), e = 3 * ((long long)x * PN + n1);
-    if constexpr (EPI == Epi::Residual) prefetch_l2(P.ep.b + b, P.ep.b + e);
-    if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) prefetch_l2(P.ep.r + b, P.ep.r + e);
+    if constexpr (EPI == Epi::Residual) prefetch_l2(P.ep.b + co + b, P.ep.b + co + e);
+    if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) prefetch_l2(P.ep.r + co + b, P.ep.r + co + e);
     if constexpr (EPI == Epi::ChebR) {
       prefetch_l2(P.ep.dinv + b, P.ep.dinv + e);
-      prefetch_l2(P.ep.x + b, P.ep.x + e);
+      prefetch_l2(P.ep.x + co + b, P.ep.x + co + e);
     }
     prefetch_l2(P.mask + b, P.mask + e);
   };
@@ -266,23 +273,23 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
     unsigned char m[3];
   };
   auto fetch = [&](int x, Epv& v) {
-    const long long base = 3 * ((long long)x * PN + n0);
+    const long long base = 3 * ((long long)x * PN + n0), cb = base + co;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const unsigned i = tid + j * NT;
       if (!((int)i < cnt && topo_in_range(base + i, g.ndof))) continue;
       v.m[j] = (P.mask + base)[i];
-      if constexpr (EPI == Epi::Residual) v.r[j] = (P.ep.b + base)[i];
-      if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) v.r[j] = (P.ep.r + base)[i];
+      if constexpr (EPI == Epi::Residual) v.r[j] = (P.ep.b + cb)[i];
+      if constexpr (EPI == Epi::RUpd || EPI == Epi::ChebR) v.r[j] = (P.ep.r + cb)[i];
       if constexpr (EPI == Epi::ChebR) {
         v.d[j] = (P.ep.dinv + base)[i];
-        v.x[j] = (P.ep.x + base)[i];
+        v.x[j] = (P.ep.x + cb)[i];
       }
-      if constexpr (EPI == Epi::ChebR || EPI == Epi::StoreDot) v.u[j] = load_u<T>(reinterpret_cast<const TU*>(P.u) + base + i);
+      if constexpr (EPI == Epi::ChebR || EPI == Epi::StoreDot) v.u[j] = load_u<T>(uc + base + i);
     }
   };
   auto finish = [&](int x, int b, const Epv& v) {
-    const long long base = 3 * ((long long)x * PN + n0);
+    const long long base = 3 * ((long long)x * PN + n0), cb = base + co;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const unsigned i = tid + j * NT;
@@ -290,21 +297,21 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
       const bool fr = v.m[j] != 0;
       const T a = pr[b * bsz + 3 * NZ + j * NT] + pr[b * bsz + P.pw_n + j * NT];
       if constexpr (EPI == Epi::Store) {
-        (P.ep.y + base)[i] = fr ? a : (T)0;
+        (yc + base)[i] = fr ? a : (T)0;
       } else if constexpr (EPI == Epi::StoreDot) {
         const T y = fr ? a : (T)0;
-        (P.ep.y + base)[i] = y;
+        (yc + base)[i] = y;
         part += (double)v.u[j] * (double)y;
       } else if constexpr (EPI == Epi::Residual) {
-        (P.ep.y + base)[i] = fr ? v.r[j] - a : (T)0;
+        (yc + base)[i] = fr ? v.r[j] - a : (T)0;
       } else if constexpr (EPI == Epi::RUpd) {
-        (P.ep.r + base)[i] = fr ? v.r[j] - P.ep.s * a : (T)0;
+        (P.ep.r + cb)[i] = fr ? v.r[j] - P.ep.s * a : (T)0;
       } else {
         const T rv = v.r[j] - P.ep.s * a;
         const T dn = P.ep.c1 * v.u[j] + P.ep.c2 * (v.d[j] * rv);
-        (P.ep.r + base)[i] = fr ? rv : (T)0;
-        (P.ep.d_out + base)[i] = fr ? dn : (T)0;
-        if (fr) (P.ep.x + base)[i] = v.x[j] + P.ep.ax * dn;
+        (P.ep.r + cb)[i] = fr ? rv : (T)0;
+        (P.ep.d_out + cb)[i] = fr ? dn : (T)0;
+        if (fr) (P.ep.x + cb)[i] = v.x[j] + P.ep.ax * dn;
       }
     }
   };
@@ -529,7 +536,7 @@ struct PtLayout {
 // than 3/4 of its elements on the halo is left out; with none left (NZ above
 // 372, in FP64 279) the general kernels take the mesh.
 template <typename T>
-bool pt_layout(const Grid& g, int s_u, int nsm, PtLayout& best) {
+bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
   const long long PN = (long long)g.NY * g.NZ;
   if (PN >= (1 << 28)) return false;
   double cost = 1e300;
@@ -540,11 +547,11 @@ bool pt_layout(const Grid& g, int s_u, int nsm, PtLayout& best) {
     L.w = w;
     L.TO = TO;
     L.nwin = (int)((PN + TO - 1) / TO);
-    const long long slots = (long long)nsm * Width<T>::PER[w];
+    const long long slots = std::max<long long>(1, (long long)nsm * Width<T>::PER[w] / nv);  // per column
     L.nseg = (int)std::max<long long>(1, std::min<long long>(g.NX, slots / L.nwin));
     const long long ctas = (long long)L.nwin * L.nseg;
     const double waves = std::ceil((double)ctas / (double)slots);
-    const double per = std::min<double>(Width<T>::PER[w], std::ceil((double)ctas / nsm));
+    const double per = std::min<double>(Width<T>::PER[w], std::ceil((double)ctas * nv / nsm));
     const double c = waves * ((g.NX + L.nseg - 1) / L.nseg + 1) * std::max(8.0, per * NW);
     const auto al = [](long long x) { return (int)((x + 127) & ~127LL); };
     L.slot = al(64 + 3LL * s_u * (31 * NW + g.NZ + 3));
@@ -561,7 +568,7 @@ bool pt_layout(const Grid& g, int s_u, int nsm, PtLayout& best) {
 }
 
 template <typename T, typename TU, bool BF, Epi EPI, int W>
-void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, cudaStream_t s) {
+void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t s) {
   auto* k = pt::k_level0_pt<T, TU, BF, EPI, Width<T>::NW[W], Width<T>::PER[W]>;
   static std::atomic<uint64_t> raised{0};  // devices where this instance's shared-memory limit is raised
   int dev = 0;
@@ -570,14 +577,15 @@ void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, cudaStream_t s) {
     TOPO_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
     if (dev <= 63) raised |= 1ull << dev;
   }
-  k<<<(unsigned)(L.nwin * L.nseg), 32 * Width<T>::NW[W], L.total, s>>>(P);
+  k<<<dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T>::NW[W], L.total, s>>>(P);
   TOPO_LAUNCH_CHECK();
 }
 
 template <typename T, typename TU, bool BF, Epi EPI>
-void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, const EpiArgs& ea, cudaStream_t s) {
+void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, const EpiArgs& ea, cudaStream_t s,
+               int nv = 1, long long vs = 0, const void* const* ul = nullptr, void* const* yl = nullptr) {
   PtLayout L;
-  if (!pt_layout<T>(g, (int)sizeof(TU), pt_device().nsm, L))
+  if (!pt_layout<T>(g, (int)sizeof(TU), nv, pt_device().nsm, L))
     throw std::runtime_error("level0 K.u: mesh not supported by the parity form");
   pt::Params<T> P;
   P.g = g;
@@ -589,6 +597,12 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   P.E = (const T*)E;
   P.mask = mask;
   P.ep = make_epi<T>(y, ea);
+  P.vs = vs;
+  P.list = ul != nullptr;
+  for (int v = 0; v < 8; ++v) {
+    P.ucol[v] = ul && v < nv ? ul[v] : nullptr;
+    P.ycol[v] = yl && v < nv ? (T*)yl[v] : nullptr;
+  }
   P.st = ea.st;
   P.red = ea.red;
   P.err = wait_error_flag();
@@ -600,9 +614,9 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   P.skip = 0;
   if (BF) wait_debug(P.skip, P.poll);
   switch (L.w) {
-    case 0: launch_pt_w<T, TU, BF, EPI, 0>(L, P, s); break;
-    case 1: launch_pt_w<T, TU, BF, EPI, 1>(L, P, s); break;
-    default: launch_pt_w<T, TU, BF, EPI, 2>(L, P, s); break;
+    case 0: launch_pt_w<T, TU, BF, EPI, 0>(L, P, nv, s); break;
+    case 1: launch_pt_w<T, TU, BF, EPI, 1>(L, P, nv, s); break;
+    default: launch_pt_w<T, TU, BF, EPI, 2>(L, P, nv, s); break;
   }
 }
 }  // namespace
@@ -644,19 +658,20 @@ bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
   const PtDevice& d = pt_device();
   PtLayout L;
   return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 &&
-         (f64 ? pt_layout<double>(g, 8, d.nsm, L) : pt_layout<float>(g, 4, d.nsm, L));
+         (f64 ? pt_layout<double>(g, 8, 1, d.nsm, L) : pt_layout<float>(g, 4, 1, d.nsm, L));
 }
 
 // f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
-// where it is read) or stored BF16 (u_bf16). Epilogues as level0_apply.
+// where it is read) or stored BF16 (u_bf16). Epilogues as level0_apply. nv
+// columns vs entries apart (u of each 16-byte aligned; one for StoreDot).
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
-                     Epi epi, const EpiArgs& ea, cudaStream_t s) {
+                     Epi epi, const EpiArgs& ea, cudaStream_t s, int nv, long long vs) {
 #define TOPO_PT_CASE(EP)                                                                                     \
   case Epi::EP:                                                                                              \
-    if (f64) launch_pt<double, double, false, Epi::EP>(g, u, E, mask, y, ea, s);                             \
-    else if (u_bf16) launch_pt<float, __nv_bfloat16, true, Epi::EP>(g, u, E, mask, y, ea, s);                \
-    else if (bf) launch_pt<float, float, true, Epi::EP>(g, u, E, mask, y, ea, s);                            \
-    else launch_pt<float, float, false, Epi::EP>(g, u, E, mask, y, ea, s);                                   \
+    if (f64) launch_pt<double, double, false, Epi::EP>(g, u, E, mask, y, ea, s, nv, vs);                     \
+    else if (u_bf16) launch_pt<float, __nv_bfloat16, true, Epi::EP>(g, u, E, mask, y, ea, s, nv, vs);        \
+    else if (bf) launch_pt<float, float, true, Epi::EP>(g, u, E, mask, y, ea, s, nv, vs);                    \
+    else launch_pt<float, float, false, Epi::EP>(g, u, E, mask, y, ea, s, nv, vs);                           \
     break;
   switch (epi) {
     TOPO_PT_CASE(Store)
@@ -664,12 +679,20 @@ void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* 
     TOPO_PT_CASE(ChebR)
     TOPO_PT_CASE(RUpd)
     case Epi::StoreDot:
+      if (nv != 1) throw std::runtime_error("level0 K.u: the dot product goes with one column");
       if (f64) launch_pt<double, double, false, Epi::StoreDot>(g, u, E, mask, y, ea, s);
       else if (!bf) launch_pt<float, float, false, Epi::StoreDot>(g, u, E, mask, y, ea, s);
       else throw std::runtime_error("level0 K.u: the dot product goes with the FP32 and FP64 operators");
       break;
   }
 #undef TOPO_PT_CASE
+}
+
+// Y_v = K U_v in FP64 for nv <= 8 columns (each U_v 16-byte aligned).
+void level0_columns_pt(const Grid& g, const double* const* U, const double* E, const uint8_t* mask, double* const* Y, int nv,
+                       cudaStream_t s) {
+  EpiArgs ea{};
+  launch_pt<double, double, false, Epi::Store>(g, nullptr, E, mask, nullptr, ea, s, nv, 0, (const void* const*)U, (void* const*)Y);
 }
 
 TOPO_BOUNDS_READER(bounds_flag_pt)

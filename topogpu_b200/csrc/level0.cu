@@ -246,14 +246,37 @@ static void launch_level0(const Grid& g, const void* u, const void* E, const uin
   TOPO_LAUNCH_CHECK();
 }
 
+// The operands of the column `at` entries on.
+struct ColumnAt {
+  const void* u;
+  void* y;
+  EpiArgs ea;
+  ColumnAt(int size, long long at, const void* u0, void* y0, const EpiArgs& e0) : ea(e0) {
+    auto mv = [&](const void* p) { return p ? (const void*)((const char*)p + size * at) : nullptr; };
+    u = mv(u0);
+    y = (void*)mv(y0);
+    ea.b = mv(e0.b);
+    ea.r = (void*)mv(e0.r);
+    ea.x = (void*)mv(e0.x);
+    ea.d_out = (void*)mv(e0.d_out);
+  }
+};
+
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, Epi epi,
-                  const EpiArgs& ea, cudaStream_t s, bool parity) {
+                  const EpiArgs& ea, cudaStream_t s, bool parity, int nv, long long vs) {
   // The parity form (kmatvec_pt.cu) takes every mesh with a window layout when
   // KE has the cube's mirror symmetry. Without it FP64 / FP32 run the
   // x-streaming kernel (kmatvec_cc.cu) when its planes fit in shared memory;
   // the brick kernel below otherwise and for the BF16 emulation.
   if (parity && level0_pt_supported(g, p == Prec::F64, p == Prec::BF16, u)) {
-    level0_apply_pt(p == Prec::F64, p == Prec::BF16, false, g, u, E, mask, y, epi, ea, s);
+    level0_apply_pt(p == Prec::F64, p == Prec::BF16, false, g, u, E, mask, y, epi, ea, s, nv, vs);
+    return;
+  }
+  if (nv > 1) {  // the general kernels take one column at a time
+    for (int v = 0; v < nv; ++v) {
+      const ColumnAt c(p == Prec::F64 ? 8 : 4, v * vs, u, y, ea);
+      level0_apply(p, g, c.u, E, mask, c.y, epi, c.ea, s, parity);
+    }
     return;
   }
   const bool al = ((uintptr_t)u & 15) == 0 && ((uintptr_t)E & 15) == 0;
@@ -273,13 +296,20 @@ void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uin
 // The tensor-core kernel's meshes and pointers (16-byte aligned vectors) are
 // what the fused epilogues accept with tc set, whichever kernel runs them.
 void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask,
-                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity) {
+                       const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity, int nv,
+                       long long vs) {
   if (tc && level0_xs_supported(g)) {
     level0_xs_check(u, E, nmask, ea);
-    if (parity && level0_pt_supported(g, false, true, u)) level0_apply_pt(false, true, u_bf16, g, u, E, mask, y, epi, ea, s);
-    else level0_apply_xs(u_bf16, g, u, E, nmask, y, epi, ea, s);
+    if (parity && level0_pt_supported(g, false, true, u)) {
+      level0_apply_pt(false, true, u_bf16, g, u, E, mask, y, epi, ea, s, nv, vs);
+    } else {
+      for (int v = 0; v < nv; ++v) {  // (columns are FP32)
+        const ColumnAt c(4, v * vs, u, y, ea);
+        level0_apply_xs(u_bf16, g, c.u, E, nmask, c.y, epi, c.ea, s);
+      }
+    }
   } else if (!u_bf16) {
-    level0_apply(Prec::BF16, g, u, E, mask, y, epi, ea, s, parity);
+    level0_apply(Prec::BF16, g, u, E, mask, y, epi, ea, s, parity, nv, vs);
   } else {
     if (epi != Epi::Store) throw std::runtime_error("topo_level0_apply: BF16-stored u on CUDA cores supports Store only");
     if (parity && level0_pt_supported(g, false, true, u)) level0_apply_pt(false, true, true, g, u, E, mask, y, epi, ea, s);

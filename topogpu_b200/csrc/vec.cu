@@ -63,8 +63,14 @@ void vmask(bool f64, long long n, void* x, const uint8_t* mask, cudaStream_t s) 
 // b itself: K 0 = 0, no operator application): d = c2 D^-1 r, x += ax d.
 template <typename T>
 __global__ void k_cheb_start(long long n, const T* __restrict__ b, T* __restrict__ r, const T* __restrict__ dinv,
-                             T c2, T ax, T* __restrict__ x, T* __restrict__ d, int x_is_zero, const KrylovState* st) {
+                             T c2, T ax, T* __restrict__ x, T* __restrict__ d, int x_is_zero, const KrylovState* st,
+                             long long vs) {
   if (st != nullptr && st->done) return;
+  const long long co = blockIdx.y * vs;  // column
+  if (b != nullptr) b += co;
+  r += co;
+  x += co;
+  d += co;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
     T ri;
@@ -81,13 +87,14 @@ __global__ void k_cheb_start(long long n, const T* __restrict__ b, T* __restrict
 }
 
 void cheb_start(bool f64, long long n, const void* b, void* r, const void* dinv, double c2, double ax, void* x,
-                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s) {
+                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s, int nv, long long vs) {
+  const dim3 nb(grid_for(n, 256), (unsigned)nv);
   if (f64)
-    k_cheb_start<double><<<grid_for(n, 256), 256, 0, s>>>(n, (const double*)b, (double*)r, (const double*)dinv, c2,
-                                                          ax, (double*)x, (double*)d, x_is_zero, st);
+    k_cheb_start<double><<<nb, 256, 0, s>>>(n, (const double*)b, (double*)r, (const double*)dinv, c2, ax, (double*)x,
+                                            (double*)d, x_is_zero, st, vs);
   else
-    k_cheb_start<float><<<grid_for(n, 256), 256, 0, s>>>(n, (const float*)b, (float*)r, (const float*)dinv,
-                                                         (float)c2, (float)ax, (float*)x, (float*)d, x_is_zero, st);
+    k_cheb_start<float><<<nb, 256, 0, s>>>(n, (const float*)b, (float*)r, (const float*)dinv, (float)c2, (float)ax,
+                                           (float*)x, (float*)d, x_is_zero, st, vs);
   TOPO_LAUNCH_CHECK();
 }
 
