@@ -61,7 +61,7 @@ def test_general_stiffness_is_not_taken():
 
 
 MESHES = [(1, 1, 1), (2, 1, 3), (1, 30, 2), (3, 2, 29), (5, 3, 30), (4, 5, 61), (6, 9, 40), (150, 2, 2), (9, 46, 17),
-          (3, 61, 92), (2, 2, 278), (2, 2, 279), (2, 3, 371), (2, 3, 372)]
+          (3, 61, 92), (2, 2, 185), (2, 2, 186), (2, 2, 278), (2, 2, 279), (2, 3, 371), (2, 3, 372)]
 
 
 @pytest.mark.gpu

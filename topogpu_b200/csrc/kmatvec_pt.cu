@@ -145,7 +145,9 @@ __device__ __forceinline__ void prefetch_l2(const void* b, const void* e) {
 }
 
 // Threads per CTA = 32 NW. MINB: CTAs per SM the registers are sized for.
-template <typename T, typename TU, bool BF, Epi EPI, int NW, int MINB>
+// COLS: several columns (a template flag: the column pointers cost registers
+// the one-column form has no room for).
+template <typename T, typename TU, bool BF, Epi EPI, bool COLS, int NW, int MINB>
 __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_constant__ Params<T> P) {
   if (P.st != nullptr && P.st->done) return;
   extern __shared__ __align__(128) unsigned char sm[];
@@ -154,9 +156,9 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Grid& g = P.g;
   const int NZ = g.NZ, PN = P.PN;
-  const long long co = (long long)blockIdx.y * P.vs;
-  const TU* const uc = P.list ? reinterpret_cast<const TU*>(P.ucol[blockIdx.y]) : reinterpret_cast<const TU*>(P.u) + co;
-  T* const yc = P.list ? P.ycol[blockIdx.y] : P.ep.y + co;
+  const long long co = COLS ? (long long)blockIdx.y * P.vs : 0LL;
+  const TU* const uc = COLS && P.list ? reinterpret_cast<const TU*>(P.ucol[blockIdx.y]) : reinterpret_cast<const TU*>(P.u) + co;
+  T* const yc = COLS && P.list ? P.ycol[blockIdx.y] : P.ep.y + co;
   const int w = (int)blockIdx.x % P.nwin, sg = (int)blockIdx.x / P.nwin;
   const int n0 = w * P.TO, n1 = min(PN, n0 + P.TO);  // output nodes of a plane
   const int xa = (int)((long long)g.NX * sg / P.nseg), xb = (int)((long long)g.NX * (sg + 1) / P.nseg);  // output planes
@@ -347,11 +349,10 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
     }
     Ep += le;
     const T En = (ev && p < pl) ? *Ep : (T)0;
-    // FP32: the epilogue's loads of plane p - 2 arrive behind the arithmetic
-    // of this step (FP64 has no registers left for them)
+    // the epilogue's loads of plane p - 2 arrive behind the arithmetic of this step
     Epv ev2;
     const bool fin = p - 2 >= xa;
-    if (ST == 4 && fin) fetch(p - 2, ev2);
+    if (fin) fetch(p - 2, ev2);
     transform(ucol + slot * P.slot + shift, b);
     V Ev;
     T t[3];
@@ -412,10 +413,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
         else backy(c, t[c], tc, buf);
       }
     }
-    if (fin) {
-      if (ST == 8) fetch(p - 2, ev2);
-      finish(p - 2, buf ^ 1, ev2);
-    }
+    if (fin) finish(p - 2, buf ^ 1, ev2);
     advance();
     return true;
   };
@@ -514,13 +512,16 @@ bool class_blocks(const double* KE, double* K) {
 }
 
 // Kernel widths: the (warps per CTA, CTAs per SM) pairs an instance is
-// compiled for, FP64 384 threads per SM (168 registers each), FP32 512 (128).
-// More threads with fewer registers spill: FP32 Store at 160x80x80 24.6 us
-// with 512 threads per SM, 30.4 with 768, 32.5 with 1024.
-template <typename T>
+// compiled for. FP32: 512 threads per SM (128 registers each); FP64: 384 (168),
+// for the Chebyshev epilogue with its five operands per DoF 256 (255). More
+// threads with fewer registers spill (160x80x80: FP32 Store 24.6 us with 512
+// threads per SM, 30.4 with 768, 32.5 with 1024; FP64 Chebyshev step at
+// 96x48x48 18 us with 256, 23 with 384).
+template <typename T, Epi EPI>
 struct Width {
-  static constexpr int NW[3] = {4, sizeof(T) == 8 ? 6 : 8, sizeof(T) == 8 ? 12 : 16};
-  static constexpr int PER[3] = {sizeof(T) == 8 ? 3 : 4, 2, 1};
+  static constexpr bool D = sizeof(T) == 8, C = D && EPI == Epi::ChebR;
+  static constexpr int NW[3] = {4, C ? 8 : D ? 6 : 8, C ? 8 : D ? 12 : 16};
+  static constexpr int PER[3] = {C ? 2 : D ? 3 : 4, C ? 1 : 2, 1};
 };
 constexpr int kPtSmem = 200 * 1024;  // dynamic shared memory of one CTA at most
 
@@ -534,24 +535,24 @@ struct PtLayout {
 // times the warps that share its SM (at least 8: below that a step is
 // latency and costs the same), over the waves of CTAs. A width that spends more
 // than 3/4 of its elements on the halo is left out; with none left (NZ above
-// 372, in FP64 279) the general kernels take the mesh.
-template <typename T>
+// 372, in FP64 186) the general kernels take the mesh.
+template <typename T, Epi EPI>
 bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
   const long long PN = (long long)g.NY * g.NZ;
   if (PN >= (1 << 28)) return false;
   double cost = 1e300;
   for (int w = 0; w < 3; ++w) {
-    const int NW = Width<T>::NW[w], TO = 31 * NW - g.NZ;
+    const int NW = Width<T, EPI>::NW[w], TO = 31 * NW - g.NZ;
     if (TO < 31 * NW / 4) continue;
     PtLayout L;
     L.w = w;
     L.TO = TO;
     L.nwin = (int)((PN + TO - 1) / TO);
-    const long long slots = std::max<long long>(1, (long long)nsm * Width<T>::PER[w] / nv);  // per column
+    const long long slots = std::max<long long>(1, (long long)nsm * Width<T, EPI>::PER[w] / nv);  // per column
     L.nseg = (int)std::max<long long>(1, std::min<long long>(g.NX, slots / L.nwin));
     const long long ctas = (long long)L.nwin * L.nseg;
     const double waves = std::ceil((double)ctas / (double)slots);
-    const double per = std::min<double>(Width<T>::PER[w], std::ceil((double)ctas * nv / nsm));
+    const double per = std::min<double>(Width<T, EPI>::PER[w], std::ceil((double)ctas * nv / nsm));
     const double c = waves * ((g.NX + L.nseg - 1) / L.nseg + 1) * std::max(8.0, per * NW);
     const auto al = [](long long x) { return (int)((x + 127) & ~127LL); };
     L.slot = al(64 + 3LL * s_u * (31 * NW + g.NZ + 3));
@@ -559,7 +560,7 @@ bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
     L.pw_n = (3 * 31 * NW + 3) & ~3;
     L.off_bar = L.off_pw + al(4LL * L.pw_n * (int)sizeof(T));
     L.total = L.off_bar + 128;
-    if (L.total <= kPtSmem / Width<T>::PER[w] && c < cost) {
+    if (L.total <= kPtSmem / Width<T, EPI>::PER[w] && c < cost) {
       cost = c;
       best = L;
     }
@@ -567,9 +568,9 @@ bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
   return cost < 1e300;
 }
 
-template <typename T, typename TU, bool BF, Epi EPI, int W>
+template <typename T, typename TU, bool BF, Epi EPI, int W, bool COLS>
 void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t s) {
-  auto* k = pt::k_level0_pt<T, TU, BF, EPI, Width<T>::NW[W], Width<T>::PER[W]>;
+  auto* k = pt::k_level0_pt<T, TU, BF, EPI, COLS, Width<T, EPI>::NW[W], Width<T, EPI>::PER[W]>;
   static std::atomic<uint64_t> raised{0};  // devices where this instance's shared-memory limit is raised
   int dev = 0;
   TOPO_CUDA_CHECK(cudaGetDevice(&dev));
@@ -577,7 +578,7 @@ void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t
     TOPO_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
     if (dev <= 63) raised |= 1ull << dev;
   }
-  k<<<dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T>::NW[W], L.total, s>>>(P);
+  k<<<dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T, EPI>::NW[W], L.total, s>>>(P);
   TOPO_LAUNCH_CHECK();
 }
 
@@ -585,7 +586,7 @@ template <typename T, typename TU, bool BF, Epi EPI>
 void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, const EpiArgs& ea, cudaStream_t s,
                int nv = 1, long long vs = 0, const void* const* ul = nullptr, void* const* yl = nullptr) {
   PtLayout L;
-  if (!pt_layout<T>(g, (int)sizeof(TU), nv, pt_device().nsm, L))
+  if (!pt_layout<T, EPI>(g, (int)sizeof(TU), nv, pt_device().nsm, L))
     throw std::runtime_error("level0 K.u: mesh not supported by the parity form");
   pt::Params<T> P;
   P.g = g;
@@ -613,11 +614,22 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   P.poll = 1 << 22;
   P.skip = 0;
   if (BF) wait_debug(P.skip, P.poll);
-  switch (L.w) {
-    case 0: launch_pt_w<T, TU, BF, EPI, 0>(L, P, nv, s); break;
-    case 1: launch_pt_w<T, TU, BF, EPI, 1>(L, P, nv, s); break;
-    default: launch_pt_w<T, TU, BF, EPI, 2>(L, P, nv, s); break;
+  auto go = [&](auto cols) {
+    constexpr bool C = decltype(cols)::value;
+    switch (L.w) {
+      case 0: launch_pt_w<T, TU, BF, EPI, 0, C>(L, P, nv, s); break;
+      case 1: launch_pt_w<T, TU, BF, EPI, 1, C>(L, P, nv, s); break;
+      default: launch_pt_w<T, TU, BF, EPI, 2, C>(L, P, nv, s); break;
+    }
+  };
+  if constexpr (EPI == Epi::Store || EPI == Epi::ChebR || EPI == Epi::RUpd) {
+    if (nv > 1 || ul) {
+      go(std::true_type{});
+      return;
+    }
   }
+  if (nv > 1) throw std::runtime_error("level0 K.u: this epilogue takes one column");
+  go(std::false_type{});
 }
 }  // namespace
 
@@ -658,7 +670,7 @@ bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
   const PtDevice& d = pt_device();
   PtLayout L;
   return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 &&
-         (f64 ? pt_layout<double>(g, 8, 1, d.nsm, L) : pt_layout<float>(g, 4, 1, d.nsm, L));
+         (f64 ? pt_layout<double, Epi::ChebR>(g, 8, 1, d.nsm, L) : pt_layout<float, Epi::ChebR>(g, 4, 1, d.nsm, L));  // (the narrowest)
 }
 
 // f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
