@@ -6,11 +6,11 @@
 // DoFs. The setup
 //   1. assembles the lower band into band storage,
 //   2. factorises it with one persistent kernel: a right-looking band
-//      Cholesky over 32-column panels with one grid barrier per panel; the
+//      Cholesky over 32-column panels ordered by two progress counters; the
 //      CTA that updates the next panel's diagonal block factors it in one
 //      warp's registers right away and publishes it (look-ahead), the others
-//      fetch the panel rows of their trailing tiles, solve them in two warps
-//      and update the tile; the factor goes to a separate band array so no
+//      fetch the panel rows of their trailing tiles meanwhile, solve them in
+//      two warps and update the tile; the factor goes to a separate band array so no
 //      CTA reads a panel row another CTA has overwritten,
 //   3. splits the rows into P diagonal blocks (boundaries on 32-row panels,
 //      each block at least `band` rows, so L is block bidiagonal and block
@@ -101,47 +101,57 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
-// Grid barrier over all CTAs of a cooperative launch on a monotonic counter:
-// barrier number `epoch` (1, 2, ...) is passed once the counter reaches
-// epoch * nblocks. Thread 0 arrives and polls with a bound (a timeout raises
-// err and is reported to every thread of the CTA).
-__device__ bool grid_barrier(unsigned* count, unsigned epoch, unsigned nblocks, int* err, int poll) {
-  __shared__ int s_ok;
+// Progress of a cooperative launch on monotonic counters: arrive adds one to
+// `count` after the CTA's writes, await polls (with a bound: a timeout raises
+// err and is reported to every thread of the CTA) until `count` reaches target.
+__device__ __forceinline__ void grid_arrive(unsigned* count, unsigned add) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    int ok = 1;
     __threadfence();
-    const unsigned target = epoch * nblocks;
-    if (atomicAdd(count, 1u) + 1u < target) {
-      int it = 0;
-      while (ld_acquire(count) < target) {
-        if (++it > poll) {
-          ok = 0;
-          atomicExch(err, 1);
-          break;
-        }
+    atomicAdd(count, add);
+  }
+}
+
+__device__ bool grid_await(const unsigned* count, unsigned target, int* err, int poll) {
+  __shared__ int s_ok;
+  if (threadIdx.x == 0) {
+    int ok = 1, it = 0;
+    while (ld_acquire(count) < target) {
+      if (++it > poll) {
+        ok = 0;
+        atomicExch(err, 1);
+        break;
       }
     }
     __threadfence();
     s_ok = ok;
   }
   __syncthreads();
-  return s_ok != 0;
+  const bool r = s_ok != 0;
+  __syncthreads();  // s_ok is written again by the next call
+  return r;
 }
 
 // ------------------------------------------------------ persistent Cholesky
-// Shared memory of one CTA: the panel's diagonal block (factored by warp 0
-// into Ld and its reciprocal pivots) and the solved panel rows of the two row
-// tiles of the trailing tile it updates.
-struct CholSmem {
-  double W[CNB][CNB + 1];
-  double Ld[CNB][CNB + 1];
+// Shared memory of one CTA: the panel's diagonal block W; of its factor the unit
+// multipliers MT[j][i] (column j over its pivot, by column) and the reciprocal
+// square roots of the pivots, and Ld, the columns themselves before that
+// scaling; the panel rows of the two row tiles of the trailing tile it updates
+// (by panel column, so that a lane per row and two rows per load are both free
+// of bank conflicts); CTA 0's copy of its next tile.
+struct __align__(16) CholSmem {
+  double Pi[CNB][CNB + 2];
+  double Pj[CNB][CNB + 2];
+  double A0[CNB][CNB + 2];
+  double MT[CNB][CNB + 2];   // MT and invd: published together
   double invd[CNB];
-  double col[CNB];
-  double Pi[CNB][CNB + 1];
-  double Pj[CNB][CNB + 1];
-  int bad;
+  double col[3][CNB];
+  double piv[CNB];
+  double Ld[CNB][CNB + 1];
+  double W[CNB][CNB + 1];
+  int bad, ok;
 };
+constexpr int LN = CNB * (CNB + 2) + CNB;  // doubles of one published factor
 
 __device__ __forceinline__ void tile_of(int t, int& ti, int& tj) {
   ti = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
@@ -150,54 +160,102 @@ __device__ __forceinline__ void tile_of(int t, int& ti, int& tj) {
   tj = t - ti * (ti + 1) / 2;
 }
 
-// One pivot of the warp-register factor of a 32x32 diagonal block (lane =
+// Two pivots of the warp-register factor of a 32x32 diagonal block (lane =
 // row). The pivot index is a template parameter so that every register index
-// is a compile-time constant (the array stays in registers). Column J is
-// broadcast through shared memory (one store per lane, broadcast reads);
-// entries right of a lane's diagonal are updated too but never read.
+// is a compile-time constant (the array stays in registers). Columns J and J+1
+// are broadcast through shared memory together. A warp issues in order and a
+// dependent FP64 operation takes about 40 cycles, so the chain is kept short
+// and free of branches: the second pivot q1 = d1 - l^2 / d0 is inverted as
+// d0 / (d0 d1 - l^2), with the determinant as a difference of products that
+// keeps its relative accuracy (Kahan: the rounding of l^2 is taken out again),
+// so both reciprocals run side by side. A reciprocal is the hardware's
+// approximation r (2^-23) and one third-order step r (1 + e + e^2),
+// e = 1 - d r, which cubes the error. The square roots of all pivots follow
+// once at the end. Entries right of a lane's diagonal are updated too but never
+// read.
 template <int J>
 __device__ __forceinline__ void chol_step(double (&wr)[CNB], int lane, CholSmem& S, bool& bad) {
-  S.col[lane] = wr[J];
+  const double c0 = wr[J], c1 = wr[J + 1];
+  S.col[0][lane] = c0;
+  S.col[1][lane] = c1;
   __syncwarp();
-  const double d = S.col[J];
-  const bool ok = d > 0.0 && isfinite(d);
-  const double dd = ok ? d : 1.0;
-  const double rs = rsqrt(dd);
-  const double lj = wr[J];
-  if (lane == J) {
-    bad |= !ok;
-    S.Ld[J][J] = dd * rs;
-    S.invd[J] = rs;
-  } else {
-    S.Ld[lane][J] = lane > J ? lj * rs : 0.0;
+  const double d0 = S.col[0][J], l = S.col[0][J + 1], d1 = S.col[1][J + 1];
+  const double ll = l * l, det = fma(d0, d1, -ll) - fma(l, l, -ll);
+  double e0 = d0, e1, r0, r1, t;
+  if (d0 > 1e-290 && d0 < 1e290 && det > 1e-290 && det < 1e290) {
+    double ra, rb;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(d0));
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(rb) : "d"(det));
+    const double ea = fma(-d0, ra, 1.0), eb = fma(-det, rb, 1.0);
+    r0 = fma(ra, fma(ea, ea, ea), ra);
+    r1 = d0 * fma(rb, fma(eb, eb, eb), rb);
+    t = l * r0;
+    e1 = det * r0;
+  } else {  // a pivot that is not positive, or out of range (it is then taken as 1)
+    const bool ok0 = d0 > 0.0 && isfinite(d0);
+    e0 = ok0 ? d0 : 1.0;
+    r0 = 1.0 / e0;
+    t = l * r0;
+    e1 = fma(-l, t, d1);
+    const bool ok1 = e1 > 0.0 && isfinite(e1);
+    if (!ok1) e1 = 1.0;
+    r1 = 1.0 / e1;
+    bad |= !ok0 || !ok1;
   }
-  const double w = lj * (rs * rs);
-#pragma unroll
-  for (int t = J + 1; t < CNB; ++t) wr[t] = fma(-S.col[t], w, wr[t]);
+  const double p1 = fma(-c0, t, c1);  // this lane's entry of column J+1 after pivot J
+  S.col[2][lane] = p1;
+  const double w0 = c0 * r0, w1 = p1 * r1;
   __syncwarp();
-  if constexpr (J + 1 < CNB) chol_step<J + 1>(wr, lane, S, bad);
-}
-
-// Panel row i (columns k .. k+nb) into registers; zero past `lim` or outside
-// the band.
-__device__ __forceinline__ void panel_load(const double* A, int band, long long ldb, int k, int nb, int i, int lim,
-                                           double (&x)[CNB]) {
 #pragma unroll
-  for (int j = 0; j < CNB; ++j)
-    x[j] = (i < lim && j < nb && i - (k + j) <= band) ? ldcg(A + bidx(i, k + j, band, ldb)) : 0.0;
+  for (int q = J + 2; q < CNB; q += 2) {
+    const double2 a = *reinterpret_cast<const double2*>(&S.col[0][q]), b = *reinterpret_cast<const double2*>(&S.col[2][q]);
+    wr[q] = fma(-b.x, w1, fma(-a.x, w0, wr[q]));
+    wr[q + 1] = fma(-b.y, w1, fma(-a.y, w0, wr[q + 1]));
+  }
+  S.MT[J][lane] = w0;
+  S.MT[J + 1][lane] = w1;
+  S.Ld[lane][J] = lane == J ? e0 : c0;
+  S.Ld[lane][J + 1] = lane == J + 1 ? e1 : p1;
+  if (lane == 0) {
+    S.piv[J] = e0;
+    S.piv[J + 1] = e1;
+  }
+  if constexpr (J + 2 < CNB) chol_step<J + 2>(wr, lane, S, bad);
 }
 
-// x Ld^T = a for one row, column by column with the reciprocal pivots.
+// Rows i .. i+31 of panel k (columns k .. k+nb) to P[column][row], zero past
+// `lim` or outside the band: warp w of nw takes every nw-th row, lanes along
+// the columns (a row is 256 contiguous bytes).
+__device__ __forceinline__ void panel_load(const double* A, int band, long long ldb, int k, int nb, int i, int lim,
+                                           double (*P)[CNB + 2], int w, int nw, int lane) {
+#pragma unroll 8
+  for (int r = w; r < CNB; r += nw)
+    P[lane][r] = (i + r < lim && lane < nb && i + r - (k + lane) <= band) ? ldcg(A + bidx(i + r, k + lane, band, ldb)) : 0.0;
+}
+
+// x Ld^T = a for one row: forward substitution with the unit multipliers (one
+// dependent operation per column), scaled by the reciprocal pivots at the end.
 template <int J>
 __device__ __forceinline__ void solve_step(double (&x)[CNB], const CholSmem& S) {
-  x[J] *= S.invd[J];
 #pragma unroll
-  for (int q = J + 1; q < CNB; ++q) x[q] -= x[J] * S.Ld[q][J];
+  for (int q = (J + 1) & ~1; q < CNB; q += 2) {
+    const double2 m = *reinterpret_cast<const double2*>(&S.MT[J][q]);
+    if (q > J) x[q] = fma(-x[J], m.x, x[q]);
+    x[q + 1] = fma(-x[J], m.y, x[q + 1]);
+  }
   if constexpr (J + 1 < CNB) solve_step<J + 1>(x, S);
 }
+__device__ __forceinline__ void solve_rows(double (*P)[CNB + 2], const CholSmem& S, int lane) {
+  double x[CNB];
+#pragma unroll
+  for (int j = 0; j < CNB; ++j) x[j] = P[j][lane];
+  solve_step<0>(x, S);
+#pragma unroll
+  for (int j = 0; j < CNB; ++j) P[j][lane] = x[j] * S.invd[j];
+}
 
-// Warp 0 factors S.W into S.Ld and the reciprocal pivots S.invd; S.bad is
-// set when a pivot was not positive (it is then taken as 1).
+// Warp 0 factors S.W into S.MT, S.Ld and S.invd; S.bad is set when a pivot was
+// not positive (it is then taken as 1).
 __device__ __forceinline__ void factor_block(CholSmem& S, int warp, int lane) {
   if (warp == 0) {
     double wr[CNB];
@@ -205,30 +263,49 @@ __device__ __forceinline__ void factor_block(CholSmem& S, int warp, int lane) {
     for (int t = 0; t < CNB; ++t) wr[t] = S.W[lane][t];
     bool bad = false;
     chol_step<0>(wr, lane, S, bad);
-    bad = __any_sync(0xffffffffu, bad);
+    __syncwarp();
+    S.invd[lane] = rsqrt(S.piv[lane]);
     if (lane == 0) S.bad = bad ? 1 : 0;
   }
 }
 
 // Warps: 0 factors diagonal blocks, 2 and 3 solve the panel rows of the two
 // row tiles of each trailing tile (3 only for off-diagonal tiles), all 256
-// threads update the tile (four outputs each). Look-ahead (band >= 32):
-// tile 0 of panel k's trailing update, which CTA 0 owns, is panel k+1's
-// diagonal block; CTA 0 keeps its updated values, factors them after its
-// tiles and publishes the factor and pivots in Lnext (double-buffered by
-// panel parity) before the barrier, so at panel k+1 the other CTAs load it
-// instead of factoring, and the panel rows they prefetch meanwhile are the
-// only load in front of their solves. Panel 0, and every panel when the
-// band is narrower than a panel, is factored by every CTA from A.
+// threads update the tile (2x2 outputs each, two partial sums). Look-ahead
+// (band >= 32): tile 0 of panel k's trailing update, which CTA 0 owns, is panel
+// k+1's diagonal block; CTA 0 keeps its updated values, factors them and
+// publishes the factor in Lnext (double-buffered by panel parity), so at panel
+// k+1 the other CTAs load it instead of factoring. Panel 0, and every panel when
+// the band is narrower than a panel, is factored by every CTA from A.
+//
+// Order between the panels: count[0] counts the CTAs that have written their
+// tiles of a panel, count[32] the published factors. The chain of a panel is
+// CTA 0's solve, update, factor and publication; while warp 0 factors, warps
+// 4-7 write the factor rows of L, wait for the other CTAs' tiles and fetch the
+// next panel's rows. The others fetch their rows while they wait for the
+// factor.
+//
+// Bound by that chain (about 14,000 cycles per panel at band 401: solve 2,700,
+// update 1,600, factor 7,200, publication 1,000). With one barrier per panel
+// behind a factor of one pivot per round, its square root on the chain, and
+// everything above in sequence: 25,000 cycles, 2.97 ms at n = 7,260; now 1.93 ms.
 __global__ void __launch_bounds__(256, 1) k_band_chol(int n, int band, long long ldb, double* A, double* L,
-                                                      double* Lnext, int* flag, unsigned* bar_count, int* err,
-                                                      int poll) {
+                                                      double* Lnext, int* flag, unsigned* count, int* err, int poll) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   CholSmem& S = *reinterpret_cast<CholSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool solver = warp == 2 || warp == 3;
   const bool ahead = band >= CNB;
-  constexpr int LN = CNB * (CNB + 1) + CNB;  // one published factor: Ld rows, then pivots
+  const int tr = (tid >> 4) * 2, tc = (tid & 15) * 2;  // this thread's 2x2 outputs of a tile
+  bool pre = false;  // CTA 0: Pi and A0 hold this panel's first tile already
+  auto tile_load = [&](int i0, int j0, int lim, double (&v)[2][2]) {
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int i = i0 + tr + a, j = j0 + tc + b;
+        v[a][b] = (i < lim && j < lim && j <= i && i - j <= band) ? ldcg(A + bidx(i, j, band, ldb)) : 0.0;
+      }
+  };
   for (int k = 0; k < n; k += CNB) {
     const int nb = min(CNB, n - k);
     const int base = k + nb;
@@ -237,112 +314,154 @@ __global__ void __launch_bounds__(256, 1) k_band_chol(int n, int band, long long
     const int ntiles = lim > base ? nt * (nt + 1) / 2 : 0;
     const int par = (k / CNB) & 1;
     const bool own = ahead && k > 0;  // this panel's factor came from the look-ahead
-    // 1. this panel's factored diagonal block and the first tile's panel rows
-    if (!own) {
-      for (int q = tid; q < CNB * CNB; q += blockDim.x) {
-        const int i = q / CNB, j = q % CNB;
-        S.W[i][j] = (i < nb && j < nb && j <= i) ? (i - j <= band ? ldcg(A + bidx(k + i, k + j, band, ldb)) : 0.0)
-                                                 : (i == j ? 1.0 : 0.0);
+    const unsigned pi = (unsigned)(k / CNB);
+    // 1. the first tile's panel rows and values, and the factored diagonal block
+    double a0[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    if (!pre) {
+      if (k > 0 && !grid_await(count, pi * gridDim.x, err, poll)) return;
+      if ((int)blockIdx.x < ntiles) {
+        int ti, tj;
+        tile_of(blockIdx.x, ti, tj);
+        panel_load(A, band, ldb, k, nb, base + CNB * ti, lim, S.Pi, warp, 8, lane);
+        if (tj != ti) panel_load(A, band, ldb, k, nb, base + CNB * tj, lim, S.Pj, warp, 8, lane);
+        tile_load(base + CNB * ti, base + CNB * tj, lim, a0);
       }
-    } else if (blockIdx.x != 0) {
-      const double* src = Lnext + par * LN;
-      for (int q = tid; q < CNB * (CNB + 1); q += blockDim.x) (&S.Ld[0][0])[q] = ldcg(src + q);
-      if (tid < CNB) S.invd[tid] = ldcg(src + CNB * (CNB + 1) + tid);
-    }
-    double x[CNB];
-    const int r = tid >> 3, c0 = (tid & 7) * 4;  // this thread's four outputs of a trailing tile
-    double a0[4] = {0.0, 0.0, 0.0, 0.0};        // their current values for the first tile
-    if ((int)blockIdx.x < ntiles) {
-      int ti, tj;
-      tile_of(blockIdx.x, ti, tj);
-      if (solver) panel_load(A, band, ldb, k, nb, (warp == 2 ? base + CNB * ti : base + CNB * tj) + lane, lim, x);
-      const int i = base + CNB * ti + r;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int j = base + CNB * tj + c0 + m;
-        if (i < lim && j < lim && j <= i && i - j <= band) a0[m] = ldcg(A + bidx(i, j, band, ldb));
-      }
-    }
-    __syncthreads();
-    if (!own) {
-      // every CTA does the same arithmetic, so all agree
-      factor_block(S, warp, lane);
-      __syncthreads();
-      if (blockIdx.x == 0) {
+      if (!own) {
         for (int q = tid; q < CNB * CNB; q += blockDim.x) {
           const int i = q / CNB, j = q % CNB;
-          if (i < nb && j <= i && i - j <= band) L[bidx(k + i, k + j, band, ldb)] = S.Ld[i][j];
+          S.W[i][j] = (i < nb && j < nb && j <= i) ? (i - j <= band ? ldcg(A + bidx(k + i, k + j, band, ldb)) : 0.0)
+                                                   : (i == j ? 1.0 : 0.0);
         }
-        if (tid == 0 && S.bad) *flag = 1;
+      } else if (blockIdx.x != 0) {
+        if (!grid_await(count + 32, pi, err, poll)) return;
+        const double* src = Lnext + par * LN;
+        for (int q = tid; q < LN; q += blockDim.x) (&S.MT[0][0])[q] = ldcg(src + q);
+      }
+      __syncthreads();
+      if (!own) {
+        // every CTA does the same arithmetic, so all agree
+        factor_block(S, warp, lane);
+        __syncthreads();
+        if (blockIdx.x == 0) {
+          for (int q = tid; q < CNB * CNB; q += blockDim.x) {
+            const int i = q / CNB, j = q % CNB;
+            if (i < nb && j <= i && i - j <= band) L[bidx(k + i, k + j, band, ldb)] = S.Ld[i][j] * S.invd[j];
+          }
+          if (tid == 0 && S.bad) *flag = 1;
+        }
       }
     }
     // 2. trailing tiles of the band window
     const bool la = ahead && blockIdx.x == 0 && base < n;  // CTA 0 builds panel k+1's block in S.W
+    // factor rows of a diagonal tile (its owner writes them; L is not read here)
+    auto write_rows = [&](int i0, int t, int nthr) {
+      for (int q = t; q < CNB * CNB; q += nthr) {
+        const int r = q / CNB, j = q % CNB, i = i0 + r;
+        if (i < lim && j < nb && i - (k + j) <= band) L[bidx(i, k + j, band, ldb)] = S.Pi[j][r];
+      }
+    };
+    int late = -1;  // first row of the diagonal tile whose factor rows are still to be written
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       int ti, tj;
       tile_of(t, ti, tj);
       const int i0 = base + CNB * ti, j0 = base + CNB * tj;
       if (i0 - (j0 + CNB - 1) > band) continue;  // whole tile outside the band (uniform)
-      if (warp == 2 || (warp == 3 && tj != ti)) {
-        if (t != (int)blockIdx.x) panel_load(A, band, ldb, k, nb, (warp == 2 ? i0 : j0) + lane, lim, x);
-        solve_step<0>(x, S);
-        double(*P)[CNB + 1] = warp == 2 ? S.Pi : S.Pj;
-#pragma unroll
-        for (int j = 0; j < CNB; ++j) P[lane][j] = x[j];
+      if (t != (int)blockIdx.x) {
+        if (late >= 0) write_rows(late, tid, 256);
+        late = -1;
+        __syncthreads();
+        panel_load(A, band, ldb, k, nb, i0, lim, S.Pi, warp, 8, lane);
+        if (tj != ti) panel_load(A, band, ldb, k, nb, j0, lim, S.Pj, warp, 8, lane);
+        tile_load(i0, j0, lim, a0);
+        __syncthreads();
       }
+      if (warp == 2) solve_rows(S.Pi, S, lane);
+      if (warp == 3 && tj != ti) solve_rows(S.Pj, S, lane);
       __syncthreads();
-      double(*Pj)[CNB + 1] = (tj == ti) ? S.Pi : S.Pj;
-      if (tj == ti) {
-        // owner of the diagonal tile writes the factor rows of this row tile
-        for (int q = tid; q < CNB * CNB; q += blockDim.x) {
-          const int r = q / CNB, j = q % CNB;
-          const int i = i0 + r;
-          if (i < lim && j < nb && i - (k + j) <= band) L[bidx(i, k + j, band, ldb)] = S.Pi[r][j];
-        }
-      }
-      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+      double(*Pj)[CNB + 2] = (tj == ti) ? S.Pi : S.Pj;
+      if (tj == ti) late = i0;
+      double acc[2][2][2] = {};
 #pragma unroll 8
       for (int q = 0; q < CNB; ++q) {
-        const double li = S.Pi[r][q];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) acc[m] = fma(li, Pj[c0 + m][q], acc[m]);
+        const double2 li = *reinterpret_cast<const double2*>(&S.Pi[q][tr]), lj = *reinterpret_cast<const double2*>(&Pj[q][tc]);
+        acc[q & 1][0][0] = fma(li.x, lj.x, acc[q & 1][0][0]);
+        acc[q & 1][0][1] = fma(li.x, lj.y, acc[q & 1][0][1]);
+        acc[q & 1][1][0] = fma(li.y, lj.x, acc[q & 1][1][0]);
+        acc[q & 1][1][1] = fma(li.y, lj.y, acc[q & 1][1][1]);
       }
-      const int i = i0 + r;
       const bool blk = la && t == 0;  // tile 0 = panel k+1's diagonal block
-      // all four loads before any store (the stores could alias them)
-      double av[4];
-      bool in[4];
+      const bool held = pre && t == (int)blockIdx.x;
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        const int j = j0 + c0 + m;
-        in[m] = i < lim && j < lim && j <= i && i - j <= band;
-        const double cur = t == (int)blockIdx.x ? a0[m] : (in[m] ? ldcg(A + bidx(i, j, band, ldb)) : 0.0);
-        av[m] = in[m] ? cur - acc[m] : 0.0;
-      }
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int m = 0; m < 4; ++m) {
-        if (in[m]) A[bidx(i, j0 + c0 + m, band, ldb)] = av[m];
-        // band >= 32: every entry of the block on or below the diagonal and
-        // below row n is in the window; rows past n are identity-padded
-        if (blk) S.W[r][c0 + m] = in[m] ? av[m] : ((i >= n && r == c0 + m) ? 1.0 : 0.0);
-      }
+        for (int b = 0; b < 2; ++b) {
+          const int i = i0 + tr + a, j = j0 + tc + b;
+          const bool in = i < lim && j < lim && j <= i && i - j <= band;
+          const double v = in ? (held ? S.A0[tc + b][tr + a] : a0[a][b]) - (acc[0][a][b] + acc[1][a][b]) : 0.0;
+          if (in && !blk) A[bidx(i, j, band, ldb)] = v;  // (the block is factored from W and not read again)
+          // band >= 32: every entry of the block on or below the diagonal and
+          // below row n is in the window; rows past n are identity-padded
+          if (blk) S.W[tr + a][tc + b] = in ? v : ((i >= n && tr + a == tc + b) ? 1.0 : 0.0);
+        }
       __syncthreads();
     }
-    if (la) {
-      // 3. look-ahead: factor panel k+1's block, publish it, write its L block
+    pre = false;
+    if (!la) {
+      grid_arrive(count, 1u);  // this CTA's tiles of panel k are written
+      if (late >= 0) write_rows(late, tid, 256);
+      continue;
+    }
+    // 3. CTA 0: factor panel k+1's block; beside it arrive, write L, fetch panel k+1's first tile
+    const int nb1 = min(CNB, n - base), base1 = base + nb1, lim1 = min(n, base1 + band);
+    auto bar47 = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+    if (warp >= 4) {
+      const int t4 = tid - 128;
+      if (t4 == 0) {
+        __threadfence();
+        atomicAdd(count, 1u);
+      }
+      if (late >= 0) write_rows(late, t4, 128);
+      bar47();  // the rows in Pi are written
+      if (t4 == 0) {
+        int ok = 1, it = 0;
+        while (ld_acquire(count) < (pi + 1) * gridDim.x)
+          if (++it > poll) {
+            ok = 0;
+            atomicExch(err, 1);
+            break;
+          }
+        __threadfence();
+        S.ok = ok;
+      }
+      bar47();
+      if (S.ok && base1 < lim1) {
+        panel_load(A, band, ldb, base, nb1, base1, lim1, S.Pi, warp - 4, 4, lane);
+        for (int q = t4; q < CNB * CNB; q += 128) {
+          const int r = q / CNB, c = q % CNB, i = base1 + r, j = base1 + c;
+          S.A0[c][r] = (i < lim1 && j <= i && i - j <= band) ? ldcg(A + bidx(i, j, band, ldb)) : 0.0;
+        }
+      }
+    } else {
       factor_block(S, warp, lane);
-      __syncthreads();
-      const int nb1 = min(CNB, n - base);
+      asm volatile("bar.sync 2, 128;" ::: "memory");  // warps 0-3: the factor is there
       double* dst = Lnext + (par ^ 1) * LN;
-      for (int q = tid; q < CNB * (CNB + 1); q += blockDim.x) dst[q] = (&S.Ld[0][0])[q];
-      if (tid < CNB) dst[CNB * (CNB + 1) + tid] = S.invd[tid];
-      for (int q = tid; q < CNB * CNB; q += blockDim.x) {
-        const int i = q / CNB, j = q % CNB;
-        if (i < nb1 && j <= i && i - j <= band) L[bidx(base + i, base + j, band, ldb)] = S.Ld[i][j];
-      }
+      for (int q = tid; q < LN; q += 128) dst[q] = (&S.MT[0][0])[q];
       if (tid == 0 && S.bad) *flag = 1;
+      asm volatile("bar.sync 2, 128;" ::: "memory");
+      if (tid == 0) {
+        __threadfence();
+        atomicAdd(count + 32, 1u);
+      }
     }
-    if (!grid_barrier(bar_count, (unsigned)(k / CNB + 1), gridDim.x, err, poll)) return;
+    __syncthreads();
+    if (!S.ok) return;
+    pre = true;
+    if (warp >= 4) {
+      for (int q = tid - 128; q < CNB * CNB; q += 128) {
+        const int i = q / CNB, j = q % CNB;
+        if (i < nb1 && j <= i && i - j <= band) L[bidx(base + i, base + j, band, ldb)] = S.Ld[i][j] * S.invd[j];
+      }
+    }
   }
 }
 
@@ -763,7 +882,7 @@ void coarsest_alloc(CoarsestFactor& f, const CoarsestPlan& p, int band, bool f64
   f.A = (double*)A(nbs * sizeof(double));
   f.L = (double*)A(nbs * sizeof(double));
   f.Dinv = (double*)A((size_t)std::max(p.nt, 1) * cst::CNB * cst::CNB * sizeof(double));
-  f.Lnext = (double*)A(2 * (size_t)(cst::CNB * (cst::CNB + 1) + cst::CNB) * sizeof(double));
+  f.Lnext = (double*)A(2 * (size_t)cst::LN * sizeof(double));
   // diagonal blocks of W: at least max(4 band, 512) rows each (every block at
   // least `band` rows), boundaries on 32-row panels
   CoarseBlocks& bk = f.blk;
@@ -794,7 +913,7 @@ void coarsest_alloc(CoarsestFactor& f, const CoarsestPlan& p, int band, bool f64
   f.W64 = (double*)A((size_t)off * sizeof(double));
   f.C = f64 ? (void*)f.W64 : A((size_t)off * sizeof(float));
   f.flag = (int*)A(sizeof(int) * 4);
-  f.bar = (unsigned*)A(sizeof(unsigned) * 4);
+  f.bar = (unsigned*)A(sizeof(unsigned) * 64);  // the two counters in lines of their own
   f.err = f.flag + 1;
   // persistent factorisation: cooperative grid sized by co-residency
   int dev = 0, nsm = 0, per_sm = 0;
@@ -834,7 +953,7 @@ void coarsest_factor(CoarsestFactor& f, cudaStream_t s) {
   const int n = p.n;
   if (n == 0) return;
   TOPO_CUDA_CHECK(cudaMemsetAsync(f.flag, 0, sizeof(int) * 4, s));
-  TOPO_CUDA_CHECK(cudaMemsetAsync(f.bar, 0, sizeof(unsigned) * 4, s));
+  TOPO_CUDA_CHECK(cudaMemsetAsync(f.bar, 0, sizeof(unsigned) * 64, s));
   TOPO_CUDA_CHECK(cudaMemsetAsync(f.L, 0, sizeof(double) * (size_t)n * f.ldb, s));
   {
     int nn = n, band = f.band;
