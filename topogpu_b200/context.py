@@ -32,7 +32,7 @@ def _ptr(t: torch.Tensor, dtype=None, n=None, name="tensor") -> int:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())  # without building a Stream object
 
 
 class TopoContext:

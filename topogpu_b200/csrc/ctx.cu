@@ -218,6 +218,11 @@ struct topo_ctx {
   bool ke_registered = false;  // holds a reference on its device's KE
   cudaStream_t cs = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
+  // the last call's stream and the event behind its work: a call on another
+  // stream waits for it (has_last: there is such a call)
+  cudaStream_t last = nullptr;
+  cudaEvent_t ev_last = nullptr, ev_dir = nullptr;
+  bool has_last = false;
   cudaEvent_t ev_ph[6] = {};     // setup phase marks (timed)
   double setup_ms[5] = {0, 0, 0, 0, 0};
   std::vector<void*> allocs;
@@ -240,16 +245,57 @@ struct topo_ctx {
 
 namespace {
 
+// A stream under capture: its events must not be waited for outside the graph,
+// so such a call leaves the bookkeeping of the last call alone.
+bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return st != cudaStreamCaptureStatusNone;
+}
+
+// Calls of many kernels run on the context's own stream between two events.
 struct StreamGuard {
   topo_ctx* c;
   cudaStream_t user;
+  bool cap;
   StreamGuard(topo_ctx* ctx, void* stream) : c(ctx), user((cudaStream_t)stream) {
     TOPO_CUDA_CHECK(cudaSetDevice(c->device));
+    cap = capturing(user);
+    if (!cap && c->has_last && c->last != user) TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_last, 0));
     TOPO_CUDA_CHECK(cudaEventRecord(c->ev_in, user));
     TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_in, 0));
   }
   ~StreamGuard() {
     if (cudaEventRecord(c->ev_out, c->cs) == cudaSuccess) cudaStreamWaitEvent(user, c->ev_out, 0);
+    if (!cap) {
+      c->last = user;
+      c->ev_last = c->ev_out;
+      c->has_last = true;
+    }
+  }
+};
+
+// Calls of one or a few kernels run on the caller's stream itself: two event
+// records and two waits less per call (matvec of 24x12x6: 11.8 us per call
+// before, 8.5 us now, kernel 4.4 us). Order with the calls before is by the
+// stream, or by ev_last where the stream changed.
+struct DirectGuard {
+  topo_ctx* c;
+  cudaStream_t user;
+  bool cap;
+  DirectGuard(topo_ctx* ctx, void* stream) : c(ctx), user((cudaStream_t)stream) {
+    TOPO_CUDA_CHECK(cudaSetDevice(c->device));
+    cap = capturing(user);
+    if (!cap && c->has_last && c->last != user) TOPO_CUDA_CHECK(cudaStreamWaitEvent(user, c->ev_last, 0));
+  }
+  ~DirectGuard() {
+    if (cap || cudaEventRecord(c->ev_dir, user) != cudaSuccess) return;
+    c->last = user;
+    c->ev_last = c->ev_dir;
+    c->has_last = true;
   }
 };
 
@@ -1223,6 +1269,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     TOPO_CUDA_CHECK(cudaStreamCreateWithFlags(&c->cs, cudaStreamNonBlocking));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming));
+    TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_dir, cudaEventDisableTiming));
     for (auto& e : c->ev_ph) TOPO_CUDA_CHECK(cudaEventCreate(&e));
     TOPO_CUDA_CHECK(cudaStreamCreateWithFlags(&c->C.bg_stream, cudaStreamNonBlocking));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->C.ev_copy, cudaEventDisableTiming));
@@ -1307,6 +1354,7 @@ int topo_ctx_destroy(topo_ctx* c) {
   if (!c) return 0;
   cudaSetDevice(c->device);
   if (c->cs) cudaStreamSynchronize(c->cs);
+  if (c->has_last) cudaEventSynchronize(c->ev_last);
   release_ke(c);
   for (void* p : c->allocs) cudaFree(p);
   if (c->h_st) cudaFreeHost(c->h_st);
@@ -1322,6 +1370,7 @@ int topo_ctx_destroy(topo_ctx* c) {
   if (c->C.side) cudaStreamDestroy(c->C.side);
   if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->ev_out) cudaEventDestroy(c->ev_out);
+  if (c->ev_dir) cudaEventDestroy(c->ev_dir);
   for (auto& e : c->ev_ph)
     if (e) cudaEventDestroy(e);
   if (c->cs) cudaStreamDestroy(c->cs);
@@ -1429,8 +1478,9 @@ int topo_set_problem(topo_ctx* c, const uint8_t* free_mask, const double* F, voi
 int topo_modulus(topo_ctx* c, const double* rho, double penal, double E0, double Emin, double* E, void* stream) {
   try {
     if (!c || !rho || !E) throw std::invalid_argument("topo_modulus: null pointer");
-    StreamGuard sg(c, stream);
-    modulus(c->L[0].g.nelem, rho, penal, E0, Emin, E, nullptr, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    modulus(c->L[0].g.nelem, rho, penal, E0, Emin, E, nullptr, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1441,14 +1491,15 @@ int topo_matvec(topo_ctx* c, int dtype, const void* u, void* y, const void* E, v
   try {
     if (!c || !u || !y || !E) throw std::invalid_argument("topo_matvec: null pointer");
     if (!c->problem_set) throw std::runtime_error("topo_matvec: call topo_set_problem first");
-    StreamGuard sg(c, stream);
-    if (xs_error_flag(c->cs, false))
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    if (xs_error_flag(us, false))
       throw std::runtime_error("level-0 K.u: an mbarrier wait of an earlier launch timed out");
     Level& L0 = c->L[0];
     EpiArgs ea{};
-    if (dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, Epi::Store, ea, c->cs);
-    else if (dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, Epi::Store, ea, c->cs);
-    else if (dtype == TOPO_BF16) level0_apply_bf16(c->use_tc, true, L0.g, u, E, L0.mask, c->nmask0, y, Epi::Store, ea, c->cs);
+    if (dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, Epi::Store, ea, us);
+    else if (dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, Epi::Store, ea, us);
+    else if (dtype == TOPO_BF16) level0_apply_bf16(c->use_tc, true, L0.g, u, E, L0.mask, c->nmask0, y, Epi::Store, ea, us);
     else throw std::invalid_argument("topo_matvec: bad dtype");
     return 0;
   } catch (const std::exception& e) {
@@ -1477,8 +1528,9 @@ int topo_level0_apply(topo_ctx* c, int u_dtype, int epi, const void* u, const vo
         break;
       default: throw std::invalid_argument("topo_level0_apply: bad epilogue");
     }
-    StreamGuard sg(c, stream);
-    if (xs_error_flag(c->cs, false))
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    if (xs_error_flag(us, false))
       throw std::runtime_error("level-0 K.u: an mbarrier wait of an earlier launch timed out");
     Level& L0 = c->L[0];
     EpiArgs ea{};
@@ -1491,10 +1543,10 @@ int topo_level0_apply(topo_ctx* c, int u_dtype, int epi, const void* u, const vo
     ea.c1 = c1;
     ea.c2 = c2;
     ea.ax = ax;
-    if (u_dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, ep, ea, c->cs);
-    else if (u_dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, ep, ea, c->cs);
+    if (u_dtype == TOPO_F64) level0_apply(Prec::F64, L0.g, u, E, L0.mask, y, ep, ea, us);
+    else if (u_dtype == TOPO_F32) level0_apply(Prec::F32, L0.g, u, E, L0.mask, y, ep, ea, us);
     else if (u_dtype == TOPO_BF16 || u_dtype == TOPO_BF16_F32IN)
-      level0_apply_bf16(c->use_tc, u_dtype == TOPO_BF16, L0.g, u, E, L0.mask, c->nmask0, y, ep, ea, c->cs);
+      level0_apply_bf16(c->use_tc, u_dtype == TOPO_BF16, L0.g, u, E, L0.mask, c->nmask0, y, ep, ea, us);
     else {
       throw std::invalid_argument("topo_level0_apply: bad dtype");
     }
@@ -1540,8 +1592,9 @@ int topo_diag(topo_ctx* c, const double* E, double* diag, void* stream) {
   try {
     if (!c || !E || !diag) throw std::invalid_argument("topo_diag: null pointer");
     if (!c->problem_set) throw std::runtime_error("topo_diag: call topo_set_problem first");
-    StreamGuard sg(c, stream);
-    level0_diag(c->L[0].g, E, c->L[0].mask, diag, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    level0_diag(c->L[0].g, E, c->L[0].mask, diag, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1564,10 +1617,11 @@ int topo_gmg_apply(topo_ctx* c, const void* r, void* z, void* stream) {
   try {
     if (!c || !r || !z) throw std::invalid_argument("topo_gmg_apply: null pointer");
     if (!c->setup_done) throw std::runtime_error("topo_gmg_apply: call topo_gmg_setup first");
-    StreamGuard sg(c, stream);
-    if (xs_error_flag(c->cs, false))
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    if (xs_error_flag(us, false))
       throw std::runtime_error("level-0 K.u: an mbarrier wait of an earlier launch timed out");
-    vcycle_apply(c, r, z, nullptr, c->cs, c->mode == TOPO_MODE_MIXED);
+    vcycle_apply(c, r, z, nullptr, us, c->mode == TOPO_MODE_MIXED);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1650,8 +1704,9 @@ int topo_sensitivity(topo_ctx* c, const void* u, int u_dtype, const double* rho,
   try {
     if (!c || !u || !rho || !dc) throw std::invalid_argument("topo_sensitivity: null pointer");
     if (u_dtype != TOPO_F64 && u_dtype != TOPO_F32) throw std::invalid_argument("topo_sensitivity: bad dtype");
-    StreamGuard sg(c, stream);
-    sensitivity(c->L[0].g, u, nullptr, u_dtype == TOPO_F32, rho, penal, E0, Emin, dc, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    sensitivity(c->L[0].g, u, nullptr, u_dtype == TOPO_F32, rho, penal, E0, Emin, dc, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1663,8 +1718,9 @@ int topo_sensitivity_adjoint(topo_ctx* c, const void* u, const void* lam, int dt
   try {
     if (!c || !u || !lam || !rho || !dc) throw std::invalid_argument("topo_sensitivity_adjoint: null pointer");
     if (dtype != TOPO_F64 && dtype != TOPO_F32) throw std::invalid_argument("topo_sensitivity_adjoint: bad dtype");
-    StreamGuard sg(c, stream);
-    sensitivity(c->L[0].g, u, lam, dtype == TOPO_F32, rho, penal, E0, Emin, dc, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    sensitivity(c->L[0].g, u, lam, dtype == TOPO_F32, rho, penal, E0, Emin, dc, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1675,8 +1731,9 @@ int topo_dot(topo_ctx* c, int dtype, const void* a, const void* b, long long n, 
   try {
     if (!c || !a || !b || !out_host) throw std::invalid_argument("topo_dot: null pointer");
     if (dtype != TOPO_F64 && dtype != TOPO_F32) throw std::invalid_argument("topo_dot: bad dtype");
-    StreamGuard sg(c, stream);
-    *out_host = dot_host(dtype == TOPO_F64, n, a, b, c->red, c->dtmp, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    *out_host = dot_host(dtype == TOPO_F64, n, a, b, c->red, c->dtmp, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1688,8 +1745,9 @@ int topo_filter(topo_ctx* c, double rmin, const double* in, double* out, int tra
     if (!c || !in || !out) throw std::invalid_argument("topo_filter: null pointer");
     if (!(rmin > 0.0)) throw std::invalid_argument("topo_filter: rmin must be > 0");
     if (in == out) throw std::invalid_argument("topo_filter: in and out must differ");
-    StreamGuard sg(c, stream);
-    filter_apply(c->fstencil, c->L[0].g, rmin, in, out, transpose != 0, c->Hs, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    filter_apply(c->fstencil, c->L[0].g, rmin, in, out, transpose != 0, c->Hs, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1700,8 +1758,9 @@ int topo_oc(topo_ctx* c, const double* rho, const double* dc, double volfrac, do
             double* out, int* out_evals, void* stream) {
   try {
     if (!c || !rho || !dc || !out) throw std::invalid_argument("topo_oc: null pointer");
-    StreamGuard sg(c, stream);
-    const int ev = oc_update(c->L[0].g.nelem, rho, dc, volfrac, move, rho_min, out, c->red, c->oc_state, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    const int ev = oc_update(c->L[0].g.nelem, rho, dc, volfrac, move, rho_min, out, c->red, c->oc_state, us);
     if (out_evals) *out_evals = ev;
     return 0;
   } catch (const std::exception& e) {
@@ -1713,9 +1772,10 @@ int topo_oc_filtered(topo_ctx* c, const double* rho, const double* dc, const dou
                      double volfrac, double move, double rho_min, double* out, int* out_evals, void* stream) {
   try {
     if (!c || !rho || !dc || !dv || !colsum || !out) throw std::invalid_argument("topo_oc_filtered: null pointer");
-    StreamGuard sg(c, stream);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
     const int ev = oc_update_filtered(c->L[0].g.nelem, rho, dc, dv, colsum, volfrac, move, rho_min, out, c->Hs,
-                                      c->red, c->oc_state, c->cs);
+                                      c->red, c->oc_state, us);
     if (out_evals) *out_evals = ev;
     return 0;
   } catch (const std::exception& e) {
@@ -1728,8 +1788,9 @@ int topo_heaviside(topo_ctx* c, const double* rho_f, double beta, double eta, do
   try {
     if (!c || !rho_f || (!phys && !dh)) throw std::invalid_argument("topo_heaviside: null pointer");
     if (phys == rho_f || dh == rho_f) throw std::invalid_argument("topo_heaviside: outputs must not alias rho_f");
-    StreamGuard sg(c, stream);
-    heaviside_apply(c->L[0].g.nelem, rho_f, beta, eta, phys, dh, c->cs);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    heaviside_apply(c->L[0].g.nelem, rho_f, beta, eta, phys, dh, us);
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
@@ -1744,10 +1805,11 @@ int topo_oc_projected(topo_ctx* c, double rmin, const double* rho, const double*
     if (!(rmin > 0.0)) throw std::invalid_argument("topo_oc_projected: rmin must be > 0");
     if (out == rho || out == dc || out == dv)
       throw std::invalid_argument("topo_oc_projected: out must not alias rho, dc or dv");
-    StreamGuard sg(c, stream);
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
     if (!c->oc_cand) c->oc_cand = c->alloc<double>(oc_projected_candidates() * c->L[0].g.nelem);
     const int ev = oc_update_projected(c->fstencil, c->L[0].g, rmin, rho, dc, dv, beta, eta, volfrac, move, rho_min, out, c->Hs,
-                                       c->oc_cand, c->red, c->oc_state, c->cs);
+                                       c->oc_cand, c->red, c->oc_state, us);
     if (out_evals) *out_evals = ev;
     return 0;
   } catch (const std::exception& e) {
@@ -1758,10 +1820,11 @@ int topo_oc_projected(topo_ctx* c, double rmin, const double* rho, const double*
 int topo_field_stats(topo_ctx* c, const double* x, long long n, double* out_host, void* stream) {
   try {
     if (!c || !x || !out_host) throw std::invalid_argument("topo_field_stats: null pointer");
-    StreamGuard sg(c, stream);
-    field_stats(n, x, c->dtmp, c->red, c->cs);
-    TOPO_CUDA_CHECK(cudaMemcpyAsync(out_host, c->dtmp, sizeof(double) * 4, cudaMemcpyDeviceToHost, c->cs));
-    TOPO_CUDA_CHECK(cudaStreamSynchronize(c->cs));
+    DirectGuard sg(c, stream);
+    cudaStream_t us = sg.user;
+    field_stats(n, x, c->dtmp, c->red, us);
+    TOPO_CUDA_CHECK(cudaMemcpyAsync(out_host, c->dtmp, sizeof(double) * 4, cudaMemcpyDeviceToHost, us));
+    TOPO_CUDA_CHECK(cudaStreamSynchronize(us));
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
