@@ -261,9 +261,8 @@ struct CoefV<__nv_bfloat16, 2> {
 // blockIdx.y is the group of NV columns (of nv).
 template <typename TC, typename T, bool BF, Epi EPI, int NPT, int NV>
 __global__ void __launch_bounds__(96)
-k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ u, const uint8_t* __restrict__ mask,
+k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* u, const uint8_t* __restrict__ mask,
           EpiDev<T> ep, const KrylovState* st, int nv, long long vs) {
-  if (st != nullptr && st->done) return;
   using V = typename CoefV<TC, NPT>::V;
   constexpr int NN = 32 * NPT, RUN = 3 * (NN + 2);
   __shared__ T us[NV][9][RUN];
@@ -283,6 +282,9 @@ k_stencil(Grid g, long long ns, const TC* __restrict__ S, const T* __restrict__ 
       for (int d = 0; d < 3; ++d) w[3 * k + d] = live ? __ldg(Sp + (long long)((9 * dx + k) * 9 + d) * step) : (V)0;
   };
   fetch(0, cf[0]);
+  chain_wait();
+  chain_release();
+  if (st != nullptr && st->done) return;
   // nodes n0 - 1 .. n0 + NN of each run, shifted by (dx, dy)
 #pragma unroll
   for (int r = 0; r < 9; ++r) {
@@ -363,21 +365,20 @@ static void launch_stencil(const Grid& g, const void* S, const void* u, const ui
   const EpiDev<T> ep = make_epi<T>(y, ea);
   switch (epi) {
     case Epi::Store:
-      k_stencil<TC, T, BF, Epi::Store, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
+      launch_chained(k_stencil<TC, T, BF, Epi::Store, NPT, NV>, nb, 96, 0, s, g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::Residual:
-      k_stencil<TC, T, BF, Epi::Residual, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
+      launch_chained(k_stencil<TC, T, BF, Epi::Residual, NPT, NV>, nb, 96, 0, s, g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::ChebR:
-      k_stencil<TC, T, BF, Epi::ChebR, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
+      launch_chained(k_stencil<TC, T, BF, Epi::ChebR, NPT, NV>, nb, 96, 0, s, g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     case Epi::RUpd:
-      k_stencil<TC, T, BF, Epi::RUpd, NPT, NV><<<nb, 96, 0, s>>>(g, ns, SS, uu, mask, ep, ea.st, nv, vs);
+      launch_chained(k_stencil<TC, T, BF, Epi::RUpd, NPT, NV>, nb, 96, 0, s, g, ns, SS, uu, mask, ep, ea.st, nv, vs);
       break;
     default:
       throw std::runtime_error("stencil_apply: unsupported epilogue");
   }
-  TOPO_LAUNCH_CHECK();
 }
 
 // Columns that share one fetch of the coefficients (static shared memory: FP64 4 x 8.1 KB).
@@ -477,9 +478,10 @@ void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_
 // right-hand side of the coarsest solve. Latency bound on small levels: one
 // thread per node over three nested loops took 7.5 us there, this RESTRICT_US.
 template <typename T>
-__global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* __restrict__ rf, const uint8_t* __restrict__ mc,
-                                                  T* __restrict__ rc, const int* __restrict__ index, double* __restrict__ compact,
+__global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* rf, const uint8_t* __restrict__ mc,
+                                                  T* rc, const int* __restrict__ index, double* compact,
                                                   const KrylovState* st, long long vsf, long long vsc, long long vscompact) {
+  chain_enter();
   if (st != nullptr && st->done) return;
   rf += blockIdx.y * vsf;  // column
   rc += blockIdx.y * vsc;
@@ -519,19 +521,19 @@ void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* 
   const int bs = 128;
   const dim3 nb((unsigned)((coarse.ndof + bs - 1) / bs), (unsigned)nv);
   if (vec64)
-    k_restrict<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st, vsf, vsc, vscompact);
+    launch_chained(k_restrict<double>, nb, bs, 0, s, fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st, vsf, vsc, vscompact);
   else
-    k_restrict<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st, vsf, vsc, vscompact);
-  TOPO_LAUNCH_CHECK();
+    launch_chained(k_restrict<float>, nb, bs, 0, s, fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st, vsf, vsc, vscompact);
 }
 
 // x_f += mask_f * P e_c: one thread per fine node, its (at most) 24 reads issued
 // together. (One thread per DoF repeats the index arithmetic three times and is
 // bound by it: 23 us on level 0 of 160x80x80, this 9 us.)
 template <typename T>
-__global__ void __launch_bounds__(128) k_prolong_add(Grid f, Grid c, const T* __restrict__ ec, const uint8_t* __restrict__ mf,
-                                                     T* __restrict__ xf, T* __restrict__ e_out, const KrylovState* st,
+__global__ void __launch_bounds__(128) k_prolong_add(Grid f, Grid c, const T* ec, const uint8_t* __restrict__ mf,
+                                                     T* xf, T* e_out, const KrylovState* st,
                                                      long long vsf, long long vsc) {
+  chain_enter();
   if (st != nullptr && st->done) return;
   ec += blockIdx.y * vsc;  // column
   xf += blockIdx.y * vsf;
@@ -578,10 +580,9 @@ void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* e
   const int bs = 128;
   const dim3 nb((unsigned)((fine.nnodes + bs - 1) / bs), (unsigned)nv);
   if (vec64)
-    k_prolong_add<double><<<nb, bs, 0, s>>>(fine, coarse, (const double*)ec, mf, (double*)xf, (double*)e_out, st, vsf, vsc);
+    launch_chained(k_prolong_add<double>, nb, bs, 0, s, fine, coarse, (const double*)ec, mf, (double*)xf, (double*)e_out, st, vsf, vsc);
   else
-    k_prolong_add<float><<<nb, bs, 0, s>>>(fine, coarse, (const float*)ec, mf, (float*)xf, (float*)e_out, st, vsf, vsc);
-  TOPO_LAUNCH_CHECK();
+    launch_chained(k_prolong_add<float>, nb, bs, 0, s, fine, coarse, (const float*)ec, mf, (float*)xf, (float*)e_out, st, vsf, vsc);
 }
 
 TOPO_BOUNDS_READER(bounds_flag_coarse)

@@ -757,7 +757,8 @@ __global__ void __launch_bounds__(256) k_couplings(int band, long long ldb, cons
 // through shared memory. With four warps per row one block
 // (about 4 band rows) is a single short wave, so the 2P dependent launches of
 // an apply cost about 5 us each. The restriction to the coarsest level writes
-// the compact right-hand side; both passes read the compact vectors through L1.
+// the compact right-hand side; both passes read the compact vectors through L1 (plain loads: the kernels of
+// a chain overlap, so nothing that one of them writes is read with __ldg).
 constexpr int RW = 4;  // warps per row
 
 // One warp's share of sum_{j in [lo, hi)} Ci[j] v[j] over a row segment:
@@ -766,7 +767,7 @@ constexpr int RW = 4;  // warps per row
 // (W_q: m columns, G_q and H_q: band columns) is padded to a multiple of 32,
 // so none leaves its segment; entries outside [lo, hi) are not used.
 template <typename TX>
-__device__ __forceinline__ double seg_dot(const TX* __restrict__ Ci, const double* __restrict__ v, int lo, int hi,
+__device__ __forceinline__ double seg_dot(const TX* __restrict__ Ci, const double* v, int lo, int hi,
                                           int lane, int sub) {
   constexpr int V = 16 / sizeof(TX);
   constexpr int STEP = RW * 32 * V;
@@ -782,7 +783,7 @@ __device__ __forceinline__ double seg_dot(const TX* __restrict__ Ci, const doubl
 #pragma unroll
       for (int q = 0; q < V; ++q) {
         const int jj = j + u * STEP + q;
-        if (jj >= lo && jj < hi) acc += (double)w[u][q] * __ldg(v + jj);
+        if (jj >= lo && jj < hi) acc += (double)w[u][q] * v[jj];
       }
   }
   for (; j < hi; j += STEP) {
@@ -791,7 +792,7 @@ __device__ __forceinline__ double seg_dot(const TX* __restrict__ Ci, const doubl
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       const int jj = j + q;
-      if (jj >= lo && jj < hi) acc += (double)w[q] * __ldg(v + jj);
+      if (jj >= lo && jj < hi) acc += (double)w[q] * v[jj];
     }
   }
   return acc;
@@ -813,8 +814,9 @@ __device__ __forceinline__ double row_sum(double acc, int warp, int lane) {
 // pass one, block q (rows b0 .. b0+m-1): y_q = W_q r_q - G_q y_{q-1}[m_{q-1}-band ..]
 template <typename TX>
 __global__ void __launch_bounds__(256) k_coarse_lower(int m, int b0, long long ld, int gofs, int band, int prev,
-                                                      const TX* __restrict__ Cq, const double* __restrict__ rc,
+                                                      const TX* __restrict__ Cq, const double* rc,
                                                       double* y, const KrylovState* st, long long vswork) {
+  chain_enter();
   if (st != nullptr && st->done) return;  // uniform over the grid
   rc += blockIdx.y * vswork;              // column
   y += blockIdx.y * vswork;
@@ -837,8 +839,9 @@ template <typename T, typename TX>
 __global__ void __launch_bounds__(256) k_coarse_upper(int m, int b0, long long ld, int hofs, int band, int next,
                                                       long long nfull, const TX* __restrict__ Cq,
                                                       const int* __restrict__ free_list, const double* y, double* z,
-                                                      T* __restrict__ x, const KrylovState* st, long long vswork,
+                                                      T* x, const KrylovState* st, long long vswork,
                                                       long long vsx) {
+  chain_enter();
   if (st != nullptr && st->done) return;  // uniform over the grid
   y += blockIdx.y * vswork;               // column
   z += blockIdx.y * vswork;
@@ -1011,16 +1014,11 @@ static void apply_blocks(const CoarsestFactor& f, double* work, T* x, const Kryl
   const TX* C = (const TX*)f.C;
   for (int q = 0; q < bk.P; ++q) {
     const int m = bk.b[q + 1] - bk.b[q];
-    cst::k_coarse_lower<TX><<<dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s>>>(
-        m, bk.b[q], bk.ld[q], bk.gofs[q], f.band, (int)(q > 0), C + bk.off[q], rc, y, st, vswork);
-    TOPO_LAUNCH_CHECK();
+    launch_chained(cst::k_coarse_lower<TX>, dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s, m, bk.b[q], bk.ld[q], bk.gofs[q], f.band, (int)(q > 0), C + bk.off[q], rc, y, st, vswork);
   }
   for (int q = bk.P - 1; q >= 0; --q) {
     const int m = bk.b[q + 1] - bk.b[q];
-    cst::k_coarse_upper<T, TX><<<dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s>>>(
-        m, bk.b[q], bk.ld[q], bk.hofs[q], f.band, (int)(q < bk.P - 1), p.nfull, C + bk.off[q], f.d_free, y, rc, x,
-        st, vswork, vsx);
-    TOPO_LAUNCH_CHECK();
+    launch_chained(cst::k_coarse_upper<T, TX>, dim3((unsigned)((m + rpb - 1) / rpb), (unsigned)nv), 256, 0, s, m, bk.b[q], bk.ld[q], bk.hofs[q], f.band, (int)(q < bk.P - 1), p.nfull, C + bk.off[q], f.d_free, y, rc, x, st, vswork, vsx);
   }
 }
 

@@ -432,6 +432,7 @@ void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cu
   Level& L0 = c->L[0];
   void* saved_b = L0.b;
   void* saved_x = L0.x;
+  LaunchChain chain;
   L0.b = const_cast<void*>(r);
   L0.x = z;
   vcycle(c, 0, st, same_bits, s);
@@ -465,6 +466,7 @@ void vcycle_columns(topo_ctx* c, int nv, cudaStream_t s) {
     Lv.b = Lv.cols[5];
   }
   c->bw = nv;
+  LaunchChain chain;
   try {
     vcycle(c, 0, nullptr, false, s);
   } catch (...) {
@@ -771,6 +773,7 @@ void do_setup(topo_ctx* c, const double* E, cudaStream_t s) {
 void pcg_iteration(topo_ctx* c, cudaStream_t s) {
   Level& L0 = c->L[0];
   const long long n = L0.g.ndof;
+  LaunchChain chain;
   EpiArgs ea{};
   ea.st = c->st;
   ea.red = c->red;
@@ -849,9 +852,12 @@ int do_pcg(topo_ctx* c, const double* b, double* x, double tol, int maxiter, int
   while (!converged && iters < maxiter && refreshes < 8) {
     k_set_state<<<1, 1, 0, s>>>(c->st, bb, tol2);
     TOPO_LAUNCH_CHECK();
-    vcycle_apply(c, c->kr, c->kz, nullptr, s);
-    pcg_rz(c->vec64, n, c->kr, c->kz, c->st, c->red, true, s);
-    pcg_p_update(c->vec64, n, c->kz, c->kp, c->st, true, s);
+    {
+      LaunchChain chain;
+      vcycle_apply(c, c->kr, c->kz, nullptr, s);
+      pcg_rz(c->vec64, n, c->kr, c->kz, c->st, c->red, true, s);
+      pcg_p_update(c->vec64, n, c->kz, c->kp, c->st, true, s);
+    }
     iters += 1;
     if (exec == nullptr) {
       cudaGraph_t graph;

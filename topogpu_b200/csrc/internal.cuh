@@ -418,6 +418,79 @@ long long launch_count();
     TOPO_CUDA_CHECK(cudaGetLastError()); \
   } while (0)
 
+// --------------------------------------------------------- launch chains
+// Inside a LaunchChain (a V-cycle, a PCG iteration) the kernels launched with
+// launch_chained start while the one before still runs: chain_wait holds a
+// kernel until every kernel before it has ended and its writes can be seen,
+// chain_release lets its successor's CTAs in. The first launch of a chain is
+// an ordinary one, so that everything enqueued before the chain has ended when
+// any of its kernels starts: ahead of chain_wait a kernel may read what no
+// kernel of the chain writes (coefficients, masks), and nothing else. Its
+// other operands change during its lifetime, so they are not read through the
+// non-coherent path either (no __ldg, no const __restrict__ pointer to them).
+//
+// The levels of a V-cycle below the finest are 2 to 6 us kernels whose launch,
+// ramp and drain this overlaps. B200, ordinary launches -> chains: FP32 V-cycle
+// of 61x30x23 (31 kernels, direct) 167 -> 119 us; state solve of 24x12x6 2091
+// -> 1900 us and of 48x24x24 5030 -> 4640 us, mixed gradient of 43x21x17 8.02
+// -> 7.22 ms (graph replays); the largest gain nothing but a percent or two.
+// Releasing ahead of the wait stacks several waiting kernels on the SMs
+// (48x24x24: 4860 us, 43x21x17: 8.2 ms); releasing at the end of the stencil
+// and K.u kernels measured the same but for block solves (96x48x48: 20.9 ms
+// after the wait, 21.5 at the end).
+class LaunchChain {
+ public:
+  LaunchChain() { ++depth(); }
+  ~LaunchChain() {
+    if (--depth() == 0) primed() = false;
+  }
+  LaunchChain(const LaunchChain&) = delete;
+  LaunchChain& operator=(const LaunchChain&) = delete;
+  // whether the next launch may overlap the one before
+  static bool next() {
+    const bool p = primed();
+    if (depth() > 0) primed() = true;
+    return p;
+  }
+  static void cut() { primed() = false; }  // after a copy or a memset
+
+ private:
+  static int& depth() {
+    static thread_local int d = 0;
+    return d;
+  }
+  static bool& primed() {
+    static thread_local bool p = false;
+    return p;
+  }
+};
+
+template <typename... P, typename... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = LaunchChain::next() ? 1 : 0;
+  TOPO_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(a)...));
+  TOPO_LAUNCH_CHECK();
+}
+
+// Without effect in a kernel that was launched in the ordinary way. Every
+// thread of a chained kernel waits before it returns, also where there is
+// nothing to do: the end of a kernel stands for the end of those before it.
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_enter() {
+  chain_wait();
+  chain_release();
+}
+
 // ------------------------------------------------ index range-check build
 // Built with -DTOPO_DEBUG_BOUNDS (python -m topogpu_b200.build
 // --debug-bounds -> libtopo_b200_dbg.so), every checked gather/scatter index

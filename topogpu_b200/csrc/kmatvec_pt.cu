@@ -149,7 +149,6 @@ __device__ __forceinline__ void prefetch_l2(const void* b, const void* e) {
 // the one-column form has no room for).
 template <typename T, typename TU, bool BF, Epi EPI, bool COLS, int NW, int MINB>
 __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_constant__ Params<T> P) {
-  if (P.st != nullptr && P.st->done) return;
   extern __shared__ __align__(128) unsigned char sm[];
   using V = typename Pair<T>::V;
   constexpr int NT = 32 * NW, SU = (int)sizeof(TU), ST = (int)sizeof(T);
@@ -174,6 +173,9 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
+  chain_wait();
+  chain_release();
+  if (P.st != nullptr && P.st->done) return;
 
   // plane p -> slot (p - pf) % RING; node n of it at byte 16 + shift + 3 SU (n - mlo),
   // where shift makes the copy's source and destination agree modulo 16
@@ -578,8 +580,7 @@ void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t
     TOPO_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
     if (dev <= 63) raised |= 1ull << dev;
   }
-  k<<<dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T, EPI>::NW[W], L.total, s>>>(P);
-  TOPO_LAUNCH_CHECK();
+  launch_chained(k, dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T, EPI>::NW[W], L.total, s, P);
 }
 
 template <typename T, typename TU, bool BF, Epi EPI>

@@ -28,6 +28,7 @@ void vfill(bool f64, long long n, void* x, double v, cudaStream_t s) {
 
 void vcopy(bool f64, long long n, const void* a, void* b, cudaStream_t s) {
   TOPO_CUDA_CHECK(cudaMemcpyAsync(b, a, (size_t)n * (f64 ? 8 : 4), cudaMemcpyDeviceToDevice, s));
+  LaunchChain::cut();
 }
 
 template <typename A, typename B>
@@ -62,9 +63,9 @@ void vmask(bool f64, long long n, void* x, const uint8_t* mask, cudaStream_t s) 
 // First Chebyshev step on the current residual (from x0 = 0 the residual is
 // b itself: K 0 = 0, no operator application): d = c2 D^-1 r, x += ax d.
 template <typename T>
-__global__ void k_cheb_start(long long n, const T* __restrict__ b, T* __restrict__ r, const T* __restrict__ dinv,
-                             T c2, T ax, T* __restrict__ x, T* __restrict__ d, int x_is_zero, const KrylovState* st,
+__global__ void k_cheb_start(long long n, const T* b, T* r, const T* __restrict__ dinv, T c2, T ax, T* x, T* d, int x_is_zero, const KrylovState* st,
                              long long vs) {
+  chain_enter();
   if (st != nullptr && st->done) return;
   const long long co = blockIdx.y * vs;  // column
   if (b != nullptr) b += co;
@@ -90,12 +91,9 @@ void cheb_start(bool f64, long long n, const void* b, void* r, const void* dinv,
                 void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s, int nv, long long vs) {
   const dim3 nb(grid_for(n, 256), (unsigned)nv);
   if (f64)
-    k_cheb_start<double><<<nb, 256, 0, s>>>(n, (const double*)b, (double*)r, (const double*)dinv, c2, ax, (double*)x,
-                                            (double*)d, x_is_zero, st, vs);
+    launch_chained(k_cheb_start<double>, nb, 256, 0, s, n, (const double*)b, (double*)r, (const double*)dinv, c2, ax, (double*)x, (double*)d, x_is_zero, st, vs);
   else
-    k_cheb_start<float><<<nb, 256, 0, s>>>(n, (const float*)b, (float*)r, (const float*)dinv, (float)c2, (float)ax,
-                                           (float*)x, (float*)d, x_is_zero, st, vs);
-  TOPO_LAUNCH_CHECK();
+    launch_chained(k_cheb_start<float>, nb, 256, 0, s, n, (const float*)b, (float*)r, (const float*)dinv, (float)c2, (float)ax, (float*)x, (float*)d, x_is_zero, st, vs);
 }
 
 // ------------------------------------------------------------------- dots
@@ -140,8 +138,8 @@ void pcg_init(KrylovState* st, double tol, cudaStream_t s) {
 // The iterate x is FP64 whatever the working precision T of r, p, Ap, so an
 // FP32 solve is not capped by the FP32 representation of x (reliable update).
 template <typename T>
-__global__ void k_pcg_xr(long long n, double* __restrict__ x, T* __restrict__ r, const T* __restrict__ p,
-                         const T* __restrict__ Ap, KrylovState* st, RedWork red) {
+__global__ void k_pcg_xr(long long n, double* x, T* r, const T* p, const T* Ap, KrylovState* st, RedWork red) {
+  chain_enter();
   if (st->done) return;
   const double alpha64 = st->alpha;
   const T alpha = (T)alpha64;
@@ -167,16 +165,16 @@ void pcg_xr_update(bool f64, long long n, void* x, void* r, const void* p, const
                    RedWork red, cudaStream_t s) {
   const unsigned nb = grid_for(n, kRedThreads, kRedBlocks);
   if (f64)
-    k_pcg_xr<double><<<nb, kRedThreads, 0, s>>>(n, (double*)x, (double*)r, (const double*)p, (const double*)Ap, st, red);
+    launch_chained(k_pcg_xr<double>, nb, kRedThreads, 0, s, n, (double*)x, (double*)r, (const double*)p, (const double*)Ap, st, red);
   else
-    k_pcg_xr<float><<<nb, kRedThreads, 0, s>>>(n, (double*)x, (float*)r, (const float*)p, (const float*)Ap, st, red);
-  TOPO_LAUNCH_CHECK();
+    launch_chained(k_pcg_xr<float>, nb, kRedThreads, 0, s, n, (double*)x, (float*)r, (const float*)p, (const float*)Ap, st, red);
 }
 
 // rz_new = r.z ; beta = rz_new / rz ; one more preconditioner application
 template <typename T>
-__global__ void k_pcg_rz(long long n, const T* __restrict__ r, const T* __restrict__ z, KrylovState* st,
+__global__ void k_pcg_rz(long long n, const T* r, const T* z, KrylovState* st,
                          RedWork red, int first) {
+  chain_enter();
   if (st->done) return;
   double v[1] = {0.0};
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -196,13 +194,13 @@ __global__ void k_pcg_rz(long long n, const T* __restrict__ r, const T* __restri
 void pcg_rz(bool f64, long long n, const void* r, const void* z, KrylovState* st, RedWork red, bool first,
             cudaStream_t s) {
   const unsigned nb = grid_for(n, kRedThreads, kRedBlocks);
-  if (f64) k_pcg_rz<double><<<nb, kRedThreads, 0, s>>>(n, (const double*)r, (const double*)z, st, red, first);
-  else k_pcg_rz<float><<<nb, kRedThreads, 0, s>>>(n, (const float*)r, (const float*)z, st, red, first);
-  TOPO_LAUNCH_CHECK();
+  if (f64) launch_chained(k_pcg_rz<double>, nb, kRedThreads, 0, s, n, (const double*)r, (const double*)z, st, red, first);
+  else launch_chained(k_pcg_rz<float>, nb, kRedThreads, 0, s, n, (const float*)r, (const float*)z, st, red, first);
 }
 
 template <typename T>
-__global__ void k_pcg_p(long long n, const T* __restrict__ z, T* __restrict__ p, const KrylovState* st, int first) {
+__global__ void k_pcg_p(long long n, const T* z, T* p, const KrylovState* st, int first) {
+  chain_enter();
   if (st->done) return;
   const T beta = first ? (T)0 : (T)st->beta;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
@@ -210,9 +208,8 @@ __global__ void k_pcg_p(long long n, const T* __restrict__ z, T* __restrict__ p,
 }
 
 void pcg_p_update(bool f64, long long n, const void* z, void* p, KrylovState* st, bool first, cudaStream_t s) {
-  if (f64) k_pcg_p<double><<<grid_for(n, 256), 256, 0, s>>>(n, (const double*)z, (double*)p, st, first);
-  else k_pcg_p<float><<<grid_for(n, 256), 256, 0, s>>>(n, (const float*)z, (float*)p, st, first);
-  TOPO_LAUNCH_CHECK();
+  if (f64) launch_chained(k_pcg_p<double>, grid_for(n, 256), 256, 0, s, n, (const double*)z, (double*)p, st, first);
+  else launch_chained(k_pcg_p<float>, grid_for(n, 256), 256, 0, s, n, (const float*)z, (float*)p, st, first);
 }
 
 // x64 += a * z (z in the working precision)
