@@ -473,18 +473,19 @@ void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_
 }
 
 // r_c = mask_c * P^T r_f: one thread per coarse DoF, its 27 reads issued
-// together (missing ones have weight zero). With `compact` (the coarsest
-// level) the value of free DoF i also goes to compact[index[i]] in FP64, the
-// right-hand side of the coarsest solve. Latency bound on small levels: one
-// thread per node over three nested loops took 7.5 us there, this RESTRICT_US.
+// together (missing ones have weight zero). On the coarsest level free DoF i
+// goes to compact[index[i]] in FP64, the right-hand side of the coarsest
+// solve; on the others r_c starts the level's smoother right here, d = c2 D^-1
+// r_c, x = ax d (x = 0 before), which saves a launch per level. Latency bound
+// on small levels: one thread per node over three nested loops took 7.5 us
+// there, this 2.4 us (and the start 1.9 us as a kernel of its own).
 template <typename T>
 __global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* rf, const uint8_t* __restrict__ mc,
-                                                  T* rc, const int* __restrict__ index, double* compact,
+                                                  SmoothStart<T> ss, const int* __restrict__ index, double* compact,
                                                   const KrylovState* st, long long vsf, long long vsc, long long vscompact) {
   chain_enter();
   if (st != nullptr && st->done) return;
   rf += blockIdx.y * vsf;  // column
-  rc += blockIdx.y * vsc;
   if (compact != nullptr) compact += blockIdx.y * vscompact;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= c.ndof) return;
@@ -511,19 +512,26 @@ __global__ void __launch_bounds__(128) k_restrict(Grid f, Grid c, const T* rf, c
 #pragma unroll
   for (int k = 0; k < 27; ++k) a += (wx[k / 9] * wy[(k / 3) % 3] * wz[k % 3]) * v[k];
   const T r = mc[i] ? a : (T)0;
-  rc[i] = r;
-  if (compact != nullptr && index[i] >= 0) compact[index[i]] = (double)r;
+  if (compact != nullptr) {
+    if (index[i] >= 0) compact[index[i]] = (double)r;
+    return;
+  }
+  const long long o = blockIdx.y * vsc + i;
+  const T d0 = ss.c2 * (ss.dinv[i] * r);
+  ss.r[o] = r;
+  ss.d[o] = d0;
+  ss.x[o] = (T)0 + ss.ax * d0;
 }
 
-void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc, void* rc,
-                  const int* index, double* compact, const KrylovState* st, cudaStream_t s, int nv, long long vsf,
-                  long long vsc, long long vscompact) {
+void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc,
+                  const SmoothStart<void>& to, const int* index, double* compact, const KrylovState* st, cudaStream_t s,
+                  int nv, long long vsf, long long vsc, long long vscompact) {
   const int bs = 128;
   const dim3 nb((unsigned)((coarse.ndof + bs - 1) / bs), (unsigned)nv);
   if (vec64)
-    launch_chained(k_restrict<double>, nb, bs, 0, s, fine, coarse, (const double*)rf, mc, (double*)rc, index, compact, st, vsf, vsc, vscompact);
+    launch_chained(k_restrict<double>, nb, bs, 0, s, fine, coarse, (const double*)rf, mc, smooth_start<double>(to), index, compact, st, vsf, vsc, vscompact);
   else
-    launch_chained(k_restrict<float>, nb, bs, 0, s, fine, coarse, (const float*)rf, mc, (float*)rc, index, compact, st, vsf, vsc, vscompact);
+    launch_chained(k_restrict<float>, nb, bs, 0, s, fine, coarse, (const float*)rf, mc, smooth_start<float>(to), index, compact, st, vsf, vsc, vscompact);
 }
 
 // x_f += mask_f * P e_c: one thread per fine node, its (at most) 24 reads issued

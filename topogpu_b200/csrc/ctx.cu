@@ -126,7 +126,7 @@ struct Level {
   int degree = 2;
   // the V-cycle's vectors for several columns (x, r, d, d2, e, b; allocated by
   // the first block solve), vs entries from column to column
-  void* cols[6] = {};
+  void* cols[6] = {};  // (the last one on level 0 only)
   long long vs = 0;
 };
 
@@ -333,22 +333,25 @@ Prec hi_prec(const Level& Lv) { return Lv.prec == Prec::BF16 ? Prec::F32 : Lv.pr
 
 // Chebyshev-Jacobi smoothing on level l (reference: multigrid_v4.py:861-889)
 // with a recursive residual: Lv.x and Lv.r are updated in place and the
-// operator only ever multiplies a direction. from_zero: x = 0 and r = b.
-// want_residual: also form the final residual r = b - K x (one more
-// application, which replaces the reference's separate residual matvec).
-// started: the first step (direction Lv.d) has been taken by the kernel before.
+// operator only ever multiplies a direction. want_residual: also form the
+// final residual r = b - K x (one more application, which replaces the
+// reference's separate residual matvec). started: the first step (direction
+// Lv.d) has been taken by the kernel before; otherwise x = 0 and r = Lv.b.
 Cheb level_cheb(const topo_ctx* c, const Level& Lv) {
   const double lam = (std::isfinite(Lv.lam) ? Lv.lam : 1.0) * c->lam_safety;
   return make_cheb(lam, c->cheb_lower, Lv.degree, c->cheb_form);
 }
 
-void smooth(topo_ctx* c, int l, bool from_zero, bool started, bool want_residual, const KrylovState* st, bool same_bits,
+SmoothStart<void> level_start(const topo_ctx* c, const Level& Lv) {
+  const Cheb ch = level_cheb(c, Lv);
+  return {Lv.r, Lv.x, Lv.d, Lv.dinv, ch.c2[0], ch.ax[0]};
+}
+
+void smooth(topo_ctx* c, int l, bool started, bool want_residual, const KrylovState* st, bool same_bits,
             cudaStream_t s) {
   Level& Lv = c->L[l];
   const Cheb ch = level_cheb(c, Lv);
-  const long long n = Lv.g.ndof;
-  if (!started) cheb_start(c->vec64, n, from_zero ? Lv.b : nullptr, Lv.r, Lv.dinv, ch.c2[0], ch.ax[0], Lv.x, Lv.d, from_zero, st,
-             s, c->bw, Lv.vs);
+  if (!started) cheb_start(c->vec64, Lv.g.ndof, Lv.b, level_start(c, Lv), st, s, c->bw, Lv.vs);
   void* dcur = Lv.d;
   void* dnext = Lv.d2;
   for (int j = 1; j < Lv.degree; ++j) {
@@ -383,22 +386,23 @@ void coarsest_solve(topo_ctx* c, const KrylovState* st, cudaStream_t s) {
 }
 
 // One V-cycle (cycle_gamma 1, multigrid_v4.py:986-1008) or W-cycle
-// (cycle_gamma 2, multigrid_v4.py:1010-1042) on level l: input Lv.b, output
+// (cycle_gamma 2, multigrid_v4.py:1010-1042) on level l: input Lv.b (level 0; on
+// the others the restriction has put it into Lv.r and started the smoother), output
 // Lv.x. Each coarse correction restricts the recursive residual, recurses,
 // adds e = P x_c and updates r -= K e, so the second correction of a W-cycle
 // restricts b - K x without a separate residual product.
 void vcycle(topo_ctx* c, int l, const KrylovState* st, bool same_bits, cudaStream_t s) {
   Level& Lv = c->L[l];
   if (l == c->n_levels - 1) {
-    if (c->n_levels == 1) smooth(c, 0, true, false, false, st, same_bits, s);
+    if (c->n_levels == 1) smooth(c, 0, false, false, st, same_bits, s);
     else coarsest_solve(c, st, s);
     return;
   }
-  smooth(c, l, true, false, true, st, same_bits, s);  // x = S b, r = b - K x
+  smooth(c, l, l > 0, true, st, same_bits, s);  // x = S b, r = b - K x
   Level& Lc = c->L[l + 1];
   for (int k = 0; k < c->cycle_gamma; ++k) {
     const bool bottom = l + 1 == c->n_levels - 1;
-    restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, Lc.b, bottom ? c->C.dof_index : nullptr,
+    restrict_vec(c->vec64, Lv.g, Lc.g, Lv.r, Lc.mask, bottom ? SmoothStart<void>{} : level_start(c, Lc), bottom ? c->C.dof_index : nullptr,
                  bottom ? (c->bw > 1 ? c->blk_y : c->C.y) + std::max(c->C.n, 1) : nullptr, st, s, c->bw, Lv.vs, Lc.vs,
                  2LL * c->C.n);
     vcycle(c, l + 1, st, same_bits, s);
@@ -425,7 +429,7 @@ void vcycle(topo_ctx* c, int l, const KrylovState* st, bool same_bits, cudaStrea
     // raised the PCG iterations of the 1M-element cantilever from ~18 to ~95
     op_apply(c, l, hi_prec(Lv), Lv.e, nullptr, epi, ea, same_bits, s);  // r -= K e
   }
-  smooth(c, l, false, true, false, st, same_bits, s);
+  smooth(c, l, true, false, st, same_bits, s);
 }
 
 void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cudaStream_t s, bool same_bits = false) {
@@ -448,7 +452,7 @@ void block_reserve(topo_ctx* c, int nv) {
   if (c->blk_cols >= nv && c->blk_n == c->C.n) return;
   for (Level& Lv : c->L) {
     Lv.vs = (Lv.g.ndof + 3) & ~3LL;  // columns 16-byte aligned in FP32 and FP64
-    for (void*& p : Lv.cols) p = c->valloc(nv * Lv.vs);
+    for (int i = 0; i < (&Lv == &c->L[0] ? 6 : 5); ++i) Lv.cols[i] = c->valloc(nv * Lv.vs);
   }
   c->blk_y = c->alloc<double>(2LL * std::max(c->C.n, 1) * nv);
   c->blk_n = c->C.n;
@@ -1316,7 +1320,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
       Lv.d = c->valloc(nd);
       Lv.d2 = c->valloc(nd);
       Lv.e = c->valloc(nd);
-      Lv.b = c->valloc(nd);
+      if (l == 0) Lv.b = c->valloc(nd);  // (the restriction writes the other levels' right-hand side to r)
       Lv.dinv = c->valloc(nd);
       if (l >= 1) {
         Lv.S64 = c->alloc<double>(243LL * Lv.g.nnodes);

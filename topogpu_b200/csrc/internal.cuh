@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 namespace topo {
@@ -262,9 +263,22 @@ void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* d
 long long stencil16_stride(long long nnodes);
 void stencil_convert(long long nnodes, const double* S, float* S32, __nv_bfloat16* S16, cudaStream_t s);
 void inject_mask(const Grid& fine, const Grid& coarse, const uint8_t* mf, uint8_t* mc, cudaStream_t s);
+// First Chebyshev step of a level from x = 0: d = c2 D^-1 r, x = ax d.
+template <typename T>
+struct SmoothStart {
+  T *r, *x, *d;
+  const T* dinv;
+  std::conditional_t<std::is_void_v<T>, double, T> c2, ax;
+};
+template <typename T>
+SmoothStart<T> smooth_start(const SmoothStart<void>& s) {
+  return {(T*)s.r, (T*)s.x, (T*)s.d, (const T*)s.dinv, (T)s.c2, (T)s.ax};
+}
+// The restriction of rf: with index and compact (coarsest level) to compact,
+// otherwise to `to`, whose x and d it starts.
 void restrict_vec(bool vec64, const Grid& fine, const Grid& coarse, const void* rf, const uint8_t* mc,
-                  void* rc, const int* index, double* compact, const KrylovState* st, cudaStream_t s, int nv = 1,
-                  long long vsf = 0, long long vsc = 0, long long vscompact = 0);
+                  const SmoothStart<void>& to, const int* index, double* compact, const KrylovState* st, cudaStream_t s,
+                  int nv = 1, long long vsf = 0, long long vsc = 0, long long vscompact = 0);
 // x_f += e = mask_f * P e_c ; e is also written to e_out when not null
 void prolong_add(bool vec64, const Grid& fine, const Grid& coarse, const void* ec, const uint8_t* mf,
                  void* xf, void* e_out, const KrylovState* st, cudaStream_t s, int nv = 1, long long vsf = 0,
@@ -341,8 +355,7 @@ void vcast(long long n, const void* src, bool src64, void* dst, bool dst64, cuda
 void vmask(bool f64, long long n, void* x, const uint8_t* mask, cudaStream_t s);
 // First Chebyshev step on residual r (copied from b first when b is not
 // null): d = c2 D^-1 r ; x = (x_is_zero ? 0 : x) + ax d
-void cheb_start(bool f64, long long n, const void* b, void* r, const void* dinv, double c2, double ax, void* x,
-                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s, int nv = 1, long long vs = 0);
+void cheb_start(bool f64, long long n, const void* b, const SmoothStart<void>& to, const KrylovState* st, cudaStream_t s, int nv = 1, long long vs = 0);
 // out = sum a_i b_i (fp64 accumulate) to a device double
 void dot_to(bool f64, long long n, const void* a, const void* b, double* out, RedWork red,
             cudaStream_t s);

@@ -60,40 +60,29 @@ void vmask(bool f64, long long n, void* x, const uint8_t* mask, cudaStream_t s) 
   TOPO_LAUNCH_CHECK();
 }
 
-// First Chebyshev step on the current residual (from x0 = 0 the residual is
-// b itself: K 0 = 0, no operator application): d = c2 D^-1 r, x += ax d.
+// r = b and the first Chebyshev step on it (from x = 0 the residual is b
+// itself: K 0 = 0, no operator application): d = c2 D^-1 r, x = ax d. Level 0
+// only; the levels below start in the restriction to them.
 template <typename T>
-__global__ void k_cheb_start(long long n, const T* b, T* r, const T* __restrict__ dinv, T c2, T ax, T* x, T* d, int x_is_zero, const KrylovState* st,
-                             long long vs) {
+__global__ void k_cheb_start(long long n, const T* b, SmoothStart<T> ss, const KrylovState* st, long long vs) {
   chain_enter();
   if (st != nullptr && st->done) return;
   const long long co = blockIdx.y * vs;  // column
-  if (b != nullptr) b += co;
-  r += co;
-  x += co;
-  d += co;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    T ri;
-    if (b != nullptr) {
-      ri = b[i];
-      r[i] = ri;
-    } else {
-      ri = r[i];
-    }
-    const T v = c2 * (dinv[i] * ri);
-    d[i] = v;
-    x[i] = (x_is_zero ? (T)0 : x[i]) + ax * v;
+    const T ri = b[co + i];
+    const T v = ss.c2 * (ss.dinv[i] * ri);
+    ss.r[co + i] = ri;
+    ss.d[co + i] = v;
+    ss.x[co + i] = (T)0 + ss.ax * v;
   }
 }
 
-void cheb_start(bool f64, long long n, const void* b, void* r, const void* dinv, double c2, double ax, void* x,
-                void* d, bool x_is_zero, const KrylovState* st, cudaStream_t s, int nv, long long vs) {
+void cheb_start(bool f64, long long n, const void* b, const SmoothStart<void>& to, const KrylovState* st,
+                cudaStream_t s, int nv, long long vs) {
   const dim3 nb(grid_for(n, 256), (unsigned)nv);
-  if (f64)
-    launch_chained(k_cheb_start<double>, nb, 256, 0, s, n, (const double*)b, (double*)r, (const double*)dinv, c2, ax, (double*)x, (double*)d, x_is_zero, st, vs);
-  else
-    launch_chained(k_cheb_start<float>, nb, 256, 0, s, n, (const float*)b, (float*)r, (const float*)dinv, (float)c2, (float)ax, (float*)x, (float*)d, x_is_zero, st, vs);
+  if (f64) launch_chained(k_cheb_start<double>, nb, 256, 0, s, n, (const double*)b, smooth_start<double>(to), st, vs);
+  else launch_chained(k_cheb_start<float>, nb, 256, 0, s, n, (const float*)b, smooth_start<float>(to), st, vs);
 }
 
 // ------------------------------------------------------------------- dots
