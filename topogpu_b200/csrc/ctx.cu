@@ -218,9 +218,10 @@ struct topo_ctx {
   bool ke_registered = false;  // holds a reference on its device's KE
   cudaStream_t cs = nullptr;
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
-  // the last call's stream and the event behind its work: a call on another
-  // stream waits for it (has_last: there is such a call)
-  cudaStream_t last = nullptr;
+  // the id of the last call's stream (a destroyed stream's handle may come back
+  // for a new one, its id does not) and the event behind that call's work: a
+  // call on another stream waits for it (has_last: there is such a call)
+  unsigned long long last = 0;
   cudaEvent_t ev_last = nullptr, ev_dir = nullptr;
   bool has_last = false;
   cudaEvent_t ev_ph[6] = {};     // setup phase marks (timed)
@@ -260,18 +261,20 @@ bool capturing(cudaStream_t s) {
 struct StreamGuard {
   topo_ctx* c;
   cudaStream_t user;
+  unsigned long long id = 0;
   bool cap;
   StreamGuard(topo_ctx* ctx, void* stream) : c(ctx), user((cudaStream_t)stream) {
     TOPO_CUDA_CHECK(cudaSetDevice(c->device));
     cap = capturing(user);
-    if (!cap && c->has_last && c->last != user) TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_last, 0));
+    if (!cap) TOPO_CUDA_CHECK(cudaStreamGetId(user, &id));
+    if (!cap && c->has_last && c->last != id) TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_last, 0));
     TOPO_CUDA_CHECK(cudaEventRecord(c->ev_in, user));
     TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_in, 0));
   }
   ~StreamGuard() {
     if (cudaEventRecord(c->ev_out, c->cs) == cudaSuccess) cudaStreamWaitEvent(user, c->ev_out, 0);
     if (!cap) {
-      c->last = user;
+      c->last = id;
       c->ev_last = c->ev_out;
       c->has_last = true;
     }
@@ -285,15 +288,17 @@ struct StreamGuard {
 struct DirectGuard {
   topo_ctx* c;
   cudaStream_t user;
+  unsigned long long id = 0;
   bool cap;
   DirectGuard(topo_ctx* ctx, void* stream) : c(ctx), user((cudaStream_t)stream) {
     TOPO_CUDA_CHECK(cudaSetDevice(c->device));
     cap = capturing(user);
-    if (!cap && c->has_last && c->last != user) TOPO_CUDA_CHECK(cudaStreamWaitEvent(user, c->ev_last, 0));
+    if (!cap) TOPO_CUDA_CHECK(cudaStreamGetId(user, &id));
+    if (!cap && c->has_last && c->last != id) TOPO_CUDA_CHECK(cudaStreamWaitEvent(user, c->ev_last, 0));
   }
   ~DirectGuard() {
     if (cap || cudaEventRecord(c->ev_dir, user) != cudaSuccess) return;
-    c->last = user;
+    c->last = id;
     c->ev_last = c->ev_dir;
     c->has_last = true;
   }

@@ -40,9 +40,9 @@
 // element and step; 20% of the elements are halo), not HBM: FP32 Store moves
 // 26 MB at 160x80x80 (4 us at the copy rate), ChebR 93 MB (14 us). Measured on
 // a B200, rotating buffers, against the kernels it replaced there (kernel
-// times): 160x80x80 FP32 Store 24.6 us (64), FP64 Store 42.7 us (130), ChebR
-// with BF16 rounding 36.0 us (67, tensor cores), FP32 RUpd 26.5 us (64);
-// 24x12x6 FP64 4.4 us (9.6). The tensor-core form of the same operator does
+// times): 160x80x80 FP32 Store 24.5 us (64), FP64 Store 37.9 us (130), ChebR
+// with BF16 rounding 35.3 us (67, tensor cores), FP32 ChebR 35.0 us, FP32 RUpd
+// 27.7 us (64); 24x12x6 FP64 4.4 us (9.6). The tensor-core form of the same operator does
 // 1152 flop per element in 39 us of MMA issue; the parity form needs 312.
 //
 // Reference semantics: MatrixFreeKff.matvec (src/gpu_fem/solver_v2.py:1183-1223)
@@ -71,6 +71,14 @@ __constant__ float2 cKbf[36];  // of KE rounded to BF16
 
 constexpr int RING = 3;
 
+// Columns share one line of planes (see the kernel): only the FP64 Chebyshev
+// step, whose 255 registers have room for the loop (the others spill with it).
+// 8 columns of 96x48x48: one segment per window and column keeps 264 CTAs of
+// 75-node windows (of 296) or 104 of 199 (of 148) busy; equal parts fill all
+// 148 with the wide ones (block solve 18.2 -> 17.0 ms).
+template <typename T, Epi EPI>
+constexpr bool line_split = sizeof(T) == 8 && EPI == Epi::ChebR;
+
 template <typename T>
 struct Params {
   Grid g;
@@ -79,7 +87,8 @@ struct Params {
   const T* E;
   const uint8_t* mask;
   EpiDev<T> ep;
-  long long vs;             // column v = blockIdx.y of every vector starts v * vs entries on (u 16-byte aligned)
+  int nv;                   // columns
+  long long vs;             // column v of every vector starts v * vs entries on (u 16-byte aligned)
   int list;                 // != 0: u and y of column v are ucol[v], ycol[v]
   const void* ucol[8];
   T* ycol[8];
@@ -155,19 +164,43 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const Grid& g = P.g;
   const int NZ = g.NZ, PN = P.PN;
-  const long long co = COLS ? (long long)blockIdx.y * P.vs : 0LL;
-  const TU* const uc = COLS && P.list ? reinterpret_cast<const TU*>(P.ucol[blockIdx.y]) : reinterpret_cast<const TU*>(P.u) + co;
-  T* const yc = COLS && P.list ? P.ycol[blockIdx.y] : P.ep.y + co;
-  const int w = (int)blockIdx.x % P.nwin, sg = (int)blockIdx.x / P.nwin;
+  // A CTA's output planes are segment sg of window w of column blockIdx.y; with
+  // LINE, the planes of all windows of all columns are one line, cut into equal
+  // parts, and a part is one or more pieces (of one window of one column each).
+  constexpr bool LINE = COLS && line_split<T, EPI>;
+  int count = 0, at = 0, end = 1;  // planes staged by the pieces before; the line
+  if constexpr (LINE) {
+    const long long all = (long long)P.nv * P.nwin * g.NX;
+    at = (int)(all * blockIdx.x / gridDim.x);
+    end = (int)(all * (blockIdx.x + 1) / gridDim.x);
+  }
+  do {
+  int cv = COLS ? (int)blockIdx.y : 0, w, xa, xb;
+  const int staged = LINE ? count : 0;
+  if constexpr (LINE) {
+    const int q = at / g.NX;
+    cv = q / P.nwin;
+    w = q - cv * P.nwin;
+    xa = at - q * g.NX;
+    xb = min(g.NX, xa + (end - at));
+    at += xb - xa;
+  } else {
+    const int sg = (int)blockIdx.x / P.nwin;
+    w = (int)blockIdx.x % P.nwin;
+    xa = (int)((long long)g.NX * sg / P.nseg);
+    xb = (int)((long long)g.NX * (sg + 1) / P.nseg);
+  }
+  const long long co = COLS ? cv * P.vs : 0LL;
+  const TU* const uc = COLS && P.list ? reinterpret_cast<const TU*>(P.ucol[cv]) : reinterpret_cast<const TU*>(P.u) + co;
+  T* const yc = COLS && P.list ? P.ycol[cv] : P.ep.y + co;
   const int n0 = w * P.TO, n1 = min(PN, n0 + P.TO);  // output nodes of a plane
-  const int xa = (int)((long long)g.NX * sg / P.nseg), xb = (int)((long long)g.NX * (sg + 1) / P.nseg);  // output planes
   const int mlo = n0 - NZ - 1;                                             // first element of the window
   const int ms = max(mlo, 0), me = min(PN, mlo + 31 * NW + NZ + 2);        // staged nodes of every plane
   const int pf = max(xa - 1, 0), pl = min(xb, g.NX - 1);                   // planes read
   const uint32_t bar0 = smem_u32(sm + P.off_bar);
 
   for (int i = tid; i < P.off_pw / 16; i += NT) reinterpret_cast<uint4*>(sm)[i] = make_uint4(0, 0, 0, 0);
-  if (tid == 0) {
+  if (tid == 0 && staged == 0) {
     for (int s = 0; s < RING; ++s) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8u * s), "r"(1) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -177,10 +210,10 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   chain_release();
   if (P.st != nullptr && P.st->done) return;
 
-  // plane p -> slot (p - pf) % RING; node n of it at byte 16 + shift + 3 SU (n - mlo),
+  // plane p -> slot (staged + p - pf) % RING; node n of it at byte 16 + shift + 3 SU (n - mlo),
   // where shift makes the copy's source and destination agree modulo 16
   auto issue = [&](int p) {  // thread 0
-    const int sl = (p - pf) % RING;
+    const int sl = (staged + p - pf) % RING;
     const int shift = (int)((((long long)p * PN + mlo) * (3 * SU)) & 15);
     const long long off0 = ((long long)p * PN + ms) * (3 * SU);
     const long long n = (long long)(me - ms) * (3 * SU);
@@ -320,8 +353,8 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
     }
   };
 
-  int slot = 0;                                                      // of the current plane
-  uint32_t phase = 0;                                                // of that slot's barrier
+  int slot = staged % RING;                                          // of the current plane
+  uint32_t phase = (uint32_t)((staged / RING) & 1);                  // of that slot's barrier
   int shift = (int)((((long long)pf * PN + mlo) * (3 * SU)) & 15);   // of the current plane
   const int dshift = (int)(((long long)PN * (3 * SU)) & 15);
   // wait for the current plane; also a CTA barrier: the step before has read
@@ -422,7 +455,7 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
 
   bool ok = arrive();
   if (ok) {
-    transform(ucol + shift, prev);
+    transform(ucol + slot * P.slot + shift, prev);
     advance();
   }
   // two steps per round, so that the two planes' registers swap roles
@@ -452,7 +485,8 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
   } else if (tid == 0) {
     for (int j = max(pf, issued - RING); j < issued; ++j)
       if (!(P.skip && j == pf))
-        for (int it = 0; it < P.poll && !mbar_try(bar0 + 8u * (uint32_t)((j - pf) % RING), (uint32_t)(((j - pf) / RING) & 1)); ++it) {
+        for (int it = 0; it < P.poll && !mbar_try(bar0 + 8u * (uint32_t)((staged + j - pf) % RING),
+                                                  (uint32_t)(((staged + j - pf) / RING) & 1)); ++it) {
         }
   }
   if constexpr (EPI == Epi::StoreDot) {
@@ -463,6 +497,10 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
       P.st->alpha = P.st->rz / tot[0];
     }
   }
+  if constexpr (!LINE) break;
+  if (!ok) break;  // (uniform)
+  count += pl - pf + 1;
+  } while (at < end);
 }
 
 }  // namespace pt
@@ -528,7 +566,7 @@ struct Width {
 constexpr int kPtSmem = 200 * 1024;  // dynamic shared memory of one CTA at most
 
 struct PtLayout {
-  int w, TO, nwin, nseg, slot, off_pw, pw_n, off_bar, total;
+  int w, TO, nwin, nseg, ctas, slot, off_pw, pw_n, off_bar, total;
 };
 
 // Window width and segments. A CTA of NW warps yields 31 NW - NZ nodes per
@@ -539,9 +577,10 @@ struct PtLayout {
 // than 3/4 of its elements on the halo is left out; with none left (NZ above
 // 372, in FP64 186) the general kernels take the mesh.
 template <typename T, Epi EPI>
-bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
+bool pt_layout(const Grid& g, int s_u, bool cols, int nv, int nsm, PtLayout& best) {
+  const bool line = cols && pt::line_split<T, EPI>;
   const long long PN = (long long)g.NY * g.NZ;
-  if (PN >= (1 << 28)) return false;
+  if (PN >= (1 << 28) || PN * g.NX >= (1LL << 31)) return false;
   double cost = 1e300;
   for (int w = 0; w < 3; ++w) {
     const int NW = Width<T, EPI>::NW[w], TO = 31 * NW - g.NZ;
@@ -550,12 +589,22 @@ bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
     L.w = w;
     L.TO = TO;
     L.nwin = (int)((PN + TO - 1) / TO);
-    const long long slots = std::max<long long>(1, (long long)nsm * Width<T, EPI>::PER[w] / nv);  // per column
-    L.nseg = (int)std::max<long long>(1, std::min<long long>(g.NX, slots / L.nwin));
-    const long long ctas = (long long)L.nwin * L.nseg;
-    const double waves = std::ceil((double)ctas / (double)slots);
-    const double per = std::min<double>(Width<T, EPI>::PER[w], std::ceil((double)ctas * nv / nsm));
-    const double c = waves * ((g.NX + L.nseg - 1) / L.nseg + 1) * std::max(8.0, per * NW);
+    const long long slots = (long long)nsm * Width<T, EPI>::PER[w], all = (long long)nv * L.nwin * g.NX;
+    double layers, waves = 1.0;
+    if (line) {
+      L.nseg = 1;
+      L.ctas = (int)std::max<long long>(1, std::min(slots, all / 4));
+      const double part = std::ceil((double)all / L.ctas);
+      layers = part + 2.0 * (1.0 + part / g.NX);  // a piece costs two: its extra layer and the start of the ring
+    } else {
+      const long long own = std::max<long long>(1, slots / nv);  // a column's share
+      L.nseg = (int)std::max<long long>(1, std::min<long long>(g.NX, own / L.nwin));
+      L.ctas = L.nwin * L.nseg;
+      waves = std::ceil((double)L.ctas / (double)own);
+      layers = (g.NX + L.nseg - 1) / L.nseg + 1;
+    }
+    const double per = std::min<double>(Width<T, EPI>::PER[w], std::ceil((double)L.ctas * (line ? 1 : nv) / nsm));
+    const double c = waves * layers * std::max(8.0, per * NW);
     const auto al = [](long long x) { return (int)((x + 127) & ~127LL); };
     L.slot = al(64 + 3LL * s_u * (31 * NW + g.NZ + 3));
     L.off_pw = pt::RING * L.slot;
@@ -571,7 +620,7 @@ bool pt_layout(const Grid& g, int s_u, int nv, int nsm, PtLayout& best) {
 }
 
 template <typename T, typename TU, bool BF, Epi EPI, int W, bool COLS>
-void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t s) {
+void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, cudaStream_t s) {
   auto* k = pt::k_level0_pt<T, TU, BF, EPI, COLS, Width<T, EPI>::NW[W], Width<T, EPI>::PER[W]>;
   static std::atomic<uint64_t> raised{0};  // devices where this instance's shared-memory limit is raised
   int dev = 0;
@@ -580,14 +629,14 @@ void launch_pt_w(const PtLayout& L, const pt::Params<T>& P, int nv, cudaStream_t
     TOPO_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmem));
     if (dev <= 63) raised |= 1ull << dev;
   }
-  launch_chained(k, dim3((unsigned)(L.nwin * L.nseg), (unsigned)nv), 32 * Width<T, EPI>::NW[W], L.total, s, P);
+  launch_chained(k, dim3((unsigned)L.ctas, COLS && !pt::line_split<T, EPI> ? (unsigned)P.nv : 1u), 32 * Width<T, EPI>::NW[W], L.total, s, P);
 }
 
 template <typename T, typename TU, bool BF, Epi EPI>
 void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, const EpiArgs& ea, cudaStream_t s,
                int nv = 1, long long vs = 0, const void* const* ul = nullptr, void* const* yl = nullptr) {
   PtLayout L;
-  if (!pt_layout<T, EPI>(g, (int)sizeof(TU), nv, pt_device().nsm, L))
+  if (!pt_layout<T, EPI>(g, (int)sizeof(TU), nv > 1 || ul, nv, pt_device().nsm, L))
     throw std::runtime_error("level0 K.u: mesh not supported by the parity form");
   pt::Params<T> P;
   P.g = g;
@@ -599,6 +648,7 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   P.E = (const T*)E;
   P.mask = mask;
   P.ep = make_epi<T>(y, ea);
+  P.nv = nv;
   P.vs = vs;
   P.list = ul != nullptr;
   for (int v = 0; v < 8; ++v) {
@@ -618,9 +668,9 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   auto go = [&](auto cols) {
     constexpr bool C = decltype(cols)::value;
     switch (L.w) {
-      case 0: launch_pt_w<T, TU, BF, EPI, 0, C>(L, P, nv, s); break;
-      case 1: launch_pt_w<T, TU, BF, EPI, 1, C>(L, P, nv, s); break;
-      default: launch_pt_w<T, TU, BF, EPI, 2, C>(L, P, nv, s); break;
+      case 0: launch_pt_w<T, TU, BF, EPI, 0, C>(L, P, s); break;
+      case 1: launch_pt_w<T, TU, BF, EPI, 1, C>(L, P, s); break;
+      default: launch_pt_w<T, TU, BF, EPI, 2, C>(L, P, s); break;
     }
   };
   if constexpr (EPI == Epi::Store || EPI == Epi::ChebR || EPI == Epi::RUpd) {
@@ -671,7 +721,7 @@ bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
   const PtDevice& d = pt_device();
   PtLayout L;
   return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 &&
-         (f64 ? pt_layout<double, Epi::ChebR>(g, 8, 1, d.nsm, L) : pt_layout<float, Epi::ChebR>(g, 4, 1, d.nsm, L));  // (the narrowest)
+         (f64 ? pt_layout<double, Epi::ChebR>(g, 8, false, 1, d.nsm, L) : pt_layout<float, Epi::ChebR>(g, 4, false, 1, d.nsm, L));  // (the narrowest)
 }
 
 // f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
