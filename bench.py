@@ -177,16 +177,16 @@ def ku_micro(reps: int = 100, pairs: int = 8):
                      "launches_per_apply": (ctx._lib.topo_launch_count() - n0) / reps}
     out["fp32"]["rel_l2_vs_fp64"] = _rel_l2(first["fp32"], first["fp64"])
     out["bf16"]["rel_l2_vs_fp64"] = _rel_l2(first["bf16"], first["fp64"])
-    out["kernels"] = {"fp64": "k_level0_cc<double, Store> (CUDA cores, TMA-staged x-planes)",
-                      "fp32": "k_level0_cc<float, Store> (CUDA cores, TMA-staged x-planes)",
-                      "bf16": "k_level0_xs<bf16, Store> (tcgen05 node-pair tiles, BF16 u, TMA-staged x-planes)"}
+    out["kernels"] = {"fp64": "k_level0_pt<double, Store> (parity form, TMA-staged x-planes)",
+                      "fp32": "k_level0_pt<float, Store> (parity form, TMA-staged x-planes)",
+                      "bf16": "k_level0_pt<bf16, Store> (parity form, BF16 u and KE, TMA-staged x-planes)"}
     ctx.close()
     return out
 
 
 def cheb_micro(reps: int = 30, sets: int = 3):
     """The Chebyshev step the mixed smoother runs on level 0, alone: the
-    tensor-core K.u with FP32 u rounded to BF16 when staged and the fused
+    parity-form K.u with FP32 u rounded to BF16 as it is read and the fused
     epilogue r -= s K u; d = c1 u + c2 dinv r; x += ax d, on the 160x80x80
     SIMP mesh with `sets` rotating vector sets (> L2). Algorithmic bytes per
     launch: ndof*(4 u + 8 r + 4 dinv + 8 x + 4 d) + nelem*4 E."""
@@ -226,7 +226,7 @@ def cheb_micro(reps: int = 30, sets: int = 3):
     ms = e0.elapsed_time(e1) / reps
     byts = nd * 28 + ne * 4
     ctx.close()
-    return {"kernel": "k_level0_xs<float, ChebR> (tcgen05 node-pair tiles, FP32 u rounded to BF16, fused Chebyshev epilogue)",
+    return {"kernel": "k_level0_pt<float, ChebR> (parity form, FP32 u rounded to BF16, fused Chebyshev epilogue)",
             "workload": "160x80x80 hex8 (3,168,963 DoF), 3 rotating vector sets", "ms": ms, "bytes": byts,
             "gbs": byts / (ms * 1e-3) / 1e9, "gdof_s": nd / (ms * 1e-3) / 1e9}
 
@@ -543,12 +543,12 @@ def main():
     roof = {"kernel": micro["kernels"]["bf16"] + ", level-0 K.u y = K(E) u",
             "workload": "192x96x48 hex8 (2,751,987 DoF), 8 rotating (u,y) pairs", "bound": "hbm",
             "achieved": b["gbs"], "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": b["gbs"] / pk["hbm_gbs"],
-            "traffic": traffic_for("k_level0_xs_bf16_store_192x96x48"), "peak_source": pk["source"],
+            "traffic": traffic_for("k_level0_pt_bf16_store_192x96x48"), "peak_source": pk["source"],
             "bytes_per_launch": b["bytes"], "launch_ms": b["ms"]}
     ch = cheb_micro()
     roof_cheb = {"kernel": ch["kernel"], "workload": ch["workload"], "bound": "hbm", "achieved": ch["gbs"],
                  "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": ch["gbs"] / pk["hbm_gbs"],
-                 "traffic": traffic_for("k_level0_xs_float_cheb_160x80x80"), "peak_source": pk["source"],
+                 "traffic": traffic_for("k_level0_pt_float_cheb_160x80x80"), "peak_source": pk["source"],
                  "bytes_per_launch": ch["bytes"], "launch_ms": ch["ms"]}
 
     iters = [r["outer_iters"] for r in mixed["rows"][args.warmup:]]

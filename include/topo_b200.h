@@ -101,15 +101,16 @@ int topo_modulus(topo_ctx* ctx, const double* rho, double penal, double E0, doub
  * FusedMatvec.matvec/matvec_full (src/gpu_fem/cuda_fused_matvec.py:336-384).
  *  dtype TOPO_F64: u,y,E double.  TOPO_F32: u,y,E float.
  *  TOPO_BF16: u bf16 (uint16 bit patterns), y float, E float; products of
- *  BF16-rounded u and KE accumulated in FP32 on the tensor cores. */
+ *  BF16-rounded u and KE accumulated in FP32. Runs on `stream` itself. */
 int topo_matvec(topo_ctx* ctx, int dtype, const void* u, void* y, const void* E, void* stream);
 
 /* Level-0 operator with its fused epilogue: the building block of the
  * smoother, exposed so each form can be checked on its own.
- *  u_dtype TOPO_F64: FP64 CUDA cores; u, E and the epilogue vectors double.
- *          TOPO_F32: FP32 CUDA cores; everything float.
- *          TOPO_BF16 / TOPO_BF16_F32IN: tensor cores, u bf16 / float, E and
- *          the epilogue vectors float.
+ *  u_dtype TOPO_F64: u, E and the epilogue vectors double.
+ *          TOPO_F32: everything float.
+ *          TOPO_BF16 / TOPO_BF16_F32IN: products of BF16-rounded u and KE
+ *          accumulated in FP32, u bf16 / float, E and the epilogue vectors
+ *          float.
  *  epi TOPO_EPI_STORE    y = K u
  *      TOPO_EPI_RESIDUAL y = b - K u
  *      TOPO_EPI_RUPD     r = r - s K u
@@ -136,10 +137,11 @@ int topo_level0_apply(topo_ctx* ctx, int u_dtype, int epi, const void* u, const 
  * level-0 kernel launched before it timed out. */
 int topo_wait_status(topo_ctx* ctx, void* stream);
 
-/* Test hook for the bounded waits: with skip_first_arrival != 0 the
- * tensor-core K.u's converter warps withhold their first arrival, so its
- * MMA role's wait runs out after poll_limit polls (<= 0: the default limit)
- * and the kernel raises the flag. Applies to later launches in this
+/* Test hook for the bounded waits: with skip_first_arrival != 0 the BF16
+ * level-0 K.u withholds its first arrival (the parity form its first plane's
+ * copy, the tensor-core form a converter warp's arrival), so the wait for it
+ * runs out after poll_limit polls (<= 0: the default limit) and the kernel
+ * raises the flag. Applies to later launches in this
  * process. */
 int topo_debug_tc_wait(int skip_first_arrival, int poll_limit);
 
@@ -194,9 +196,9 @@ int topo_fgmres(topo_ctx* ctx, const void* b, void* x, double tol, int maxiter, 
  * the reference refactorises synchronously (multigrid_v4.py:774-811). */
 int topo_set_coarse_lag(topo_ctx* ctx, int on);
 
-/* BF16 level-0 operator on the tensor cores (on != 0, the default) or on the
- * CUDA cores (same BF16 inputs and FP32 accumulation, another summation
- * order); a tuning switch with no reference counterpart. */
+/* BF16 level-0 operator, where KE or the mesh does not allow the parity form:
+ * on the tensor cores (on != 0, the default) or on the CUDA cores (same BF16
+ * inputs and FP32 accumulation, another summation order); a tuning switch with no reference counterpart. */
 int topo_set_tc(topo_ctx* ctx, int on);
 
 /* Block PCG for nrhs load cases (1..8) on the current hierarchy: B and X are

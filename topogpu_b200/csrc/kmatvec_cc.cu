@@ -1,7 +1,7 @@
 // kmatvec_cc.cu - level-0 hex8 K.u on the CUDA cores (FP32 or FP64),
 // streaming along x with TMA-staged node planes. Runs the stiffnesses without
 // the cube's mirror symmetry and z extents above the windows of kmatvec_pt.cu
-// (which takes the others: FP32 24.6 us against 64 us at 160x80x80).
+// (which takes the others: FP32 24.5 us against 64 us at 160x80x80).
 //
 // Same work decomposition as the tensor-core kernel: a persistent CTA takes
 // a contiguous range of (window, node plane) items; a window owns R

@@ -554,7 +554,7 @@ bool class_blocks(const double* KE, double* K) {
 // Kernel widths: the (warps per CTA, CTAs per SM) pairs an instance is
 // compiled for. FP32: 512 threads per SM (128 registers each); FP64: 384 (168),
 // for the Chebyshev epilogue with its five operands per DoF 256 (255). More
-// threads with fewer registers spill (160x80x80: FP32 Store 24.6 us with 512
+// threads with fewer registers spill (160x80x80: FP32 Store 24.5 us with 512
 // threads per SM, 30.4 with 768, 32.5 with 1024; FP64 Chebyshev step at
 // 96x48x48 18 us with 256, 23 with 384).
 template <typename T, Epi EPI>

@@ -1,7 +1,7 @@
 // kmatvec_xs.cu - level-0 hex8 K.u with BF16 inputs on the tcgen05 tensor
 // cores (FP32 accumulation in tensor memory), streaming along x. Runs the
 // stiffnesses without the cube's mirror symmetry (kmatvec_pt.cu takes the
-// others: 36 us against 67 us for a Chebyshev step at 160x80x80).
+// others: 35 us against 67 us for a Chebyshev step at 160x80x80).
 //
 // Memory order of every level-0 vector is z fastest (DoF 3*node+c, node
 // (ix*NY+iy)*NZ+iz), so one x-plane of a window of consecutive y-rows is one
