@@ -220,6 +220,7 @@ __device__ __forceinline__ void chol_step(double (&wr)[CNB], int lane, CholSmem&
     S.piv[J] = e0;
     S.piv[J + 1] = e1;
   }
+  __syncwarp();  // every lane has read the columns that the next round overwrites
   if constexpr (J + 2 < CNB) chol_step<J + 2>(wr, lane, S, bad);
 }
 
