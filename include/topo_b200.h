@@ -145,6 +145,11 @@ int topo_wait_status(topo_ctx* ctx, void* stream);
  * process. */
 int topo_debug_tc_wait(int skip_first_arrival, int poll_limit);
 
+/* Test query (host only, no GPU work): the largest number of CTAs that leave a
+ * partial sum when the level-0 operator of this mesh runs with its dot product
+ * on a GPU of nsm SMs, and the partial sums a context of the mesh has room for. */
+int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long long* blocks, long long* room);
+
 /* Index range checks (no reference counterpart). In the library built with
  * -DTOPO_DEBUG_BOUNDS (libtopo_b200_dbg.so: python -m topogpu_b200.build
  * --debug-bounds) every checked gather/scatter index of the kernels is

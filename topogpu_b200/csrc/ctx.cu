@@ -1352,7 +1352,9 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->Fvec = c->alloc<double>(g0.ndof);
     c->st = c->alloc<KrylovState>(1);
     TOPO_CUDA_CHECK(cudaMallocHost((void**)&c->h_st, sizeof(KrylovState)));
-    c->red.partials = c->alloc<double>(1 << 18);
+    int nsm = 0;
+    TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+    c->red.partials = c->alloc<double>(reduction_room(g0, nsm));
     c->red.ticket = c->alloc<unsigned int>(1);
     c->dtmp = c->alloc<double>(64);
     c->oc_state = c->alloc<double>(32);
@@ -1606,6 +1608,20 @@ int topo_debug_bounds(int* tripped) {
 #endif
   } catch (const std::exception& e) {
     return fail(nullptr, e);
+  }
+}
+
+int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long long* blocks, long long* room) {
+  try {
+    if (!blocks || !room) throw std::invalid_argument("topo_debug_reduction: null pointer");
+    if (nelx < 1 || nely < 1 || nelz < 1 || nsm < 1) throw std::invalid_argument("topo_debug_reduction: sizes must be >= 1");
+    const Grid g = make_grid(nelx, nely, nelz);
+    *blocks = level0_dot_blocks(g, f64 != 0, nsm);
+    *room = reduction_room(g, nsm);
+    return 0;
+  } catch (const std::exception& e) {
+    set_global_error(e.what());
+    return -1;
   }
 }
 

@@ -125,7 +125,7 @@ constexpr int kRedThreads = 256;
 constexpr int kRedSlots = 8;
 
 struct RedWork {
-  double* partials;   // kRedBlocks * kRedSlots
+  double* partials;   // reduction_room(grid, SMs) doubles
   unsigned int* ticket;
 };
 
@@ -218,6 +218,11 @@ void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uin
 void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask,
                        const uint8_t* nmask, void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true, int nv = 1,
                        long long vs = 0);
+// CTAs of the largest launch of the level-0 operator with its dot product (each
+// leaves one partial sum), whichever kernel takes the mesh; doubles a context's
+// partial sums need, with room for the vector reductions
+long long level0_dot_blocks(const Grid& g, bool f64, int nsm);
+long long reduction_room(const Grid& g, int nsm);
 void level0_diag(const Grid& g, const double* E, const uint8_t* mask, double* diag, cudaStream_t s);
 // tensor-core BF16-input operator streaming along x (kmatvec_xs.cu); the
 // KE tile and the error flag are per device
@@ -237,6 +242,7 @@ void level0_apply_cc(bool f64, const Grid& g, const void* u, const void* E, cons
 // level-0 K.u in parity form (kmatvec_pt.cu): KE with the cube's mirror symmetry
 void pt_prepare(const double* KE_host);
 bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u);
+long long pt_dot_blocks(const Grid& g, bool f64, int nsm);  // CTAs of the StoreDot form (0: no layout)
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
                      Epi epi, const EpiArgs& ea, cudaStream_t s, int nv = 1, long long vs = 0);
 void level0_columns_pt(const Grid& g, const double* const* U, const double* E, const uint8_t* mask, double* const* Y, int nv,

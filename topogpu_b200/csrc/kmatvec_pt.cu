@@ -724,6 +724,12 @@ bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
          (f64 ? pt_layout<double, Epi::ChebR>(g, 8, false, 1, d.nsm, L) : pt_layout<float, Epi::ChebR>(g, 4, false, 1, d.nsm, L));  // (the narrowest)
 }
 
+long long pt_dot_blocks(const Grid& g, bool f64, int nsm) {
+  PtLayout L;
+  const bool ok = f64 ? pt_layout<double, Epi::StoreDot>(g, 8, false, 1, nsm, L) : pt_layout<float, Epi::StoreDot>(g, 4, false, 1, nsm, L);
+  return ok ? L.ctas : 0;
+}
+
 // f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
 // where it is read) or stored BF16 (u_bf16). Epilogues as level0_apply. nv
 // columns vs entries apart (u of each 16-byte aligned; one for StoreDot).

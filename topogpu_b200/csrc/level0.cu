@@ -246,6 +246,15 @@ static void launch_level0(const Grid& g, const void* u, const void* E, const uin
   TOPO_LAUNCH_CHECK();
 }
 
+long long level0_dot_blocks(const Grid& g, bool f64, int nsm) {
+  const long long brick = (long long)((g.NZ + TZ - 1) / TZ) * ((g.NY + TY - 1) / TY) * ((g.NX + TX - 1) / TX);
+  return std::max({brick, pt_dot_blocks(g, f64, nsm), (long long)nsm});
+}
+
+long long reduction_room(const Grid& g, int nsm) {
+  return std::max({1LL << 18, level0_dot_blocks(g, true, nsm), level0_dot_blocks(g, false, nsm)});
+}
+
 // The operands of the column `at` entries on.
 struct ColumnAt {
   const void* u;
