@@ -230,15 +230,24 @@ struct topo_ctx {
   long long bytes = 0;
   std::string err;
 
+  // Device memory of the context. alloc zeroes it on the context's stream: a
+  // memset on the default stream is not ordered with that stream or with a
+  // caller's non-blocking one. Memory that a call on the caller's stream makes
+  // comes from alloc_raw and is written there before it is read.
   template <typename T>
-  T* alloc(long long count) {
+  T* alloc_raw(long long count) {
     void* p = nullptr;
     const size_t sz = (size_t)std::max<long long>(count, 1) * sizeof(T);
     TOPO_CUDA_CHECK(cudaMalloc(&p, sz));
-    TOPO_CUDA_CHECK(cudaMemset(p, 0, sz));
     allocs.push_back(p);
     bytes += (long long)sz;
     return (T*)p;
+  }
+  template <typename T>
+  T* alloc(long long count) {
+    T* p = alloc_raw<T>(count);
+    TOPO_CUDA_CHECK(cudaMemsetAsync(p, 0, (size_t)std::max<long long>(count, 1) * sizeof(T), cs));
+    return p;
   }
   void* valloc(long long count) { return vec64 ? (void*)alloc<double>(count) : (void*)alloc<float>(count); }
   size_t vsize() const { return vec64 ? 8 : 4; }
@@ -1368,6 +1377,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->C.scrA = c->alloc<double>(maxc);
     c->C.scrB = c->alloc<double>(maxc);
     c->C.scrC = c->alloc<double>(maxc);
+    TOPO_CUDA_CHECK(cudaStreamSynchronize(c->cs));  // calls on other streams find the zeroes
     *out = c;
     return 0;
   } catch (const std::exception& e) {
@@ -1849,7 +1859,7 @@ int topo_oc_projected(topo_ctx* c, double rmin, const double* rho, const double*
       throw std::invalid_argument("topo_oc_projected: out must not alias rho, dc or dv");
     DirectGuard sg(c, stream);
     cudaStream_t us = sg.user;
-    if (!c->oc_cand) c->oc_cand = c->alloc<double>(oc_projected_candidates() * c->L[0].g.nelem);
+    if (!c->oc_cand) c->oc_cand = c->alloc_raw<double>(oc_projected_candidates() * c->L[0].g.nelem);
     const int ev = oc_update_projected(c->fstencil, c->L[0].g, rmin, rho, dc, dv, beta, eta, volfrac, move, rho_min, out, c->Hs,
                                        c->oc_cand, c->red, c->oc_state, us);
     if (out_evals) *out_evals = ev;
