@@ -124,8 +124,8 @@ struct Level {
   __nv_bfloat16* S16 = nullptr;
   double lam = NAN;
   int degree = 2;
-  // the V-cycle's vectors for several columns (x, r, d, d2, e, b; allocated by
-  // the first block solve), vs entries from column to column
+  // the V-cycle's vectors for several columns (x, r, d, d2, e, b; made by
+  // block_reserve), vs entries from column to column
   void* cols[6] = {};  // (the last one on level 0 only)
   long long vs = 0;
 };
@@ -134,6 +134,7 @@ struct Level {
 struct FactorSlot {
   double* S64c = nullptr;   // copy of the coarsest stencil the factor is built from
   CoarsestFactor f;
+  std::vector<void*> own;   // its allocations
 };
 
 struct Coarsest {
@@ -198,13 +199,13 @@ struct topo_ctx {
   cudaGraphExec_t pcg_exec = nullptr;
   long long pcg_exec_kernels = 0;
   std::vector<double> pcg_key;
-  // block PCG workspace (FP64 columns R, Z, P, Q, Pn; allocated per block width)
-  int blk_nv = 0;
+  // block PCG workspace, grown by the widest block so far (block_reserve)
   int bw = 1;                   // columns the V-cycle works on
-  int blk_cols = 0;             // columns the levels' block vectors hold
-  int blk_n = 0;                // coarsest size they were made for
-  double* blk_y = nullptr;      // coarsest work of every column
-  double* blk = nullptr;
+  int blk_cols = 0;             // columns the workspace holds
+  void* blk_vecs = nullptr;     // the levels' vectors of every column
+  double* blk = nullptr;        // FP64 columns R, Z, P, Q, Pn
+  double* blk_y = nullptr;      // coarsest work of every column,
+  int blk_y_n = 0, blk_y_cols = 0;  // made for this coarsest size and this many columns
   double* blk_part = nullptr;
   double* blk_G = nullptr;
   double* blk_Gh = nullptr;  // pinned host copy
@@ -226,7 +227,7 @@ struct topo_ctx {
   bool has_last = false;
   cudaEvent_t ev_ph[6] = {};     // setup phase marks (timed)
   double setup_ms[5] = {0, 0, 0, 0, 0};
-  std::vector<void*> allocs;
+  std::vector<std::pair<void*, size_t>> allocs;
   long long bytes = 0;
   std::string err;
 
@@ -239,9 +240,19 @@ struct topo_ctx {
     void* p = nullptr;
     const size_t sz = (size_t)std::max<long long>(count, 1) * sizeof(T);
     TOPO_CUDA_CHECK(cudaMalloc(&p, sz));
-    allocs.push_back(p);
+    allocs.push_back({p, sz});
     bytes += (long long)sz;
     return (T*)p;
+  }
+  // Give back what a call has replaced; the caller has waited for its users.
+  void release(void* p) {
+    for (size_t i = 0; i < allocs.size(); ++i)
+      if (allocs[i].first == p) {
+        bytes -= (long long)allocs[i].second;
+        allocs.erase(allocs.begin() + (long)i);
+        cudaFree(p);
+        return;
+      }
   }
   template <typename T>
   T* alloc(long long count) {
@@ -462,15 +473,38 @@ void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cu
 // last of its block vectors. Every kernel covers all columns, so a launch and
 // (on the coarse levels) a fetch of the coefficients serve all of them; the
 // columns one after another left most kernels latency bound.
-void block_reserve(topo_ctx* c, int nv) {
-  if (c->blk_cols >= nv && c->blk_n == c->C.n) return;
-  for (Level& Lv : c->L) {
-    Lv.vs = (Lv.g.ndof + 3) & ~3LL;  // columns 16-byte aligned in FP32 and FP64
-    for (int i = 0; i < (&Lv == &c->L[0] ? 6 : 5); ++i) Lv.cols[i] = c->valloc(nv * Lv.vs);
+//
+// The workspace of nv columns: made by the first block solve, replaced by a
+// wider one's, and kept. Only the coarsest work depends on the coarsest size.
+void block_reserve(topo_ctx* c, int nv, cudaStream_t s) {
+  if (c->blk_cols < nv) {
+    TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
+    c->blk_cols = 0;
+    c->release(c->blk_vecs);
+    c->release(c->blk);
+    c->blk_vecs = c->blk = nullptr;
+    long long total = 0;
+    for (Level& Lv : c->L) {
+      Lv.vs = (Lv.g.ndof + 3) & ~3LL;  // columns 16-byte aligned in FP32 and FP64
+      std::fill(Lv.cols, Lv.cols + 6, nullptr);
+      total += (&Lv == &c->L[0] ? 6 : 5) * nv * Lv.vs;
+    }
+    c->blk = c->alloc<double>(5 * nv * c->L[0].vs);
+    c->blk_vecs = c->valloc(total);
+    char* at = (char*)c->blk_vecs;
+    for (Level& Lv : c->L)
+      for (int i = 0; i < (&Lv == &c->L[0] ? 6 : 5); ++i, at += c->vsize() * nv * Lv.vs) Lv.cols[i] = at;
+    c->blk_cols = nv;
   }
-  c->blk_y = c->alloc<double>(2LL * std::max(c->C.n, 1) * nv);
-  c->blk_n = c->C.n;
-  c->blk_cols = nv;
+  if (c->blk_y_n != c->C.n || c->blk_y_cols < nv) {
+    TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
+    c->blk_y_cols = 0;
+    c->release(c->blk_y);
+    c->blk_y = nullptr;
+    c->blk_y = c->alloc<double>(2LL * std::max(c->C.n, 1) * c->blk_cols);
+    c->blk_y_n = c->C.n;
+    c->blk_y_cols = c->blk_cols;
+  }
 }
 
 // b, x: level 0's input and output columns, Lv.vs entries apart.
@@ -649,11 +683,28 @@ void* ctx_alloc_bytes(void* ctx, size_t bytes) {
   return static_cast<void*>(static_cast<topo_ctx*>(ctx)->alloc<char>((long long)bytes));
 }
 
+void release_slot(topo_ctx* c, FactorSlot& f) {
+  for (void* p : f.own) c->release(p);
+  f = FactorSlot();
+}
+
+// The buffers of one slot: all of them, or none when an allocation fails.
 void alloc_slot(topo_ctx* c, FactorSlot& f) {
-  f.S64c = c->alloc<double>(243LL * c->L[c->n_levels - 1].g.nnodes);
-  coarsest_alloc(f.f, c->C.plan, c->C.band, c->vec64, ctx_alloc_bytes, c);
+  const size_t before = c->allocs.size();
+  auto keep = [&] {
+    for (size_t i = before; i < c->allocs.size(); ++i) f.own.push_back(c->allocs[i].first);
+  };
+  try {
+    f.S64c = c->alloc<double>(243LL * c->L[c->n_levels - 1].g.nnodes);
+    coarsest_alloc(f.f, c->C.plan, c->C.band, c->vec64, ctx_alloc_bytes, c);
+  } catch (...) {
+    keep();
+    release_slot(c, f);
+    throw;
+  }
   f.f.d_free = c->C.free_list;
   f.f.kind = 0;
+  keep();
 }
 
 // Assembly (from the slot's stencil copy) and factorisation of one slot.
@@ -981,17 +1032,11 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
                  double* out_relres, cudaStream_t s) {
   Level& L0 = c->L[0];
   const long long n = L0.g.ndof;
-  const long long ld = (n + 3) & ~3LL;  // column stride: 16-byte aligned columns
-  if (c->blk_nv != nv) {
-    c->blk = c->alloc<double>(5LL * nv * ld);
-    if (!c->blk_part) {
-      c->blk_part = c->alloc<double>((long long)block_gram_partials());
-      c->blk_G = c->alloc<double>(64);
-      TOPO_CUDA_CHECK(cudaMallocHost(&c->blk_Gh, 64 * sizeof(double)));
-    }
-    c->blk_nv = nv;
-  }
-  block_reserve(c, nv);
+  if (!c->blk_part) c->blk_part = c->alloc<double>((long long)block_gram_partials());
+  if (!c->blk_G) c->blk_G = c->alloc<double>(64);
+  if (!c->blk_Gh) TOPO_CUDA_CHECK(cudaMallocHost(&c->blk_Gh, 64 * sizeof(double)));
+  block_reserve(c, nv, s);
+  const long long ld = L0.vs;  // column stride
   double *R0 = c->blk, *Z0 = R0 + nv * ld, *P0 = Z0 + nv * ld, *Q0 = P0 + nv * ld, *N0 = Q0 + nv * ld;
   auto col = [&](double* base, int j) { return base + j * ld; };
   auto gram = [&](double* const* A, int na, double* const* Bm, int nb, double* Gout) {
@@ -1008,7 +1053,7 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     char* b0 = (char*)L0b.cols[5];
     char* x0 = (char*)L0b.cols[0];
     const long long st = L0b.vs * (long long)c->vsize();
-    bool side = c->vec64 && L0b.vs == ld;
+    bool side = c->vec64;
     for (int a = 1; a < k; ++a) side = side && r[a] == r[0] + a * ld && z[a] == z[0] + a * ld;
     if (side) {
       vcycle_columns(c, k, r[0], z[0], s);
@@ -1394,7 +1439,7 @@ int topo_ctx_destroy(topo_ctx* c) {
   if (c->cs) cudaStreamSynchronize(c->cs);
   if (c->has_last) cudaEventSynchronize(c->ev_last);
   release_ke(c);
-  for (void* p : c->allocs) cudaFree(p);
+  for (auto& a : c->allocs) cudaFree(a.first);
   if (c->h_st) cudaFreeHost(c->h_st);
   if (c->blk_Gh) cudaFreeHost(c->blk_Gh);
   if (c->pcg_exec) cudaGraphExecDestroy(c->pcg_exec);
@@ -1485,18 +1530,26 @@ int topo_set_problem(topo_ctx* c, const uint8_t* free_mask, const double* F, voi
       c->C.have = false;
       CoarsestPlan plan = coarsest_plan(Lc.g, fl);
       if (c->C.n != n || c->C.band != band || c->C.cur.S64c == nullptr) {
+        // replace the factors' buffers; nothing uses the old ones after the
+        // wait above and the PCG graph that names them, and a call that fails
+        // on the way leaves a context without a problem
+        c->problem_set = c->setup_done = false;
+        if (c->pcg_exec) cudaGraphExecDestroy(c->pcg_exec);
+        c->pcg_exec = nullptr;
+        const bool lagged = c->C.nxt.S64c != nullptr;
+        release_slot(c, c->C.cur);
+        release_slot(c, c->C.nxt);
+        for (void* p : {(void*)c->C.dof_index, (void*)c->C.free_list, (void*)c->C.y}) c->release(p);
+        c->C.dof_index = c->C.free_list = nullptr;
+        c->C.y = nullptr;
         c->C.n = n;
         c->C.band = band;
         c->C.plan = plan;
         c->C.dof_index = c->alloc<int>(Lc.g.ndof);
         c->C.free_list = c->alloc<int>(std::max(n, 1));
         c->C.y = c->alloc<double>(2 * (size_t)std::max(n, 1));
-        c->C.cur = FactorSlot();
+        if (lagged) alloc_slot(c, c->C.nxt);
         alloc_slot(c, c->C.cur);
-        if (c->C.nxt.S64c) {
-          c->C.nxt = FactorSlot();
-          alloc_slot(c, c->C.nxt);
-        }
       }
       TOPO_CUDA_CHECK(cudaMemsetAsync(Lc.x, 0, c->vsize() * Lc.g.ndof, s));
       if (Lc.cols[0]) TOPO_CUDA_CHECK(cudaMemsetAsync(Lc.cols[0], 0, c->vsize() * Lc.vs * c->blk_cols, s));
