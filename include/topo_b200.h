@@ -129,20 +129,21 @@ int topo_level0_apply(topo_ctx* ctx, int u_dtype, int epi, const void* u, const 
  * flag in mapped host memory, drains its copies in flight and exits. The
  * asynchronous entries (topo_matvec, topo_level0_apply, topo_gmg_apply)
  * report a flag raised by an earlier launch that has finished, before they
- * launch; topo_pcg / topo_solve and topo_wait_status synchronise and report
- * it at once. The flag is cleared when reported. */
+ * launch; topo_gmg_setup, topo_pcg, topo_fgmres, topo_block_pcg and
+ * topo_wait_status synchronise and report it at once. The flag is cleared when
+ * reported. */
 
 /* Synchronises the context's stream (stream != NULL: that stream) and
  * returns nonzero, with the message in topo_last_error, when a wait of a
  * level-0 kernel launched before it timed out. */
 int topo_wait_status(topo_ctx* ctx, void* stream);
 
-/* Test hook for the bounded waits: with skip_first_arrival != 0 the BF16
- * level-0 K.u withholds its first arrival (the parity form its first plane's
- * copy, the tensor-core form a converter warp's arrival), so the wait for it
- * runs out after poll_limit polls (<= 0: the default limit) and the kernel
- * raises the flag. Applies to later launches in this
- * process. */
+/* Test hook for the bounded waits: with skip_first_arrival != 0 the level-0
+ * K.u withholds its first arrival (the parity form, every precision, its first
+ * plane's copy; the tensor-core form a converter warp's arrival), so the wait
+ * for it runs out after poll_limit polls (<= 0: the default limit) and the
+ * kernel raises the flag. Applies to later launches in this process, and to
+ * replays of a PCG iteration that was recorded meanwhile. */
 int topo_debug_tc_wait(int skip_first_arrival, int poll_limit);
 
 /* Test query (host only, no GPU work): the largest number of CTAs that leave a

@@ -333,6 +333,12 @@ int fail(topo_ctx* c, const std::exception& e) {
 Prec outer_prec(const topo_ctx* c) { return c->vec64 ? Prec::F64 : Prec::F32; }
 const void* outer_E(const topo_ctx* c) { return c->vec64 ? (const void*)c->E64 : (const void*)c->E32; }
 
+// After the host has waited for the stream: a level-0 kernel whose bounded wait
+// ran out has left its part of the result as it was.
+void check_waits(cudaStream_t s) {
+  if (xs_error_flag(s, false)) throw std::runtime_error("level-0 K.u: an mbarrier wait timed out");
+}
+
 // ----------------------------------------------------------- operators
 // same_bits: the general level-0 kernels, whatever KE's symmetry. A V-cycle
 // with BF16 operators rounds its directions to BF16, and there a last-bit
@@ -762,7 +768,9 @@ void do_setup(topo_ctx* c, const double* E, cudaStream_t s) {
   const double Emax = st4[2];
   const bool re = std::isnan(c->lam_Emax) || std::fabs(Emax - c->lam_Emax) / std::max(std::fabs(c->lam_Emax), 1e-12) > 0.10;
   if (re) {
-    L0.lam = lambda_fine(c, s);
+    const double lam = lambda_fine(c, s);
+    check_waits(s);
+    L0.lam = lam;
     c->lam_Emax = Emax;
   }
   TOPO_CUDA_CHECK(cudaEventRecord(c->ev_ph[1], s));
@@ -979,7 +987,7 @@ int do_pcg(topo_ctx* c, const double* b, double* x, double tol, int maxiter, int
     ++refreshes;
   }
   rr = true_residual(c, s);
-  if (xs_error_flag(s)) throw std::runtime_error("level-0 K.u: an mbarrier wait timed out");
+  check_waits(s);
   if (!std::isfinite(rr)) throw std::runtime_error("topo_pcg: the iteration produced NaN or Inf");
   TOPO_CUDA_CHECK(cudaMemcpyAsync(x, c->kx64, vb, cudaMemcpyDeviceToDevice, s));
   if (out_iters) *out_iters = iters;
@@ -1043,6 +1051,7 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     block_gram(n, (const double* const*)A, na, (const double* const*)Bm, nb, c->blk_part, c->blk_G, s);
     TOPO_CUDA_CHECK(cudaMemcpyAsync(c->blk_Gh, c->blk_G, 64 * sizeof(double), cudaMemcpyDeviceToHost, s));
     TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
+    check_waits(s);  // (a Gram sum follows every K.u and every V-cycle)
     std::memcpy(Gout, c->blk_Gh, 64 * sizeof(double));
   };
   // Z_a = M R_a for the k active columns at once; in place where they lie side
@@ -1201,6 +1210,7 @@ int do_fgmres(topo_ctx* c, const double* b, double* x, double tol, int maxiter, 
   auto Hij = [&](int i, int j) -> double& { return H[i * restart + j]; };
   while (!converged && total < maxiter) {
     const double beta = std::sqrt(true_residual(c, s));
+    check_waits(s);
     if (beta / bn <= tol) {
       converged = true;
       break;
@@ -1220,6 +1230,7 @@ int do_fgmres(topo_ctx* c, const double* b, double* x, double tol, int maxiter, 
         axpby(f64, n, -Hij(i, j), c->fg_V[i], 1.0, c->kt, s);
       }
       const double hn = std::sqrt(dot_host(f64, n, c->kt, c->kt, c->red, c->dtmp, s));
+      check_waits(s);
       Hij(j + 1, j) = hn;
       if (hn > 1e-14) axpby(f64, n, 1.0 / hn, c->kt, 0.0, c->fg_V[j + 1], s);
       for (int i = 0; i < j; ++i) {
@@ -1257,6 +1268,7 @@ int do_fgmres(topo_ctx* c, const double* b, double* x, double tol, int maxiter, 
     for (int i = 0; i < jf; ++i) axpy_to64(f64, n, y[i], c->fg_Z[i], c->kx64, s);
   }
   const double rr = true_residual(c, s);
+  check_waits(s);
   TOPO_CUDA_CHECK(cudaMemcpyAsync(x, c->kx64, vb, cudaMemcpyDeviceToDevice, s));
   if (out_iters) *out_iters = total;
   if (out_relres) *out_relres = bn > 0 ? std::sqrt(rr) / bn : 0.0;

@@ -662,9 +662,7 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   P.off_pw = L.off_pw;
   P.pw_n = L.pw_n;
   P.off_bar = L.off_bar;
-  P.poll = 1 << 22;
-  P.skip = 0;
-  if (BF) wait_debug(P.skip, P.poll);
+  wait_debug(P.skip, P.poll);
   auto go = [&](auto cols) {
     constexpr bool C = decltype(cols)::value;
     switch (L.w) {
