@@ -1418,9 +1418,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->Fvec = c->alloc<double>(g0.ndof);
     c->st = c->alloc<KrylovState>(1);
     TOPO_CUDA_CHECK(cudaMallocHost((void**)&c->h_st, sizeof(KrylovState)));
-    int nsm = 0;
-    TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    c->red.partials = c->alloc<double>(reduction_room(g0, nsm));
+    c->red.partials = c->alloc<double>(reduction_room(g0, sm_count(c->device)));
     c->red.ticket = c->alloc<unsigned int>(1);
     c->dtmp = c->alloc<double>(64);
     c->oc_state = c->alloc<double>(32);

@@ -12,6 +12,8 @@
 #include <type_traits>
 #include <vector>
 
+#include "per_device.cuh"
+
 namespace topo {
 
 // Structured hex grid of one multigrid level: element counts and derived node
@@ -541,6 +543,12 @@ __device__ __forceinline__ constexpr bool topo_in_range(long long, long long) { 
 #endif
 
 namespace topo {
+inline int sm_count(int dev) {
+  int n = 0;
+  TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  return n;
+}
+
 // per translation unit: read and clear its range-check flag (0 in the normal build)
 int bounds_flag_level0();
 int bounds_flag_xs();

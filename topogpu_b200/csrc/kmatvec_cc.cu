@@ -23,8 +23,8 @@
 #include "internal.cuh"
 #include "reduce.cuh"
 
+#include <atomic>
 #include <cstring>
-#include <mutex>
 #include <stdexcept>
 #include <vector>
 
@@ -408,19 +408,16 @@ __global__ void __launch_bounds__(NT) k_level0_cc(const Params<T> P) {
 namespace topo {
 namespace {
 struct CcDevice {
-  int nsm = 0;
-  uint32_t attr_done = 0;
+  std::atomic<int> nsm{0};
+  std::atomic<uint32_t> attr_done{0};  // bit per kernel instance
 };
-std::mutex g_cc_mu;
-std::vector<CcDevice> g_cc;
+PerDevice<CcDevice> g_cc;
 
 CcDevice& cc_device() {
   int dev = 0;
   TOPO_CUDA_CHECK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(g_cc_mu);
-  if ((int)g_cc.size() <= dev) g_cc.resize(dev + 1);
-  CcDevice& d = g_cc[dev];
-  if (d.nsm == 0) TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev));
+  CcDevice& d = g_cc.at(dev);
+  if (d.nsm == 0) d.nsm = sm_count(dev);
   return d;
 }
 
@@ -462,7 +459,6 @@ void launch_cc(const Grid& g, const void* u, const void* E, const uint8_t* mask,
   constexpr int inst = (int)EPI * 2 + (sizeof(T) == 8 ? 1 : 0);
   if (!(d.attr_done & (1u << inst))) {
     TOPO_CUDA_CHECK(cudaFuncSetAttribute(cc::k_level0_cc<T, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCcSmemMax));
-    std::lock_guard<std::mutex> lk(g_cc_mu);
     d.attr_done |= 1u << inst;
   }
   cc::Params<T> P;

@@ -54,7 +54,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
-#include <mutex>
 #include <stdexcept>
 #include <type_traits>
 #include <vector>
@@ -508,19 +507,17 @@ __global__ void __launch_bounds__(32 * NW, MINB) k_level0_pt(const __grid_consta
 // ----------------------------------------------------------------- host side
 namespace {
 struct PtDevice {
-  bool sym64 = false, sym32 = false, symbf = false;  // KE / KE rounded to FP32 / BF16 has the mirror symmetry
-  int nsm = 0;
+  // KE / KE rounded to FP32 / BF16 has the mirror symmetry (set with the device's KE)
+  std::atomic<bool> sym64{false}, sym32{false}, symbf{false};
+  std::atomic<int> nsm{0};
 };
-std::mutex g_pt_mu;
-std::vector<PtDevice> g_pt;
+PerDevice<PtDevice> g_pt;
 
 PtDevice& pt_device() {
   int dev = 0;
   TOPO_CUDA_CHECK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(g_pt_mu);
-  if ((int)g_pt.size() <= dev) g_pt.resize(dev + 1);
-  PtDevice& d = g_pt[dev];
-  if (d.nsm == 0) TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev));
+  PtDevice& d = g_pt.at(dev);
+  if (d.nsm == 0) d.nsm = sm_count(dev);
   return d;
 }
 

@@ -51,6 +51,7 @@
 // (src/gpu_fem/solver_v2.py:1183-1223) for the operator.
 #include "internal.cuh"
 
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <stdexcept>
@@ -632,21 +633,19 @@ struct XsDevice {
   __nv_bfloat16* B = nullptr;
   int* err = nullptr;       // device alias of err_host
   int* err_host = nullptr;
-  int nsm = 0;
-  uint32_t attr_done = 0;  // bit per kernel instance
+  std::atomic<int> nsm{0};
+  std::atomic<uint32_t> attr_done{0};  // bit per kernel instance
 };
 std::mutex g_xs_mu;
-std::vector<XsDevice> g_xs;
+PerDevice<XsDevice> g_xs;
 int g_xs_skip = 0;         // test hook (topo_debug_tc_wait)
 int g_xs_poll = 1 << 22;   // mbarrier poll limit
 
 XsDevice& xs_device() {
   int dev = 0;
   TOPO_CUDA_CHECK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(g_xs_mu);
-  if ((int)g_xs.size() <= dev) g_xs.resize(dev + 1);
-  XsDevice& d = g_xs[dev];
-  if (d.nsm == 0) TOPO_CUDA_CHECK(cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev));
+  XsDevice& d = g_xs.at(dev);
+  if (d.nsm == 0) d.nsm = sm_count(dev);
   return d;
 }
 
@@ -711,7 +710,6 @@ void launch_xs(const Grid& g, const void* u, const void* E, const uint8_t* nmask
   if (!(d.attr_done & (1u << inst))) {
     TOPO_CUDA_CHECK(
         cudaFuncSetAttribute(xs::k_level0_xs<TU, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax + 1024));
-    std::lock_guard<std::mutex> lk(g_xs_mu);
     d.attr_done |= 1u << inst;
   }
   // Each CTA allocates all 512 tensor-memory columns, so no two may share an
