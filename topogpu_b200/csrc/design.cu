@@ -26,7 +26,8 @@ static void set_filter(FilterStencil& fs, double rmin, cudaStream_t s) {
   std::vector<double> w;
   TapGroups tg;
   tg.R = R;
-  if (R > kMaxFilterR) throw std::runtime_error("filter radius too large (rmin must be < 6)");
+  const char* too_large = "filter radius too large (more than 1331 elements within rmin)";
+  if (R > kMaxFilterR) throw std::runtime_error(too_large);
   for (int dz = -R; dz <= R; ++dz) {  // taps of one dz together: one z test per group
     tg.start[dz + R] = (int)w.size();
     for (int dx = -R; dx <= R; ++dx)
@@ -42,7 +43,7 @@ static void set_filter(FilterStencil& fs, double rmin, cudaStream_t s) {
       }
   }
   tg.start[2 * R + 1] = (int)w.size();
-  if ((int)w.size() > kMaxFilterOff) throw std::runtime_error("filter radius too large (rmin must be < 6)");
+  if ((int)w.size() > kMaxFilterOff) throw std::runtime_error(too_large);
   TOPO_CUDA_CHECK(cudaMemcpyAsync(fs.off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, s));
   TOPO_CUDA_CHECK(cudaMemcpyAsync(fs.w, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice, s));
   TOPO_CUDA_CHECK(cudaStreamSynchronize(s));

@@ -386,8 +386,8 @@ void scale_dev(bool f64, long long n, const void* x, const double* num, const do
 // Offsets and weights of the linear-hat density filter for one radius, in
 // device memory owned by a context (so contexts with different radii, or on
 // different devices, never share it).
-constexpr int kMaxFilterOff = 1331;  // (2*5+1)^3: rmin < 6
-constexpr int kMaxFilterR = 5;
+constexpr int kMaxFilterOff = 1331;  // neighbours of an element: rmin up to 6.78
+constexpr int kMaxFilterR = 6;       // (7 has 1365)
 struct TapGroups {  // taps start[dz + R] .. start[dz + R + 1] - 1 have this dz
   int R;
   int start[2 * kMaxFilterR + 2];
