@@ -151,6 +151,12 @@ int topo_debug_tc_wait(int skip_first_arrival, int poll_limit);
  * on a GPU of nsm SMs, and the partial sums a context of the mesh has room for. */
 int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long long* blocks, long long* room);
 
+/* Test query (host only): the eight 3x3 parity-class blocks (72 doubles, entry
+ * (c, d) of class q at 9 q + 3 c + d, q = 4 qx + 2 qy + qz) of the element
+ * stiffness KE (host, 576 doubles) as the parity form of K.u uses them, and
+ * whether KE has the mirror symmetry that the form needs. */
+int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric);
+
 /* Index range checks (no reference counterpart). In the library built with
  * -DTOPO_DEBUG_BOUNDS (libtopo_b200_dbg.so: python -m topogpu_b200.build
  * --debug-bounds) every checked gather/scatter index of the kernels is

@@ -1698,6 +1698,15 @@ int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long lo
   }
 }
 
+int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric) {
+  if (!KE || !blocks || !symmetric) {
+    set_global_error("topo_debug_class_blocks: null pointer");
+    return -1;
+  }
+  *symmetric = pt_class_blocks(KE, blocks) ? 1 : 0;
+  return 0;
+}
+
 int topo_debug_tc_wait(int skip_first_arrival, int poll_limit) {
   xs_debug(skip_first_arrival, poll_limit);
   return 0;

@@ -243,6 +243,7 @@ void level0_apply_cc(bool f64, const Grid& g, const void* u, const void* E, cons
                      const EpiArgs& ea, int* err, cudaStream_t s);
 // level-0 K.u in parity form (kmatvec_pt.cu): KE with the cube's mirror symmetry
 void pt_prepare(const double* KE_host);
+bool pt_class_blocks(const double* KE, double* K);  // host only: the 72 block entries; whether KE has the symmetry
 bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u);
 long long pt_dot_blocks(const Grid& g, bool f64, int nsm);  // CTAs of the StoreDot form (0: no layout)
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,

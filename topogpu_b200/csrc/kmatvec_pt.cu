@@ -522,30 +522,49 @@ PtDevice& pt_device() {
 }
 
 // Class blocks of H KE H^T / 64; false when a coupling between classes is
-// above 1e-12 of the largest entry (KE then needs the general kernels).
+// above 1e-12 of the largest entry (KE then needs the general kernels). H is the
+// product of three butterflies; the sums are carried in 64 bits of mantissa, so
+// that a block's entry is KE's to one rounding (sums in double left up to 3.4
+// ulp, which took K.u's error on a small mesh from 1.8e-16 to 4.2e-16).
 bool class_blocks(const double* KE, double* K) {
   static const int corner[8][3] = {{0, 0, 0}, {1, 0, 0}, {1, 1, 0}, {0, 1, 0}, {0, 0, 1}, {1, 0, 1}, {1, 1, 1}, {0, 1, 1}};
-  auto h = [&](int p, int a) {  // basis function of parity p = 4 px + 2 py + pz at corner a
-    int s = 1;
-    for (int d = 0; d < 3; ++d)
-      if (((p >> (2 - d)) & 1) && !corner[a][d]) s = -s;
-    return s;
-  };
   static const int e[3] = {4, 2, 1};
   double top = 0.0, cross = 0.0;
   for (int c = 0; c < 3; ++c)
-    for (int d = 0; d < 3; ++d)
+    for (int d = 0; d < 3; ++d) {
+      long double M[8][8];  // rows and columns by corner 4 x + 2 y + z, then by parity
+      for (int a = 0; a < 8; ++a)
+        for (int b = 0; b < 8; ++b)
+          M[4 * corner[a][0] + 2 * corner[a][1] + corner[a][2]][4 * corner[b][0] + 2 * corner[b][1] + corner[b][2]] =
+              KE[(3 * a + c) * 24 + 3 * b + d];
+      for (int bit = 1; bit < 8; bit *= 2)
+        for (int i = 0; i < 8; ++i) {
+          if (i & bit) continue;
+          for (int j = 0; j < 8; ++j) {  // rows
+            const long double lo = M[i][j], hi = M[i | bit][j];
+            M[i][j] = lo + hi;
+            M[i | bit][j] = hi - lo;
+          }
+        }
+      for (int bit = 1; bit < 8; bit *= 2)
+        for (int j = 0; j < 8; ++j) {
+          if (j & bit) continue;
+          for (int i = 0; i < 8; ++i) {  // columns
+            const long double lo = M[i][j], hi = M[i][j | bit];
+            M[i][j] = lo + hi;
+            M[i][j | bit] = hi - lo;
+          }
+        }
       for (int p = 0; p < 8; ++p)
         for (int r = 0; r < 8; ++r) {
-          double v = 0.0;
-          for (int a = 0; a < 8; ++a)
-            for (int b = 0; b < 8; ++b) v += h(p, a) * h(r, b) * KE[(3 * a + c) * 24 + 3 * b + d];
-          v /= 64.0;
+          const double v = (double)(M[p][r] / 64.0L);
+          if (!std::isfinite(v)) return false;
           top = std::max(top, std::fabs(v));
           if ((p ^ e[c]) == (r ^ e[d])) K[(p ^ e[c]) * 9 + 3 * c + d] = v;
           else cross = std::max(cross, std::fabs(v));
         }
-  return std::isfinite(top) && cross <= 1e-12 * top;
+    }
+  return cross <= 1e-12 * top;
 }
 
 // Kernel widths: the (warps per CTA, CTAs per SM) pairs an instance is
@@ -680,7 +699,7 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
 }  // namespace
 
 void pt_prepare(const double* KE) {
-  double K[72], Kf[72], Kb[72], KEf[576], KEb[576];
+  double K[72] = {}, Kf[72] = {}, Kb[72] = {}, KEf[576], KEb[576];
   double2 d64[36];
   float2 f[36], fb[36];
   for (int i = 0; i < 576; ++i) {
@@ -758,6 +777,8 @@ void level0_columns_pt(const Grid& g, const double* const* U, const double* E, c
   EpiArgs ea{};
   launch_pt<double, double, false, Epi::Store>(g, nullptr, E, mask, nullptr, ea, s, nv, 0, (const void* const*)U, (void* const*)Y);
 }
+
+bool pt_class_blocks(const double* KE, double* K) { return class_blocks(KE, K); }
 
 TOPO_BOUNDS_READER(bounds_flag_pt)
 
