@@ -79,3 +79,23 @@ def test_calls_alternate_between_streams():
         for i, (a, b) in enumerate(zip(got, want)):
             assert torch.equal(a, b), (turn, i)
     s.close()
+
+
+def test_a_captured_call_leaves_the_order_of_the_others():
+    s = _solver()
+    ctx = s.ctx
+    rho, _, _, r, _ = _inputs(s)
+    E = ctx.modulus(rho, 3.0, 1.0, 1e-9)
+    y0 = ctx.matvec(r, E)
+    ctx.gmg_setup(E)  # the last call before the capture ran on the context's stream
+    op0 = ctx.level_operator(1)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        op = ctx.level_operator(1)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        y = ctx.matvec(r, E)  # waits for the set-up, not for the captured copy
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, y0) and torch.equal(op, op0)
+    s.close()

@@ -223,7 +223,7 @@ struct topo_ctx {
   // for a new one, its id does not) and the event behind that call's work: a
   // call on another stream waits for it (has_last: there is such a call)
   unsigned long long last = 0;
-  cudaEvent_t ev_last = nullptr, ev_dir = nullptr;
+  cudaEvent_t ev_last = nullptr, ev_dir = nullptr, ev_cap = nullptr;
   bool has_last = false;
   cudaEvent_t ev_ph[6] = {};     // setup phase marks (timed)
   double setup_ms[5] = {0, 0, 0, 0, 0};
@@ -267,7 +267,8 @@ struct topo_ctx {
 namespace {
 
 // A stream under capture: its events must not be waited for outside the graph,
-// so such a call leaves the bookkeeping of the last call alone.
+// so such a call leaves the bookkeeping of the last call alone and ends on an
+// event of its own (ev_out may be the one the next call waits for).
 bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
@@ -292,7 +293,8 @@ struct StreamGuard {
     TOPO_CUDA_CHECK(cudaStreamWaitEvent(c->cs, c->ev_in, 0));
   }
   ~StreamGuard() {
-    if (cudaEventRecord(c->ev_out, c->cs) == cudaSuccess) cudaStreamWaitEvent(user, c->ev_out, 0);
+    const cudaEvent_t out = cap ? c->ev_cap : c->ev_out;
+    if (cudaEventRecord(out, c->cs) == cudaSuccess) cudaStreamWaitEvent(user, out, 0);
     if (!cap) {
       c->last = id;
       c->ev_last = c->ev_out;
@@ -1362,6 +1364,7 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_dir, cudaEventDisableTiming));
+    TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->ev_cap, cudaEventDisableTiming));
     for (auto& e : c->ev_ph) TOPO_CUDA_CHECK(cudaEventCreate(&e));
     TOPO_CUDA_CHECK(cudaStreamCreateWithFlags(&c->C.bg_stream, cudaStreamNonBlocking));
     TOPO_CUDA_CHECK(cudaEventCreateWithFlags(&c->C.ev_copy, cudaEventDisableTiming));
@@ -1464,6 +1467,7 @@ int topo_ctx_destroy(topo_ctx* c) {
   if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->ev_out) cudaEventDestroy(c->ev_out);
   if (c->ev_dir) cudaEventDestroy(c->ev_dir);
+  if (c->ev_cap) cudaEventDestroy(c->ev_cap);
   for (auto& e : c->ev_ph)
     if (e) cudaEventDestroy(e);
   if (c->cs) cudaStreamDestroy(c->cs);
