@@ -213,7 +213,7 @@ __device__ __forceinline__ void epilogue_store(const EpiDev<T>& e, long long i, 
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
                   Epi epi, const EpiArgs& ea, cudaStream_t s, bool parity = true, int nv = 1, long long vs = 0);
 // nv > 1: that many columns, every vector of column v starting v * vs entries on
-// (vs a multiple of 4); epilogues Store, ChebR, RUpd.
+// (vs a multiple of 4); epilogues ChebR and RUpd.
 // BF16-input operator (u stored BF16 or FP32, rounded); tc: the tensor-core
 // kernel may be used where the parity form does not apply. parity = false:
 // the general kernels only (same results to the last bit of rounding order)

@@ -687,13 +687,14 @@ void launch_pt(const Grid& g, const void* u, const void* E, const uint8_t* mask,
       default: launch_pt_w<T, TU, BF, EPI, 2, C>(L, P, s); break;
     }
   };
-  if constexpr (EPI == Epi::Store || EPI == Epi::ChebR || EPI == Epi::RUpd) {
+  // several columns: the V-cycle's two epilogues, and the block solve's FP64 product
+  if constexpr (sizeof(TU) != 2 && (EPI == Epi::ChebR || EPI == Epi::RUpd || (EPI == Epi::Store && sizeof(T) == 8))) {
     if (nv > 1 || ul) {
       go(std::true_type{});
       return;
     }
   }
-  if (nv > 1) throw std::runtime_error("level0 K.u: this epilogue takes one column");
+  if (nv > 1 || ul) throw std::runtime_error("level0 K.u: this form takes one column");
   go(std::false_type{});
 }
 }  // namespace
@@ -746,7 +747,8 @@ long long pt_dot_blocks(const Grid& g, bool f64, int nsm) {
 
 // f64: FP64 throughout; else FP32 vectors with u FP32 (bf: rounded to BF16
 // where it is read) or stored BF16 (u_bf16). Epilogues as level0_apply. nv
-// columns vs entries apart (u of each 16-byte aligned; one for StoreDot).
+// columns vs entries apart (u of each 16-byte aligned; ChebR and RUpd, u not
+// stored BF16).
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
                      Epi epi, const EpiArgs& ea, cudaStream_t s, int nv, long long vs) {
 #define TOPO_PT_CASE(EP)                                                                                     \
