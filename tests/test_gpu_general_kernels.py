@@ -2,7 +2,8 @@
 the cube's mirror symmetry (tensor-core and CUDA-core streaming kernels, the block
 solve's brick kernel, columns one after another) and z extents beyond its windows.
 Every epilogue against a dense sum over the elements, whole solves by their residual
-under that sum, and the tensor-core kernel's bounded wait. In child processes: the contexts of a device
+under that sum, the tensor-core kernel's bounded wait, and a stiffness that changes
+from context to context on one device. In child processes: the contexts of a device
 share one stiffness, and no other context may be open when it changes.
 
 Tolerances: FP64 sums of a few hundred terms to 1e-13, FP32 to 2e-6, BF16 inputs with
@@ -137,7 +138,22 @@ c.ctx.wait_status()
 c.ctx.close()
 """
 
-@pytest.mark.parametrize("name", ["EPILOGUES", "SOLVES", "LONG_Z", "WAIT"])
+CHANGES = COMMON + r"""
+def product(KE):
+    c = Case((24, 12, 6), KE)
+    u = c.vec(True).astype(np.float64)
+    y = c.ctx.matvec(t(u, torch.float64), t(c.E, torch.float64))
+    assert rel(y, c.K(u)) < 1e-13
+    c.ctx.close()
+    return y
+G = general_stiffness()
+a, b = product(KE_UNIT), product(G)
+for _ in range(2):
+    assert torch.equal(product(KE_UNIT), a) and torch.equal(product(KE_UNIT), a) and torch.equal(product(G), b)
+"""
+
+
+@pytest.mark.parametrize("name", ["EPILOGUES", "SOLVES", "LONG_Z", "WAIT", "CHANGES"])
 def test_general_kernels(cuda_dev, name):
     env = {**os.environ, "PYTHONPATH": os.pathsep.join([str(ROOT), str(ROOT / "tests")])}
     r = subprocess.run([sys.executable, "-c", globals()[name] + "\nprint('all ok')"], cwd=ROOT, env=env, capture_output=True,

@@ -1288,7 +1288,8 @@ extern "C" {
 // uploads it; later contexts must use the same KE to 1e-12 relative (a
 // different one is refused, since it would silently change the operator of
 // the others; one equal up to rounding uses the uploaded copy) and do not
-// write it again while kernels of other contexts may be reading it.
+// write it again while kernels of other contexts may be reading it. With no
+// live context, a KE equal to the uploaded one to the bit is not uploaded again.
 namespace {
 struct DeviceKE {
   std::vector<double> ke;
@@ -1314,7 +1315,8 @@ static void register_ke(topo_ctx* c, const double* KE) {
       throw std::invalid_argument(
           "topo_ctx_create: another live context on this device uses a different element stiffness KE "
           "(KE is held in constant memory shared by all contexts of a device)");
-  } else {
+  } else if (d.ke.size() != 576 || std::memcmp(d.ke.data(), KE, 576 * sizeof(double)) != 0) {
+    d.ke.clear();  // (until every copy is there)
     set_ke(KE);
     cc_set_ke(KE);
     set_ke_block(KE);
@@ -1323,6 +1325,8 @@ static void register_ke(topo_ctx* c, const double* KE) {
     set_galerkin_q(Q.data());
     xs_prepare(KE);
     pt_prepare(KE);
+    // a copy from pageable memory may return before it has reached the device
+    TOPO_CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy));
     d.ke.assign(KE, KE + 576);
   }
   d.live += 1;
