@@ -71,7 +71,7 @@ def epilogues(c, dt, tol, u, ud, KE, **kw):
     r, x, d = t(r0, dt), t(x0, dt), t(0 * x0, dt)
     c.ctx.level0_apply(u, E, "cheb", r=r, x=x, d_out=d, dinv=t(dinv, dt), s=0.7, c1=0.3, c2=1.1, ax=0.9, **kw)
     rr = (r0 - 0.7 * w) * m
-    dd = (0.3 * ud + 1.1 * dinv * rr) * m
+    dd = (0.3 * ud + 1.1 * dinv.astype(np.float64) * rr) * m  # (a float times a float32 array would round to float32)
     assert rel(r, rr) < tol and rel(d, dd) < tol and rel(x, x0 + 0.9 * dd) < tol
 
 def solves(c, tol=1e-6):
