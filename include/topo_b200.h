@@ -157,6 +157,10 @@ int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long lo
  * whether KE has the mirror symmetry that the form needs. */
 int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric);
 
+/* Test query: r[i] = 1 / d[i] (n values in device memory, d in (1e-290, 1e290))
+ * with the reciprocal that the coarsest factorisation takes of its pivots. */
+int topo_debug_recip(long long n, const double* d, double* r, void* stream);
+
 /* Index range checks (no reference counterpart). In the library built with
  * -DTOPO_DEBUG_BOUNDS (libtopo_b200_dbg.so: python -m topogpu_b200.build
  * --debug-bounds) every checked gather/scatter index of the kernels is

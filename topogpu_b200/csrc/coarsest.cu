@@ -160,6 +160,25 @@ __device__ __forceinline__ void tile_of(int t, int& ti, int& tj) {
   tj = t - ti * (ti + 1) / 2;
 }
 
+// 1/d for d in (1e-290, 1e290), where nothing on the way leaves the normal
+// numbers: the start r of the PTX instruction rcp.approx.ftz.f64 (its result has
+// 20 fraction bits, formed from d's first 20: |e| <= 2^-19 for e = 1 - d r) and
+// one step of the hyperpower iteration of order three, r (1 + e + e^2) (Altman,
+// Pacific J. Math. 10, 1960), whose error is e^3 <= 2^-57. With the roundings
+// of the last two operations that is within one unit in the last place of 1/d,
+// which the tests check against the division over the range.
+__device__ __forceinline__ double hyper_recip(double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double e = fma(-d, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+__global__ void k_recip(long long n, const double* __restrict__ d, double* __restrict__ r) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    r[i] = hyper_recip(d[i]);
+}
+
 // Two pivots of the warp-register factor of a 32x32 diagonal block (lane =
 // row). The pivot index is a template parameter so that every register index
 // is a compile-time constant (the array stays in registers). Columns J and J+1
@@ -168,9 +187,7 @@ __device__ __forceinline__ void tile_of(int t, int& ti, int& tj) {
 // and free of branches: the second pivot q1 = d1 - l^2 / d0 is inverted as
 // d0 / (d0 d1 - l^2), with the determinant as a difference of products that
 // keeps its relative accuracy (Kahan: the rounding of l^2 is taken out again),
-// so both reciprocals run side by side. A reciprocal is the hardware's
-// approximation r (2^-23) and one third-order step r (1 + e + e^2),
-// e = 1 - d r, which cubes the error. The square roots of all pivots follow
+// so both reciprocals run side by side. The square roots of all pivots follow
 // once at the end. Entries right of a lane's diagonal are updated too but never
 // read.
 template <int J>
@@ -183,12 +200,8 @@ __device__ __forceinline__ void chol_step(double (&wr)[CNB], int lane, CholSmem&
   const double ll = l * l, det = fma(d0, d1, -ll) - fma(l, l, -ll);
   double e0 = d0, e1, r0, r1, t;
   if (d0 > 1e-290 && d0 < 1e290 && det > 1e-290 && det < 1e290) {
-    double ra, rb;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(d0));
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(rb) : "d"(det));
-    const double ea = fma(-d0, ra, 1.0), eb = fma(-det, rb, 1.0);
-    r0 = fma(ra, fma(ea, ea, ea), ra);
-    r1 = d0 * fma(rb, fma(eb, eb, eb), rb);
+    r0 = hyper_recip(d0);
+    r1 = d0 * hyper_recip(det);
     t = l * r0;
     e1 = det * r0;
   } else {  // a pivot that is not positive, or out of range (it is then taken as 1)
@@ -931,6 +944,11 @@ void coarsest_alloc(CoarsestFactor& f, const CoarsestPlan& p, int band, bool f64
   TOPO_CUDA_CHECK(cudaFuncSetAttribute(cst::k_tri_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(cst::TriSmem)));
   f.plan = p;
+}
+
+void pivot_recip(long long n, const double* d, double* r, cudaStream_t s) {
+  cst::k_recip<<<(unsigned)std::min<long long>((n + 255) / 256, 1184), 256, 0, s>>>(n, d, r);
+  TOPO_LAUNCH_CHECK();
 }
 
 void coarsest_assemble(CoarsestFactor& f, const Grid& g, const double* S, const int* dof_index, cudaStream_t s) {

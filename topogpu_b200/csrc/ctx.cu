@@ -1715,6 +1715,18 @@ int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric) {
   return 0;
 }
 
+int topo_debug_recip(long long n, const double* d, double* r, void* stream) {
+  try {
+    if (!d || !r) throw std::invalid_argument("topo_debug_recip: null pointer");
+    if (n < 1) throw std::invalid_argument("topo_debug_recip: n must be >= 1");
+    pivot_recip(n, d, r, (cudaStream_t)stream);
+    return 0;
+  } catch (const std::exception& e) {
+    set_global_error(e.what());
+    return -1;
+  }
+}
+
 int topo_debug_tc_wait(int skip_first_arrival, int poll_limit) {
   xs_debug(skip_first_arrival, poll_limit);
   return 0;

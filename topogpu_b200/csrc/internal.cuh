@@ -337,6 +337,7 @@ struct CoarsestFactor {
 CoarsestPlan coarsest_plan(const Grid& g, const std::vector<int>& free_list);
 void coarsest_alloc(CoarsestFactor& f, const CoarsestPlan& p, int band, bool f64, void* (*alloc_bytes)(void*, size_t),
                     void* ctx);
+void pivot_recip(long long n, const double* d, double* r, cudaStream_t s);  // the factor's reciprocal, for its test
 void coarsest_assemble(CoarsestFactor& f, const Grid& g, const double* S, const int* dof_index, cudaStream_t s);
 void coarsest_regularise(CoarsestFactor& f, double* dtmp, cudaStream_t s);
 void coarsest_factor(CoarsestFactor& f, cudaStream_t s);
