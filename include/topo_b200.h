@@ -151,6 +151,12 @@ int topo_debug_tc_wait(int skip_first_arrival, int poll_limit);
  * on a GPU of nsm SMs, and the partial sums a context of the mesh has room for. */
 int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long long* blocks, long long* room);
 
+/* Test query (host only): the kernel that runs the level-0 operator of a mesh with
+ * a mirror-symmetric KE, 16-byte aligned vectors and tensor cores on: 0 parity
+ * form, 1 tcgen05 streaming, 2 CUDA-core streaming, 3 brick. u_dtype and epi as
+ * topo_level0_apply (3: with the dot product), nsm the SM count. */
+int topo_debug_route(int nelx, int nely, int nelz, int u_dtype, int epi, int nsm, int* kernel);
+
 /* Test query (host only): the eight 3x3 parity-class blocks (72 doubles, entry
  * (c, d) of class q at 9 q + 3 c + d, q = 4 qx + 2 qy + qz) of the element
  * stiffness KE (host, 576 doubles) as the parity form of K.u uses them, and

@@ -40,6 +40,7 @@ SIGNATURES = {
     "topo_wait_status": (_i, [_vp, _vp]),
     "topo_debug_tc_wait": (_i, [_i, _i]),
     "topo_debug_reduction": (_i, [_i, _i, _i, _i, _i, C.POINTER(_ll), C.POINTER(_ll)]),
+    "topo_debug_route": (_i, [_i, _i, _i, _i, _i, _i, C.POINTER(_i)]),
     "topo_debug_class_blocks": (_i, [_vp, _vp, C.POINTER(_i)]),
     "topo_debug_recip": (_i, [_ll, _vp, _vp, _vp]),
     "topo_debug_bounds": (_i, [C.POINTER(_i)]),

@@ -1076,7 +1076,7 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
   };
   // Y = K U: one launch for all columns where the parity form applies
   auto apply = [&](double* const* U, double* const* Y, int k) {
-    if (level0_pt_supported(L0.g, true, false, c->blk))
+    if (level0_pt_takes(L0.g, true, false, c->blk, Epi::Store, level0_general(Prec::F64, false, L0.g)))
       level0_columns_pt(L0.g, (const double* const*)U, c->E64, L0.mask, Y, k, s);
     else
       level0_apply_block(L0.g, (const double* const*)U, c->E64, L0.mask, Y, k, s);
@@ -1699,6 +1699,23 @@ int topo_debug_reduction(int nelx, int nely, int nelz, int f64, int nsm, long lo
     const Grid g = make_grid(nelx, nely, nelz);
     *blocks = level0_dot_blocks(g, f64 != 0, nsm);
     *room = reduction_room(g, nsm);
+    return 0;
+  } catch (const std::exception& e) {
+    set_global_error(e.what());
+    return -1;
+  }
+}
+
+int topo_debug_route(int nelx, int nely, int nelz, int u_dtype, int epi, int nsm, int* kernel) {
+  try {
+    if (!kernel) throw std::invalid_argument("topo_debug_route: null pointer");
+    if (nelx < 1 || nely < 1 || nelz < 1 || nsm < 1) throw std::invalid_argument("topo_debug_route: sizes must be >= 1");
+    if (u_dtype < TOPO_F64 || u_dtype > TOPO_BF16_F32IN || epi < TOPO_EPI_STORE || epi > TOPO_EPI_RUPD)
+      throw std::invalid_argument("topo_debug_route: bad dtype or epilogue");
+    const Grid g = make_grid(nelx, nely, nelz);
+    const Prec p = u_dtype == TOPO_F64 ? Prec::F64 : u_dtype == TOPO_F32 ? Prec::F32 : Prec::BF16;
+    const Level0Kernel other = level0_general(p, true, g);
+    *kernel = (int)(pt_pays(g, p == Prec::F64, (Epi)epi, nsm, other) ? Level0Kernel::Parity : other);
     return 0;
   } catch (const std::exception& e) {
     set_global_error(e.what());

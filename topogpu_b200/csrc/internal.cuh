@@ -244,7 +244,13 @@ void level0_apply_cc(bool f64, const Grid& g, const void* u, const void* E, cons
 // level-0 K.u in parity form (kmatvec_pt.cu): KE with the cube's mirror symmetry
 void pt_prepare(const double* KE_host);
 bool pt_class_blocks(const double* KE, double* K);  // host only: the 72 block entries; whether KE has the symmetry
-bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u);
+// the kernels of the level-0 operator: parity form, tcgen05 streaming, CUDA-core
+// streaming, brick
+enum class Level0Kernel : int { Parity = 0, Tensor = 1, Stream = 2, Brick = 3 };
+// other: the kernel that runs where the parity form does not
+bool level0_pt_takes(const Grid& g, bool f64, bool bf, const void* u, Epi epi, Level0Kernel other);
+bool pt_pays(const Grid& g, bool f64, Epi epi, int nsm, Level0Kernel other);
+Level0Kernel level0_general(Prec p, bool tc, const Grid& g);
 long long pt_dot_blocks(const Grid& g, bool f64, int nsm);  // CTAs of the StoreDot form (0: no layout)
 void level0_apply_pt(bool f64, bool bf, bool u_bf16, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y,
                      Epi epi, const EpiArgs& ea, cudaStream_t s, int nv = 1, long long vs = 0);

@@ -583,6 +583,7 @@ constexpr int kPtSmem = 200 * 1024;  // dynamic shared memory of one CTA at most
 
 struct PtLayout {
   int w, TO, nwin, nseg, ctas, slot, off_pw, pw_n, off_bar, total;
+  double cost;  // layers times warps per SM
 };
 
 // Window width and segments. A CTA of NW warps yields 31 NW - NZ nodes per
@@ -591,7 +592,7 @@ struct PtLayout {
 // times the warps that share its SM (at least 8: below that a step is
 // latency and costs the same), over the waves of CTAs. A width that spends more
 // than 3/4 of its elements on the halo is left out; with none left (NZ above
-// 372, in FP64 186) the general kernels take the mesh.
+// 372, in FP64 186) the general kernels take the mesh, and where pt_pays says so.
 template <typename T, Epi EPI>
 bool pt_layout(const Grid& g, int s_u, bool cols, int nv, int nsm, PtLayout& best) {
   const bool line = cols && pt::line_split<T, EPI>;
@@ -628,7 +629,7 @@ bool pt_layout(const Grid& g, int s_u, bool cols, int nv, int nsm, PtLayout& bes
     L.off_bar = L.off_pw + al(4LL * L.pw_n * (int)sizeof(T));
     L.total = L.off_bar + 128;
     if (L.total <= kPtSmem / Width<T, EPI>::PER[w] && c < cost) {
-      cost = c;
+      cost = L.cost = c;
       best = L;
     }
   }
@@ -730,13 +731,46 @@ void pt_prepare(const double* KE) {
   d.symbf = sbf;
 }
 
+// Whether the parity form is the faster one. Its time follows pt_layout's cost c
+// (B200: FP32 Store 2 us + 0.074 c, FP64 Store 5 + 0.10 c, FP64 Chebyshev step
+// 3.5 + 0.168 c), which counts halo rows, the extra layer of a segment, idle SMs
+// and last waves with the elements: 1.5 to 2 times the elements' own share n =
+// nodes / (31 SMs) on ordinary meshes, 3 to 6 times where a window is little
+// more than its halo row or barely more windows than SMs make a second wave. The
+// general kernels do not pay for that. Measured with z extents from 60 to 371 at
+// 60,000 and a million elements (n = 14, 225), times of the parity form against
+// the other: brick kernel, FP64 Chebyshev step 114 against 115 us at c = 2.9 n,
+// 207 against 123 at 5.9 n, 14.7 against 14.7 at c = 64 (n = 14), 16.8 against
+// 14.6 at 80; FP32 step 62 against 62 at 3.0 n, 110 against 62 at 5.9 n.
+// CUDA-core streaming kernel: 39 against 95 us at 1.5 n (FP64), 29 against 64 at
+// 1.6 n (FP32), and 15 to 43 us on the small meshes against 8 to 13. Tensor-core
+// kernel, whose time goes with rows and z padded to 16: plain product 37 against
+// 39 us at c = 1.65 of the padded n, 37 against 35 at 1.8; Chebyshev step 47
+// against 60 at 1.8.
+bool pt_pays(const Grid& g, bool f64, Epi epi, int nsm, Level0Kernel other) {
+  PtLayout L, narrow;
+  const bool cheb = epi == Epi::ChebR;
+  if (!(f64 ? pt_layout<double, Epi::ChebR>(g, 8, false, 1, nsm, narrow) : pt_layout<float, Epi::ChebR>(g, 4, false, 1, nsm, narrow)))
+    return false;
+  if (!f64 || cheb) L = narrow;  // (FP32: the same widths)
+  else if (!pt_layout<double, Epi::Store>(g, 8, false, 1, nsm, L)) return false;
+  const double n = (double)g.nnodes / (31.0 * nsm);
+  switch (other) {
+    case Level0Kernel::Stream: return L.cost <= 80.0 + 3.2 * n;
+    case Level0Kernel::Tensor: {
+      const double padded = n * ((g.NY + 15) / 16 * 16) / g.NY * ((g.NZ + 15) / 16 * 16) / g.NZ;
+      return L.cost <= 48.0 + (epi == Epi::Store || epi == Epi::Residual ? 1.55 : 2.0) * padded;
+    }
+    default: return L.cost <= 30.0 + 2.95 * n;
+  }
+}
+
 // The parity form takes this operator: the element stiffness has the mirror
-// symmetry, the mesh a window layout, and the copies' 16-byte alignment holds.
-bool level0_pt_supported(const Grid& g, bool f64, bool bf, const void* u) {
+// symmetry, the mesh a window layout, the copies' 16-byte alignment holds, and
+// the kernel that would run instead is the slower one.
+bool level0_pt_takes(const Grid& g, bool f64, bool bf, const void* u, Epi epi, Level0Kernel other) {
   const PtDevice& d = pt_device();
-  PtLayout L;
-  return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 &&
-         (f64 ? pt_layout<double, Epi::ChebR>(g, 8, false, 1, d.nsm, L) : pt_layout<float, Epi::ChebR>(g, 4, false, 1, d.nsm, L));  // (the narrowest)
+  return (bf ? d.symbf : f64 ? d.sym64 : d.sym32) && ((uintptr_t)u & 15) == 0 && pt_pays(g, f64, epi, d.nsm, other);
 }
 
 long long pt_dot_blocks(const Grid& g, bool f64, int nsm) {

@@ -271,13 +271,18 @@ struct ColumnAt {
   }
 };
 
+Level0Kernel level0_general(Prec p, bool tc, const Grid& g) {
+  if (p == Prec::BF16) return tc && level0_xs_supported(g) ? Level0Kernel::Tensor : Level0Kernel::Brick;
+  return level0_cc_supported(g, p == Prec::F64) ? Level0Kernel::Stream : Level0Kernel::Brick;
+}
+
 void level0_apply(Prec p, const Grid& g, const void* u, const void* E, const uint8_t* mask, void* y, Epi epi,
                   const EpiArgs& ea, cudaStream_t s, bool parity, int nv, long long vs) {
-  // The parity form (kmatvec_pt.cu) takes every mesh with a window layout when
-  // KE has the cube's mirror symmetry. Without it FP64 / FP32 run the
-  // x-streaming kernel (kmatvec_cc.cu) when its planes fit in shared memory;
-  // the brick kernel below otherwise and for the BF16 emulation.
-  if (parity && level0_pt_supported(g, p == Prec::F64, p == Prec::BF16, u)) {
+  // The parity form (kmatvec_pt.cu) runs where KE has the cube's mirror symmetry
+  // and the mesh suits its windows. Elsewhere FP64 / FP32 run the x-streaming
+  // kernel (kmatvec_cc.cu) when its planes fit in shared memory; the brick kernel
+  // below otherwise and for the BF16 emulation.
+  if (parity && level0_pt_takes(g, p == Prec::F64, p == Prec::BF16, u, epi, level0_general(p, false, g))) {
     level0_apply_pt(p == Prec::F64, p == Prec::BF16, false, g, u, E, mask, y, epi, ea, s, nv, vs);
     return;
   }
@@ -309,7 +314,7 @@ void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const
                        long long vs) {
   if (tc && level0_xs_supported(g)) {
     level0_xs_check(u, E, nmask, ea);
-    if (parity && level0_pt_supported(g, false, true, u)) {
+    if (parity && level0_pt_takes(g, false, true, u, epi, Level0Kernel::Tensor)) {
       level0_apply_pt(false, true, u_bf16, g, u, E, mask, y, epi, ea, s, nv, vs);
     } else {
       for (int v = 0; v < nv; ++v) {  // (columns are FP32)
@@ -321,7 +326,7 @@ void level0_apply_bf16(bool tc, bool u_bf16, const Grid& g, const void* u, const
     level0_apply(Prec::BF16, g, u, E, mask, y, epi, ea, s, parity, nv, vs);
   } else {
     if (epi != Epi::Store) throw std::runtime_error("topo_level0_apply: BF16-stored u on CUDA cores supports Store only");
-    if (parity && level0_pt_supported(g, false, true, u)) level0_apply_pt(false, true, true, g, u, E, mask, y, epi, ea, s);
+    if (parity && level0_pt_takes(g, false, true, u, epi, Level0Kernel::Brick)) level0_apply_pt(false, true, true, g, u, E, mask, y, epi, ea, s);
     else launch_level0<float, __nv_bfloat16, true>(g, u, E, mask, y, epi, ea, s);
   }
 }
