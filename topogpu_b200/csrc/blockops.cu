@@ -2,8 +2,8 @@
 // one density field).
 //
 //   * k_level0_block: Y_v = K(E) U_v for v < nv in one launch, for the
-//     stiffnesses and meshes the parity form (kmatvec_pt.cu, 62 us for eight
-//     columns of 96x48x48 against 221 us here) does not take. A CTA stages
+//     stiffnesses and meshes the parity form (kmatvec_pt.cu, 64 us for eight
+//     columns of 96x48x48 against 229 us here) does not take. A CTA stages
 //     its brick of moduli once and reuses it for every vector (KE sits in
 //     constant memory), so E is read once per launch instead of once per
 //     load case.

@@ -37,9 +37,9 @@
 // flag, the copies in flight are drained (bounded) and the CTA exits.
 //
 // Bound: issue slots and the barrier per plane (about 280 instructions per
-// element and step; 20% of the elements are halo), not HBM: FP32 Store moves
-// 26 MB at 160x80x80 (4 us at the copy rate), ChebR 93 MB (14 us). Measured on
-// a B200, rotating buffers, against the kernels it replaced there (kernel
+// element and step; 20% of the elements are halo), not HBM: at 160x80x80 FP32
+// Store moves 29.4 MB (4.5 us at the copy rate), ChebR 92.8 MB (14 us), each and
+// 3.2 MB of mask. Measured on a B200, rotating buffers, against the kernels it replaced there (kernel
 // times): 160x80x80 FP32 Store 24.5 us (64), FP64 Store 37.9 us (130), ChebR
 // with BF16 rounding 35.3 us (67, tensor cores), FP32 ChebR 35.0 us, FP32 RUpd
 // 27.7 us (64); 24x12x6 FP64 4.4 us (9.6). The tensor-core form of the same operator does
