@@ -88,6 +88,9 @@ int topo_set_cycle(topo_ctx* ctx, int gamma);
 int topo_last_error(topo_ctx* ctx, char* buf, int len);
 
 /* Free mask (uint8 per DoF, 1 = free) and load vector F (FP64, all DoFs).
+ * Supports that change the number of the coarsest level's free DoFs, or their
+ * band, replace its buffers: capture a CUDA graph that holds a V-cycle of this
+ * context (topo_gmg_apply) again after such a change.
  * Replaces the free/F upload of GPUFEMSolver._upload_cupy (src/gpu_fem/fem_gpu.py:361-379). */
 int topo_set_problem(topo_ctx* ctx, const uint8_t* free_mask, const double* F, void* stream);
 
@@ -220,15 +223,16 @@ int topo_set_coarse_lag(topo_ctx* ctx, int on);
 
 /* BF16 level-0 operator, where KE or the mesh does not allow the parity form:
  * on the tensor cores (on != 0, the default) or on the CUDA cores (same BF16
- * inputs and FP32 accumulation, another summation order); a tuning switch with no reference counterpart. */
+ * inputs and FP32 accumulation, another summation order); a tuning switch with
+ * no reference counterpart. */
 int topo_set_tc(topo_ctx* ctx, int on);
 
 /* Block PCG for nrhs load cases (1..8) on the current hierarchy: B and X are
  * nrhs full-length FP64 vectors stored one after another (X holds the
  * initial guesses and receives the solutions). One multi-vector FP64 K.u per
- * iteration (moduli staged once for all columns), the GMG V-cycle on every
- * column, alpha/beta from nrhs x nrhs Gram matrices; columns leave the block
- * once ||r_j|| <= tol ||mask b_j||. out_relres receives nrhs values.
+ * iteration, one V-cycle over all columns, alpha/beta from nrhs x nrhs Gram
+ * matrices; columns leave the block once ||r_j|| <= tol ||mask b_j||.
+ * out_relres receives nrhs values.
  * Returns 0 (all converged), 1 (maxiter reached) or < 0. The reference solves
  * one load case per PCG (_cupy_pcg, src/gpu_fem/solver_v2.py:552-624); this
  * replaces nrhs of those calls. */

@@ -7,10 +7,11 @@ own CUDA stream. The ctypes calls into libtopo_b200.so release the GIL, so the
 kernels of different meshes overlap on the GPU and the host-side polling of
 one solve hides behind the kernels of the others.
 
-``autotune`` picks the worker count and the level-0 operator variant (tcgen05
-or CUDA cores, same BF16 inputs and FP32 accumulation) by timing one round of
-solves per candidate; the choice is cached under the batch's size signature
-and reused by ``solve``.
+``autotune`` picks the worker count and the switch of the level-0 operator's
+general form (``TopoContext.set_tensor_cores``: without effect on meshes that
+the parity form takes, which is every ordinary one) by timing one round of
+solves per candidate; the choice is cached under the batch's size signature and
+reused by ``solve``.
 
 The reference solves one mesh at a time; this is the batched form of its
 SolverV4.solve (src/gpu_fem/solver_v4.py:147-269) for many independent

@@ -128,8 +128,8 @@ class TopoContext:
         """One level-0 operator application with its fused epilogue (see
         topo_level0_apply): "store" y = K u, "residual" y = b - K u, "rupd"
         r -= s K u, "cheb" r -= s K u; d_out = c1 u + c2 dinv r; x += ax d_out.
-        u's dtype picks the arithmetic (f64, f32, bf16); u_fp32_to_bf16 runs
-        an f32 u through the BF16 tensor-core operator (the smoother's form).
+        u's dtype picks the arithmetic (f64, f32, bf16); u_fp32_to_bf16 rounds
+        an f32 u to BF16 where it is read (the smoother's form).
         The other vectors are f64 for an f64 u and f32 otherwise. Returns y
         for "store"/"residual", else None (r, x, d_out are updated)."""
         if epi not in self.EPILOGUES:
@@ -200,7 +200,9 @@ class TopoContext:
         self._chk(self._lib.topo_set_cycle(self._h, 1 if cycle_type == "v" else 2), "set_cycle")
 
     def set_tensor_cores(self, on: bool):
-        """BF16 level-0 K.u on tcgen05 (True) or on the CUDA cores (False)."""
+        """Where the parity form does not take the BF16 level-0 K.u (a KE without
+        the mirror symmetry, z extents that do not suit its windows): tcgen05
+        (True) or the CUDA cores (False)."""
         self._chk(self._lib.topo_set_tc(self._h, int(bool(on))), "set_tc")
 
     def block_pcg(self, B, X, tol=1e-5, maxiter=800):

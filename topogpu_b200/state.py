@@ -126,6 +126,8 @@ class StateSolver:
         return [float(torch.dot(Bm[j], U[j])) for j in range(B.shape[0])], U
 
     # -- diagnostics (GalerkinMatFreeGMG.probe_quality / estimate_kappa_eff) --
+    # In mixed mode a single V-cycle (gmg_apply) runs the general level-0 kernels,
+    # PCG's own the parity form: the same operator, products summed in another order.
     def _precondition(self, r):
         vdt = self.ctx.vec_dtype
         return self.ctx.gmg_apply(r.to(vdt).contiguous()).to(torch.float64)
