@@ -166,6 +166,12 @@ int topo_debug_route(int nelx, int nely, int nelz, int u_dtype, int epi, int nsm
  * whether KE has the mirror symmetry that the form needs. */
 int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric);
 
+/* Test query (host only): doubles of scratch that a context of this mesh (three
+ * levels or more) keeps for R.A.P; test hook: the context's next set-ups use no
+ * more of it than rap_planes (>= 3) planes of level 1, as on a larger mesh. */
+int topo_debug_rap_room(int nelx, int nely, int nelz, long long* doubles);
+int topo_debug_scratch(topo_ctx* ctx, int rap_planes);
+
 /* Test query: r[i] = 1 / d[i] (n values in device memory, d in (1e-290, 1e290))
  * with the reciprocal that the coarsest factorisation takes of its pivots. */
 int topo_debug_recip(long long n, const double* d, double* r, void* stream);

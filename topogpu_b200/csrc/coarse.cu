@@ -147,12 +147,16 @@ struct RapDim {
   long long inner;       // nodes below it (stride of the dimension)
   long long outer;       // nodes above it
   int kstride;           // step of the dimension's offset in k: 9, 3 or 1
+  long long sin, sout;   // nodes between two coefficients of the input / output
+  int i0, ni;            // the output's first node along the dimension and its number of them
+  int f0, nfs;           // the input's
+  long long at;          // node of the first output in the coarse grid (last pass)
 };
 
 template <bool MASK>
 __global__ void __launch_bounds__(256) k_rap_dim(RapDim D, const double* __restrict__ Sin, double* __restrict__ Sout, Grid c,
                                                  const uint8_t* __restrict__ mc) {
-  const long long nin = D.outer * (D.nf + 1) * D.inner, nout = D.outer * (D.nc + 1) * D.inner;
+  const long long nin = D.sin, nout = D.outer * D.ni * D.inner;
   const long long o = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (o >= nout) return;
   const int cq = blockIdx.y;  // (other two offsets) * 9 + coefficient
@@ -160,9 +164,9 @@ __global__ void __launch_bounds__(256) k_rap_dim(RapDim D, const double* __restr
   // k of the middle block (offset 0 along the dimension)
   const int k0 = D.kstride == 1 ? kk * 3 + 1 : D.kstride == 3 ? (kk / 3) * 9 + 3 + kk % 3 : 9 + kk;
   const long long in_ = o % D.inner, t = o / D.inner;
-  const int I = (int)(t % (D.nc + 1));
-  const long long out_ = t / (D.nc + 1);
-  const double* base = Sin + (long long)(k0 * 9 + q) * nin + (out_ * (D.nf + 1) + 2 * I) * D.inner + in_;
+  const int I = D.i0 + (int)(t % D.ni);
+  const long long out_ = t / D.ni;
+  const double* base = Sin + (long long)(k0 * 9 + q) * nin + (out_ * D.nfs + 2 * I - D.f0) * D.inner + in_;
   const long long ks = (long long)D.kstride * 9 * nin;
   const bool h = I + 1 <= D.nc, up = 2 * I + 1 <= D.nf, dn = I >= 1;
   const double a = h ? 0.5 : 1.0;
@@ -192,34 +196,53 @@ __global__ void __launch_bounds__(256) k_rap_dim(RapDim D, const double* __restr
     double v = r[d];
     if (MASK) {  // last pass: rows and columns of fixed DoFs
       int ix, iy, iz;
-      node_xyz(c, o, ix, iy, iz);
+      node_xyz(c, D.at + o, ix, iy, iz);
       const int jx = ix + k / 9 - 1, jy = iy + (k / 3) % 3 - 1, jz = iz + k % 3 - 1;
       const bool jin = jx >= 0 && jx < c.NX && jy >= 0 && jy < c.NY && jz >= 0 && jz < c.NZ;
       const long long J = jin ? ((long long)jx * c.NY + jy) * c.NZ + jz : 0;
-      if (!(jin && mc[3 * o + q / 3] && mc[3 * J + q % 3])) v = 0.0;
+      if (!(jin && mc[3 * (D.at + o) + q / 3] && mc[3 * J + q % 3])) v = 0.0;
     }
-    Sout[(long long)(k * 9 + q) * nout + o] = v;
+    Sout[(long long)(k * 9 + q) * D.sout + o] = v;
   }
 }
 
-// Doubles of scratch the passes need between `fine` and `coarse`.
+// Scratch of the passes: two intermediate operators on some x planes of the
+// fine grid. 2P + 1 planes give P planes of the coarse grid, so the passes run
+// slab by slab where the whole is above kRapScratch, 512 MB (160x80x80 needs 205;
+// about 2.7 million elements reach it): the intermediates are three quarters of
+// level 1's operator, memory that the largest meshes do not have. A slab repeats
+// one fine plane of the one before.
+constexpr long long kRapScratch = 1LL << 26;  // doubles
+static long long rap_plane(const Grid& f, const Grid& c) { return 243LL * (f.NY + c.NY) * c.NZ; }
+
 long long rap_scratch(const Grid& f, const Grid& c) {
-  return 243LL * ((long long)f.NX * f.NY * c.NZ + (long long)f.NX * c.NY * c.NZ);
+  const long long w = rap_plane(f, c);
+  return std::min((long long)f.NX, std::max(3LL, kRapScratch / w)) * w;
 }
 
+// room: doubles of scratch (three planes or the whole, at least)
 void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c, double* scratch,
-         cudaStream_t s) {
+         long long room, cudaStream_t s) {
   const Grid &f = fine, &c = coarse;
-  double* T1 = scratch;
-  double* T2 = scratch + 243LL * f.NX * f.NY * c.NZ;
-  const RapDim dz{f.nz, c.nz, 1, (long long)f.NX * f.NY, 1}, dy{f.ny, c.ny, c.NZ, f.NX, 3}, dx{f.nx, c.nx, (long long)c.NY * c.NZ, 1, 9};
-  auto nb = [](const RapDim& D) { return dim3((unsigned)((D.outer * (D.nc + 1) * D.inner + 255) / 256), 81); };
-  k_rap_dim<false><<<nb(dz), 256, 0, s>>>(dz, S_f, T1, c, mask_c);
-  TOPO_LAUNCH_CHECK();
-  k_rap_dim<false><<<nb(dy), 256, 0, s>>>(dy, T1, T2, c, mask_c);
-  TOPO_LAUNCH_CHECK();
-  k_rap_dim<true><<<nb(dx), 256, 0, s>>>(dx, T2, S_c, c, mask_c);
-  TOPO_LAUNCH_CHECK();
+  const long long fits = room / rap_plane(f, c), inner = (long long)c.NY * c.NZ;
+  const int P = fits >= f.NX ? c.NX : (int)((fits - 1) / 2);
+  if (P < 1) throw std::runtime_error("R.A.P: too little scratch");
+  auto nb = [](const RapDim& D) { return dim3((unsigned)((D.outer * D.ni * D.inner + 255) / 256), 81); };
+  for (int I0 = 0; I0 < c.NX; I0 += P) {
+    const int I1 = std::min(c.NX, I0 + P), f0 = std::max(0, 2 * I0 - 1), np = std::min(f.nx, 2 * I1 - 1) - f0 + 1;
+    const long long n1 = (long long)np * f.NY * c.NZ, n2 = np * inner;
+    double* T1 = scratch;
+    double* T2 = scratch + 243LL * n1;
+    const RapDim dz{f.nz, c.nz, 1, (long long)np * f.NY, 1, f.nnodes, n1, 0, c.NZ, 0, f.NZ, 0},
+        dy{f.ny, c.ny, c.NZ, np, 3, n1, n2, 0, c.NY, 0, f.NY, 0},
+        dx{f.nx, c.nx, inner, 1, 9, n2, c.nnodes, I0, I1 - I0, f0, np, I0 * inner};
+    k_rap_dim<false><<<nb(dz), 256, 0, s>>>(dz, S_f + (long long)f0 * f.NY * f.NZ, T1, c, mask_c);
+    TOPO_LAUNCH_CHECK();
+    k_rap_dim<false><<<nb(dy), 256, 0, s>>>(dy, T1, T2, c, mask_c);
+    TOPO_LAUNCH_CHECK();
+    k_rap_dim<true><<<nb(dx), 256, 0, s>>>(dx, T2, S_c + I0 * inner, c, mask_c);
+    TOPO_LAUNCH_CHECK();
+  }
 }
 
 // ------------------------------------------------------------- stencil apply

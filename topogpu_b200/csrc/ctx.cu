@@ -184,6 +184,7 @@ struct topo_ctx {
   uint8_t* nmask0 = nullptr;  // level 0: per-node free bits, bit c = DoF 3n+c (read by the tensor-core K.u)
   double* diag0 = nullptr;
   double* rap_tmp = nullptr;  // between the passes of R.A.P (sized for levels 1 -> 2, the largest)
+  long long rap_room = 0;     // its doubles
   double lam_Emax = NAN;
   bool problem_set = false;
   bool setup_done = false;
@@ -785,7 +786,7 @@ void do_setup(topo_ctx* c, const double* E, cudaStream_t s) {
   for (int l = 1; l < c->n_levels; ++l) {
     Level& Lv = c->L[l];
     if (l == 1) level1_assemble(c->L[0].g, Lv.g, c->E64, Lv.mask, Lv.S64, s);
-    else rap(c->L[l - 1].g, Lv.g, c->L[l - 1].S64, Lv.mask, Lv.S64, c->rap_tmp, s);
+    else rap(c->L[l - 1].g, Lv.g, c->L[l - 1].S64, Lv.mask, Lv.S64, c->rap_tmp, c->rap_room, s);
   }
   TOPO_CUDA_CHECK(cudaEventRecord(c->ev_ph[2], s));
   TOPO_CUDA_CHECK(cudaEventRecord(c->ev_ph[3], s));
@@ -1413,7 +1414,10 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
     c->E32 = c->alloc<float>(g0.nelem);
     c->nmask0 = c->alloc<uint8_t>(g0.nnodes + 16);
     c->diag0 = c->alloc<double>(g0.ndof);
-    if (n_levels > 2) c->rap_tmp = c->alloc<double>(rap_scratch(c->L[1].g, c->L[2].g));
+    if (n_levels > 2) {
+      c->rap_room = rap_scratch(c->L[1].g, c->L[2].g);
+      c->rap_tmp = c->alloc<double>(c->rap_room);
+    }
     c->kr = c->valloc(g0.ndof);
     c->kz = c->valloc(g0.ndof);
     c->kp = c->valloc(g0.ndof);
@@ -1737,6 +1741,33 @@ int topo_debug_recip(long long n, const double* d, double* r, void* stream) {
     if (!d || !r) throw std::invalid_argument("topo_debug_recip: null pointer");
     if (n < 1) throw std::invalid_argument("topo_debug_recip: n must be >= 1");
     pivot_recip(n, d, r, (cudaStream_t)stream);
+    return 0;
+  } catch (const std::exception& e) {
+    set_global_error(e.what());
+    return -1;
+  }
+}
+
+int topo_debug_scratch(topo_ctx* c, int rap_planes) {
+  try {
+    if (!c) throw std::invalid_argument("topo_debug_scratch: null context");
+    if (rap_planes < 3) throw std::invalid_argument("topo_debug_scratch: at least 3 planes");
+    if (c->n_levels > 2) {
+      const Grid &f = c->L[1].g, &k = c->L[2].g;
+      c->rap_room = std::min(rap_scratch(f, k), 243LL * (f.NY + k.NY) * k.NZ * rap_planes);
+    }
+    return 0;
+  } catch (const std::exception& e) {
+    return fail(c, e);
+  }
+}
+
+int topo_debug_rap_room(int nelx, int nely, int nelz, long long* doubles) {
+  try {
+    if (!doubles) throw std::invalid_argument("topo_debug_rap_room: null pointer");
+    if (nelx < 1 || nely < 1 || nelz < 1) throw std::invalid_argument("topo_debug_rap_room: sizes must be >= 1");
+    auto half = [](int n, int times) { return std::max(1, n >> times); };
+    *doubles = rap_scratch(make_grid(half(nelx, 1), half(nely, 1), half(nelz, 1)), make_grid(half(nelx, 2), half(nely, 2), half(nelz, 2)));
     return 0;
   } catch (const std::exception& e) {
     set_global_error(e.what());

@@ -269,7 +269,7 @@ void level1_assemble(const Grid& fine, const Grid& coarse, const double* E_f, co
                      double* S, cudaStream_t s);
 long long rap_scratch(const Grid& fine, const Grid& coarse);  // doubles
 void rap(const Grid& fine, const Grid& coarse, const double* S_f, const uint8_t* mask_c, double* S_c, double* scratch,
-         cudaStream_t s);
+         long long room, cudaStream_t s);
 void stencil_apply(Prec p, bool vec64, const Grid& g, const void* S, const void* u, const uint8_t* mask,
                    void* y, Epi epi, const EpiArgs& ea, cudaStream_t s, int nv = 1, long long vs = 0);
 void stencil_dinv(const Grid& g, const double* S, const uint8_t* mask, double* dinv64, float* dinv32,
