@@ -172,6 +172,10 @@ int topo_debug_class_blocks(const double* KE, double* blocks, int* symmetric);
 int topo_debug_rap_room(int nelx, int nely, int nelz, long long* doubles);
 int topo_debug_scratch(topo_ctx* ctx, int rap_planes);
 
+/* Test hook: the context's block solves run the V-cycle on at most this many
+ * columns (1..8) at once, as on a device without memory for more. */
+int topo_debug_block_columns(topo_ctx* ctx, int columns);
+
 /* Test query: r[i] = 1 / d[i] (n values in device memory, d in (1e-290, 1e290))
  * with the reciprocal that the coarsest factorisation takes of its pivots. */
 int topo_debug_recip(long long n, const double* d, double* r, void* stream);
@@ -236,10 +240,10 @@ int topo_set_tc(topo_ctx* ctx, int on);
 /* Block PCG for nrhs load cases (1..8) on the current hierarchy: B and X are
  * nrhs full-length FP64 vectors stored one after another (X holds the
  * initial guesses and receives the solutions). One multi-vector FP64 K.u per
- * iteration, one V-cycle over all columns, alpha/beta from nrhs x nrhs Gram
- * matrices; columns leave the block once ||r_j|| <= tol ||mask b_j||.
- * out_relres receives nrhs values.
- * Returns 0 (all converged), 1 (maxiter reached) or < 0. The reference solves
+ * iteration, one V-cycle over all columns (over groups of them where the device
+ * has no memory for all at once), alpha/beta from nrhs x nrhs Gram matrices;
+ * columns leave the block once ||r_j|| <= tol ||mask b_j||. out_relres receives
+ * nrhs values. Returns 0 (all converged), 1 (maxiter reached) or < 0. The reference solves
  * one load case per PCG (_cupy_pcg, src/gpu_fem/solver_v2.py:552-624); this
  * replaces nrhs of those calls. */
 int topo_block_pcg(topo_ctx* ctx, const double* B, double* X, int nrhs, double tol, int maxiter,

@@ -45,6 +45,7 @@ SIGNATURES = {
     "topo_debug_recip": (_i, [_ll, _vp, _vp, _vp]),
     "topo_debug_rap_room": (_i, [_i, _i, _i, C.POINTER(_ll)]),
     "topo_debug_scratch": (_i, [_vp, _i]),
+    "topo_debug_block_columns": (_i, [_vp, _i]),
     "topo_debug_bounds": (_i, [C.POINTER(_i)]),
     "topo_diag": (_i, [_vp, _vp, _vp, _vp]),
     "topo_gmg_setup": (_i, [_vp, _vp, _vp]),

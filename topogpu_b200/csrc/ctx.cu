@@ -202,8 +202,10 @@ struct topo_ctx {
   std::vector<double> pcg_key;
   // block PCG workspace, grown by the widest block so far (block_reserve)
   int bw = 1;                   // columns the V-cycle works on
-  int blk_cols = 0;             // columns the workspace holds
-  void* blk_vecs = nullptr;     // the levels' vectors of every column
+  int blk_nv = 0;               // load cases it holds
+  int blk_cols = 0;             // columns the V-cycle takes at once (0: one, in its own vectors)
+  int blk_most = 8;             // and at most
+  void* blk_vecs = nullptr;     // the levels' vectors of that many columns
   double* blk = nullptr;        // FP64 columns R, Z, P, Q, Pn
   double* blk_y = nullptr;      // coarsest work of every column,
   int blk_y_n = 0, blk_y_cols = 0;  // made for this coarsest size and this many columns
@@ -244,6 +246,21 @@ struct topo_ctx {
     allocs.push_back({p, sz});
     bytes += (long long)sz;
     return (T*)p;
+  }
+  // Zeroed memory that leaves at least as much free, or null.
+  void* alloc_spare(size_t sz) {
+    size_t free = 0, total = 0;
+    void* p = nullptr;
+    TOPO_CUDA_CHECK(cudaMemGetInfo(&free, &total));
+    if (sz > free / 2) return nullptr;
+    if (cudaMalloc(&p, sz) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    allocs.push_back({p, sz});
+    bytes += (long long)sz;
+    TOPO_CUDA_CHECK(cudaMemsetAsync(p, 0, sz, cs));
+    return p;
   }
   // Give back what a call has replaced; the caller has waited for its users.
   void release(void* p) {
@@ -483,29 +500,38 @@ void vcycle_apply(topo_ctx* c, const void* r, void* z, const KrylovState* st, cu
 // (on the coarse levels) a fetch of the coefficients serve all of them; the
 // columns one after another left most kernels latency bound.
 //
-// The workspace of nv columns: made by the first block solve, replaced by a
-// wider one's, and kept. Only the coarsest work depends on the coarsest size.
+// The workspace of nv load cases: made by the first block solve, replaced by a
+// wider one's, and kept. The V-cycle's vectors of all columns are about as large as
+// the solve's own, so where memory is short it takes fewer columns at once, and with
+// no room for two it runs them one after another in the context's vectors. Only the
+// coarsest work depends on the coarsest size.
 void block_reserve(topo_ctx* c, int nv, cudaStream_t s) {
-  if (c->blk_cols < nv) {
+  if (c->blk_nv < nv) {
     TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
-    c->blk_cols = 0;
+    c->blk_nv = c->blk_cols = 0;
     c->release(c->blk_vecs);
     c->release(c->blk);
     c->blk_vecs = c->blk = nullptr;
-    long long total = 0;
+    long long column = 0;
     for (Level& Lv : c->L) {
       Lv.vs = (Lv.g.ndof + 3) & ~3LL;  // columns 16-byte aligned in FP32 and FP64
       std::fill(Lv.cols, Lv.cols + 6, nullptr);
-      total += (&Lv == &c->L[0] ? 6 : 5) * nv * Lv.vs;
+      column += (&Lv == &c->L[0] ? 6 : 5) * Lv.vs;
     }
     c->blk = c->alloc<double>(5 * nv * c->L[0].vs);
-    c->blk_vecs = c->valloc(total);
-    char* at = (char*)c->blk_vecs;
-    for (Level& Lv : c->L)
-      for (int i = 0; i < (&Lv == &c->L[0] ? 6 : 5); ++i, at += c->vsize() * nv * Lv.vs) Lv.cols[i] = at;
-    c->blk_cols = nv;
+    int w = std::min(nv, c->blk_most);
+    while (w > 1 && !(c->blk_vecs = c->alloc_spare(c->vsize() * w * column))) w = (w + 1) / 2;
+    if (w > 1) {
+      char* at = (char*)c->blk_vecs;
+      for (Level& Lv : c->L)
+        for (int i = 0; i < (&Lv == &c->L[0] ? 6 : 5); ++i, at += c->vsize() * w * Lv.vs) Lv.cols[i] = at;
+      c->blk_cols = w;
+    }
+    c->blk_nv = nv;
   }
-  if (c->blk_y_n != c->C.n || c->blk_y_cols < nv) {
+  if (c->blk_cols == 0) return;
+  const int nv_y = c->blk_cols;
+  if (c->blk_y_n != c->C.n || c->blk_y_cols < nv_y) {
     TOPO_CUDA_CHECK(cudaStreamSynchronize(s));
     c->blk_y_cols = 0;
     c->release(c->blk_y);
@@ -1059,8 +1085,9 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
   };
   // Z_a = M R_a for the k active columns at once; in place where they lie side
   // by side (until a column in the middle has converged), through the V-cycle's
-  // own vectors where not (8 columns of 96x48x48: 16 copies of 7 us each)
-  auto precond = [&](double* const* r, double* const* z, int k) {
+  // own vectors where not (8 columns of 96x48x48: 16 copies of 7 us each); in
+  // groups of blk_cols where the workspace holds fewer
+  auto group = [&](double* const* r, double* const* z, int k) {
     Level& L0b = c->L[0];
     char* b0 = (char*)L0b.cols[5];
     char* x0 = (char*)L0b.cols[0];
@@ -1074,6 +1101,21 @@ int do_block_pcg(topo_ctx* c, const double* B, double* X, int nv, double tol, in
     for (int a = 0; a < k; ++a) vcast(n, r[a], true, b0 + a * st, c->vec64, s);
     vcycle_columns(c, k, b0, x0, s);
     for (int a = 0; a < k; ++a) vcast(n, x0 + a * st, c->vec64, z[a], true, s);
+  };
+  auto precond = [&](double* const* r, double* const* z, int k) {
+    if (c->blk_cols > 0) {
+      for (int a = 0; a < k; a += c->blk_cols) group(r + a, z + a, std::min(c->blk_cols, k - a));
+      return;
+    }
+    for (int a = 0; a < k; ++a) {
+      if (c->vec64) {
+        vcycle_apply(c, r[a], z[a], nullptr, s);
+      } else {
+        vcast(n, r[a], true, c->kr, false, s);
+        vcycle_apply(c, c->kr, c->kz, nullptr, s);
+        vcast(n, c->kz, false, z[a], true, s);
+      }
+    }
   };
   // Y = K U: one launch for all columns where the parity form applies
   auto apply = [&](double* const* U, double* const* Y, int k) {
@@ -1756,6 +1798,18 @@ int topo_debug_scratch(topo_ctx* c, int rap_planes) {
       const Grid &f = c->L[1].g, &k = c->L[2].g;
       c->rap_room = std::min(rap_scratch(f, k), 243LL * (f.NY + k.NY) * k.NZ * rap_planes);
     }
+    return 0;
+  } catch (const std::exception& e) {
+    return fail(c, e);
+  }
+}
+
+int topo_debug_block_columns(topo_ctx* c, int columns) {
+  try {
+    if (!c) throw std::invalid_argument("topo_debug_block_columns: null context");
+    if (columns < 1 || columns > 8) throw std::invalid_argument("topo_debug_block_columns: columns must be 1..8");
+    c->blk_most = columns;
+    c->blk_nv = 0;  // the next block solve makes its workspace again
     return 0;
   } catch (const std::exception& e) {
     return fail(c, e);
