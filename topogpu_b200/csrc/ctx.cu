@@ -217,7 +217,7 @@ struct topo_ctx {
   double* dtmp = nullptr;       // 64 device doubles
   double* oc_state = nullptr;
   double* Hs = nullptr;        // nelem doubles: scratch of the filter and the OC updates
-  double* oc_cand = nullptr;   // candidates of the projected OC (allocated by its first call)
+  double* oc_cand = nullptr;   // candidates of the projected OC (level 0's x, r and d)
   FilterStencil fstencil;
   bool ke_registered = false;  // holds a reference on its device's KE
   cudaStream_t cs = nullptr;
@@ -234,17 +234,17 @@ struct topo_ctx {
   long long bytes = 0;
   std::string err;
 
-  // Device memory of the context. alloc zeroes it on the context's stream: a
-  // memset on the default stream is not ordered with that stream or with a
-  // caller's non-blocking one. Memory that a call on the caller's stream makes
-  // comes from alloc_raw and is written there before it is read.
+  // Device memory of the context, made by its creation and by calls that run on
+  // the context's stream. alloc zeroes it there: a memset on the default stream is
+  // not ordered with that stream or with a caller's non-blocking one.
   template <typename T>
-  T* alloc_raw(long long count) {
+  T* alloc(long long count) {
     void* p = nullptr;
     const size_t sz = (size_t)std::max<long long>(count, 1) * sizeof(T);
     TOPO_CUDA_CHECK(cudaMalloc(&p, sz));
     allocs.push_back({p, sz});
     bytes += (long long)sz;
+    TOPO_CUDA_CHECK(cudaMemsetAsync(p, 0, sz, cs));
     return (T*)p;
   }
   // Zeroed memory that leaves at least as much free, or null.
@@ -271,12 +271,6 @@ struct topo_ctx {
         cudaFree(p);
         return;
       }
-  }
-  template <typename T>
-  T* alloc(long long count) {
-    T* p = alloc_raw<T>(count);
-    TOPO_CUDA_CHECK(cudaMemsetAsync(p, 0, (size_t)std::max<long long>(count, 1) * sizeof(T), cs));
-    return p;
   }
   void* valloc(long long count) { return vec64 ? (void*)alloc<double>(count) : (void*)alloc<float>(count); }
   size_t vsize() const { return vec64 ? 8 : 4; }
@@ -1436,9 +1430,15 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
       Level& Lv = c->L[l];
       const long long nd = Lv.g.ndof;
       Lv.mask = c->alloc<uint8_t>(nd + 16);  // the tensor-core K.u reads aligned 4-byte mask words
-      Lv.x = c->valloc(nd);
-      Lv.r = c->valloc(nd);
-      Lv.d = c->valloc(nd);
+      // x, r and d of a level side by side, each 16-byte aligned. A V-cycle and the
+      // spectral bound write all of them before they read any, so level 0's serve
+      // the projected OC too (9 entries per node hold its doubles per element)
+      static_assert(kOcCandidates * sizeof(double) <= 9 * sizeof(float), "more candidates than room");
+      const long long va = (nd + 3) & ~3LL;
+      Lv.x = c->valloc(3 * va);
+      Lv.r = (char*)Lv.x + c->vsize() * va;
+      Lv.d = (char*)Lv.r + c->vsize() * va;
+      if (l == 0) c->oc_cand = (double*)Lv.x;
       Lv.d2 = c->valloc(nd);
       Lv.e = c->valloc(nd);
       if (l == 0) Lv.b = c->valloc(nd);  // (the restriction writes the other levels' right-hand side to r)
@@ -2053,7 +2053,6 @@ int topo_oc_projected(topo_ctx* c, double rmin, const double* rho, const double*
       throw std::invalid_argument("topo_oc_projected: out must not alias rho, dc or dv");
     DirectGuard sg(c, stream);
     cudaStream_t us = sg.user;
-    if (!c->oc_cand) c->oc_cand = c->alloc_raw<double>(oc_projected_candidates() * c->L[0].g.nelem);
     const int ev = oc_update_projected(c->fstencil, c->L[0].g, rmin, rho, dc, dv, beta, eta, volfrac, move, rho_min, out, c->Hs,
                                        c->oc_cand, c->red, c->oc_state, us);
     if (out_evals) *out_evals = ev;

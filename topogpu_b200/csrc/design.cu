@@ -623,7 +623,7 @@ void heaviside_apply(long long n, const double* rho_f, double beta, double eta, 
 // filters all of them at every element with one pass over the taps, projects
 // and sums. At 96x48x48 (rmin 2) a sweep is 36 us and a call takes about 6 of
 // them, against 60 sequential evaluations of 26 us.
-constexpr int OP_NC = 4;
+constexpr int OP_NC = kOcCandidates;
 
 __global__ void __launch_bounds__(256) k_ocp_cand(long long n, const double* __restrict__ rho, const double* __restrict__ sv,
                                                   double move, double rho_min, const double* st, double* __restrict__ cand) {
@@ -703,8 +703,6 @@ int oc_update_projected(FilterStencil& fs, const Grid& g, double rmin, const dou
   TOPO_LAUNCH_CHECK();
   return evals;
 }
-
-int oc_projected_candidates() { return OP_NC; }
 
 // ------------------------------------------------------------ field stats
 __global__ void k_stats(long long n, const double* __restrict__ x, double* out4, RedWork red) {

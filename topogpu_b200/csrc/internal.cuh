@@ -419,7 +419,7 @@ void heaviside_apply(long long n, const double* rho_f, double beta, double eta, 
 int oc_update_projected(FilterStencil& fs, const Grid& g, double rmin, const double* rho, const double* dc, const double* dv,
                         double beta, double eta, double volfrac, double move, double rho_min, double* out,
                         double* work, double* cand, RedWork red, double* st, cudaStream_t s);
-int oc_projected_candidates();  // cand holds this many doubles per element
+constexpr int kOcCandidates = 4;  // cand holds this many doubles per element
 void field_stats(long long n, const double* x, double* out4_dev, RedWork red, cudaStream_t s);
 
 // error plumbing
