@@ -1430,11 +1430,11 @@ int topo_ctx_create(int nelx, int nely, int nelz, int n_levels, int mode, int fi
       Level& Lv = c->L[l];
       const long long nd = Lv.g.ndof;
       Lv.mask = c->alloc<uint8_t>(nd + 16);  // the tensor-core K.u reads aligned 4-byte mask words
-      // x, r and d of a level side by side, each 16-byte aligned. A V-cycle and the
+      // x, r and d of a level side by side, each at the start of a line. A V-cycle and the
       // spectral bound write all of them before they read any, so level 0's serve
       // the projected OC too (9 entries per node hold its doubles per element)
       static_assert(kOcCandidates * sizeof(double) <= 9 * sizeof(float), "more candidates than room");
-      const long long va = (nd + 3) & ~3LL;
+      const long long va = (nd + 127) & ~127LL;
       Lv.x = c->valloc(3 * va);
       Lv.r = (char*)Lv.x + c->vsize() * va;
       Lv.d = (char*)Lv.r + c->vsize() * va;
