@@ -242,8 +242,9 @@ int topo_set_tc(topo_ctx* ctx, int on);
  * initial guesses and receives the solutions). One multi-vector FP64 K.u per
  * iteration, one V-cycle over all columns (over groups of them where the device
  * has no memory for all at once), alpha/beta from nrhs x nrhs Gram matrices;
- * columns leave the block once ||r_j|| <= tol ||mask b_j||. out_relres receives
- * nrhs values. Returns 0 (all converged), 1 (maxiter reached) or < 0. The reference solves
+ * columns leave the block once ||r_j|| <= tol ||mask b_j||. Where the residuals
+ * become dependent the columns left are solved one after another, out_iters
+ * counting the longest of them. out_relres receives nrhs values. Returns 0 (all converged), 1 (maxiter reached) or < 0. The reference solves
  * one load case per PCG (_cupy_pcg, src/gpu_fem/solver_v2.py:552-624); this
  * replaces nrhs of those calls. */
 int topo_block_pcg(topo_ctx* ctx, const double* B, double* X, int nrhs, double tol, int maxiter,
